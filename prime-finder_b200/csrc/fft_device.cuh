@@ -1,0 +1,658 @@
+// Floating-point form of the Montgomery step (the strong test's and the
+// modular powers' squarings): exact integer products by weighted complex
+// FFTs in double precision, one CTA per candidate.
+//
+// x is held as n = 2 C signed limbs of b bits (B = 2^b), limb j and limb
+// j + C together one complex point.  With the Montgomery radix R' = B^n + 1:
+//
+//   D  = x^2 mod (B^n + 1)
+//   m  = D N'' mod (B^n + 1)                 N'' = -N^-1 mod R', spectrum stored
+//   U  = (x^2 + m N) / R'                    spectrum of N stored
+//
+// U is found modulo M2 = B^n + B^(n/2) + 1, where R' = -B^(n/2) has the
+// inverse B^(n/2) + 1: the sum x^2 + m N is formed on the spectra (one
+// inverse transform for both), and division by R' is a linear map of the two
+// halves.  Seven complex transforms of length C per squaring, where the
+// integer form (mr_device.cuh) takes eight of length 2 C for each of two
+// primes.
+//
+//   B^n + 1:             z_j = x_j + i x_(j+C)      modulo y^C - i
+//   B^n + B^(n/2) + 1:   z_j = x_j + w x_(j+C)      modulo y^C - w, w = e^(2 pi i/3)
+//
+// The transform is the remainder tree of y^C - e^(i phi): a node y^(2m) - r^2
+// has the children y^m - r and y^m + r, so a butterfly is (lo + r hi, lo - r
+// hi) with one r per node: no weighting sweeps, and the first pass has the
+// same few constants in every thread.
+//
+// Limbs are signed and redundant (|limb| <= B/2 + 40): the coefficients are
+// brought back to limbs by three local carry steps, with no carry chain over
+// the number.  |U| < 0.7 N is a signed residue; B^n is far above it, so the
+// limbs found modulo M2 are U itself and not U plus a multiple of M2.
+//
+// Exactness.  A product of two operands z, z' of C points by these transforms
+// has an error below |z| |z'| (3 levels + 4) 5 2^-53 in every coefficient
+// (2-norms; the argument of Percival, "Rapid multiplication modulo the sum
+// and difference of highly composite numbers", Math. Comp. 72 (2003), with 5
+// units for a level: a fused forward butterfly with its rounded root makes
+// at most 3.8 of the norm it hands on, an inverse one 3.8).  With |limb| at
+// most B/2 + 40, |z|^2 <= 1.5 n limb^2 modulo M2 (z = x + w y); U adds two
+// products, and its halves are re -+ im / sqrt(3): 3.5 n limb^2 in all.
+// limb_bits() keeps that below 0.4, so the rounding to integers is exact for
+// all inputs, not only for likely ones.
+#pragma once
+#include <cuda_runtime.h>
+#include <math.h>
+#include <stdint.h>
+#include <string.h>
+
+namespace pfb {
+namespace mr {
+namespace fp {
+
+struct alignas(16) Cplx {
+    double re, im;
+};
+
+// ---- length classes --------------------------------------------------------
+// C complex points, passes of radix R1, R2, R3, R4 (R4 = 1: three passes),
+// T = C / R1 threads: a thread holds one group of the first pass, and the
+// last inverse pass, the carries and the next first pass stay in registers.
+// SQS: x^2's spectrum waits in shared memory (else in global memory); PADL:
+// one unused point per 2^PADL in shared memory against bank conflicts of the
+// last pass.
+template <int ID_, int C_, int R1_, int R2_, int R3_, int R4_, bool SQS_, int MINB_>
+struct Cls {
+    static constexpr int ID = ID_, C = C_, R1 = R1_, R2 = R2_, R3 = R3_, R4 = R4_, T = C_ / R1_, N = 2 * C_;
+    static constexpr bool SQS = SQS_;
+    static constexpr int MINB = MINB_;
+    static constexpr int NPASS = R4_ > 1 ? 4 : 3;
+    static constexpr int RM = R4_ > 1 ? R4_ : R3_;  // radix of the middle sweep
+    static constexpr int PADL = RM >= 16 ? 4 : 3;
+    static constexpr int WARPS = T / 32;
+    static_assert(R1_ * R2_ * R3_ * R4_ == C_ && T % 32 == 0, "pass radices");
+    // bytes: points (padded), x limbs, boundary carries, flags, x^2's spectrum
+    static constexpr int A_PTS = C_ + (C_ >> PADL);
+    static constexpr size_t smem() {
+        return (size_t)A_PTS * 16 + (size_t)C_ * 8 + (size_t)2 * WARPS * R1_ * 8 + 256 + (SQS_ ? (size_t)C_ * 16 : 0);
+    }
+};
+
+constexpr int kClasses = 8;
+using Cls0 = Cls<0, 64, 2, 4, 8, 1, true, 8>;
+using Cls1 = Cls<1, 128, 4, 4, 8, 1, true, 8>;
+using Cls2 = Cls<2, 256, 4, 8, 8, 1, true, 8>;
+using Cls3 = Cls<3, 512, 8, 8, 8, 1, true, 6>;
+using Cls4 = Cls<4, 1024, 8, 16, 8, 1, true, 3>;
+using Cls5 = Cls<5, 2048, 16, 16, 8, 1, true, 2>;
+using Cls6 = Cls<6, 4096, 16, 16, 16, 1, true, 1>;
+using Cls7 = Cls<7, 8192, 16, 8, 8, 8, false, 1>;
+#define PFB_FP_CLASSES(F) F(Cls0) F(Cls1) F(Cls2) F(Cls3) F(Cls4) F(Cls5) F(Cls6) F(Cls7)
+
+inline int class_points(int cls) {
+    static const int c[kClasses] = {64, 128, 256, 512, 1024, 2048, 4096, 8192};
+    return c[cls];
+}
+
+// Largest b for which every coefficient is provably rounded to the right
+// integer (see the head of the file).
+inline int limb_bits(int cls) {
+    const int C = class_points(cls);
+    int lv = 0;
+    while ((1 << lv) < C) lv++;
+    for (int b = 24;; b--) {
+        const double limb = ldexp(1.0, b - 1) + 40.0;
+        const double err = 3.5 * (2.0 * C) * limb * limb * (3.0 * lv + 4.0) * 5.0 * ldexp(1.0, -53);
+        if (err < 0.4) return b;
+    }
+}
+
+// ---- tables ----------------------------------------------------------------
+// Roots of the passes after the first: [modulus][pass - 2] planes [q][node],
+// R/2 planes per pass (level 0: 1 root, level s: 2^(s-1) roots; the others
+// are i times those).
+struct Tab {
+    const Cplx *t[2][3];
+};
+
+// The first pass' roots, the same for every length: entry q of a radix-16
+// group at the root of the tree.
+struct First {
+    Cplx r[2][8];
+};
+__constant__ First c_first;
+
+#ifdef __CUDA_ARCH__
+__device__ __forceinline__ Cplx ldg(const Cplx *p) {
+    const double2 v = __ldg(reinterpret_cast<const double2 *>(p));
+    return Cplx{v.x, v.y};
+}
+__device__ __forceinline__ Cplx ldcg(const Cplx *p) {
+    const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
+    return Cplx{v.x, v.y};
+}
+__device__ __forceinline__ long long bits_of(double d) { return __double_as_longlong(d); }
+__device__ __forceinline__ double from_bits(long long v) { return __longlong_as_double(v); }
+#else
+inline Cplx ldg(const Cplx *p) { return *p; }
+inline Cplx ldcg(const Cplx *p) { return *p; }
+inline long long bits_of(double d) {
+    long long v;
+    memcpy(&v, &d, 8);
+    return v;
+}
+inline double from_bits(long long v) {
+    double d;
+    memcpy(&d, &v, 8);
+    return d;
+}
+#endif
+
+template <class F>
+__device__ __forceinline__ void cta_sync() {
+#ifdef __CUDA_ARCH__
+    if (F::T == 32) __syncwarp();
+    else __syncthreads();
+#else
+    __syncthreads();
+#endif
+}
+
+template <class F>
+__device__ __forceinline__ int padx(int i) {
+    return i + (i >> F::PADL);
+}
+
+// int (|v| < 2^31) to double without the conversion unit: 2^52 + 2^31 + v has
+// v + 2^31 in its low word.
+__device__ __forceinline__ double to_double(int v) {
+    const unsigned u = (unsigned)v ^ 0x80000000u;
+    return from_bits((long long)((0x43300000ull << 32) | u)) - 4503601774854144.0;
+}
+
+// ---- butterflies -----------------------------------------------------------
+// (a, b) <- (a + r b, a - r b), r replaced by i r when ROT.
+template <bool ROT>
+__device__ __forceinline__ void bf_fwd(Cplx &a, Cplx &b, const Cplx &r) {
+    const double br = ROT ? -b.im : b.re, bi = ROT ? b.re : b.im;
+    const double tr = fma(-r.im, bi, fma(r.re, br, a.re));
+    const double ti = fma(r.re, bi, fma(r.im, br, a.im));
+    b.re = fma(2.0, a.re, -tr);
+    b.im = fma(2.0, a.im, -ti);
+    a.re = tr;
+    a.im = ti;
+}
+
+// The inverse, twice it: (p, q) <- (p + q, (p - q) conj(r)).
+template <bool ROT>
+__device__ __forceinline__ void bf_inv(Cplx &p, Cplx &q, const Cplx &r) {
+    const double dr0 = p.re - q.re, di0 = p.im - q.im;
+    p.re += q.re;
+    p.im += q.im;
+    const double dr = ROT ? di0 : dr0, di = ROT ? -dr0 : di0;  // times conj(i) = -i
+    q.re = fma(dr, r.re, di * r.im);
+    q.im = fma(di, r.re, -(dr * r.im));
+}
+
+// A group's levels; tw[0] the root of the first level, tw[2^(s-1) + u] that
+// of node 2u of level s.
+template <int R>
+__device__ __forceinline__ void fwd_group(Cplx *v, const Cplx *tw) {
+#pragma unroll
+    for (int half = R / 2, nodes = 1; half >= 1; half >>= 1, nodes <<= 1) {
+#pragma unroll
+        for (int nd = 0; nd < nodes; nd++) {
+            const Cplx &r = tw[nodes == 1 ? 0 : nodes / 2 + nd / 2];
+#pragma unroll
+            for (int e = 0; e < half; e++) {
+                const int at = nd * 2 * half + e;
+                if (nd & 1) bf_fwd<true>(v[at], v[at + half], r);
+                else bf_fwd<false>(v[at], v[at + half], r);
+            }
+        }
+    }
+}
+
+template <int R>
+__device__ __forceinline__ void inv_group(Cplx *v, const Cplx *tw) {
+#pragma unroll
+    for (int half = 1, nodes = R / 2; half < R; half <<= 1, nodes >>= 1) {
+#pragma unroll
+        for (int nd = 0; nd < nodes; nd++) {
+            const Cplx &r = tw[nodes == 1 ? 0 : nodes / 2 + nd / 2];
+#pragma unroll
+            for (int e = 0; e < half; e++) {
+                const int at = nd * 2 * half + e;
+                if (nd & 1) bf_inv<true>(v[at], v[at + half], r);
+                else bf_inv<false>(v[at], v[at + half], r);
+            }
+        }
+    }
+}
+
+template <int R>
+__device__ __forceinline__ void load_roots(Cplx *tw, const Cplx *tab, int nodes, int node) {
+#pragma unroll
+    for (int q = 0; q < R / 2; q++) tw[q] = ldg(tab + q * nodes + node);
+}
+
+// One pass of radix R over the C points in A: NODES nodes of C / NODES
+// points, element stride SUB.
+template <class F, int R, int NODES, bool INV>
+__device__ __forceinline__ void pass(Cplx *A, const Cplx *tab) {
+    constexpr int SUB = F::C / NODES / R, G = F::C / R;
+#pragma unroll 1
+    for (int g = threadIdx.x; g < G; g += F::T) {
+        const int node = g / SUB, j0 = g % SUB, base = node * (R * SUB) + j0;
+        Cplx tw[R / 2], v[R];
+        load_roots<R>(tw, tab, NODES, node);
+#pragma unroll
+        for (int e = 0; e < R; e++) v[e] = A[padx<F>(base + e * SUB)];
+        if constexpr (INV) inv_group<R>(v, tw);
+        else fwd_group<R>(v, tw);
+#pragma unroll
+        for (int e = 0; e < R; e++) A[padx<F>(base + e * SUB)] = v[e];
+    }
+    cta_sync<F>();
+}
+
+enum MidOp { MID_STORE_SQ, MID_STORE, MID_SQ, MID_MUL, MID_MULADD };
+
+// The last forward pass, the pointwise operation and the first inverse pass
+// on groups of RM consecutive points.  Spectra outside A are laid out
+// [element][group], so a warp reads and writes them contiguously, and S is
+// read back by the thread that wrote it.
+//   MID_STORE_SQ, MID_STORE: S <- v^2, S <- v, no inverse
+//   MID_SQ: v^2    MID_MUL: v G    MID_MULADD: v G + S
+template <class F>
+__device__ __forceinline__ void mid(Cplx *A, const Cplx *tab, int op, const Cplx *Gs, Cplx *S) {
+    constexpr int R = F::RM, G = F::C / R;
+#pragma unroll 1
+    for (int g = threadIdx.x; g < G; g += F::T) {
+        Cplx tw[R / 2], v[R];
+        load_roots<R>(tw, tab, G, g);
+        const int base = padx<F>(g * R);
+#pragma unroll
+        for (int e = 0; e < R; e++) v[e] = A[R <= (1 << F::PADL) ? base + e : padx<F>(g * R + e)];
+        fwd_group<R>(v, tw);
+        if (op == MID_MUL || op == MID_MULADD) {
+#pragma unroll
+            for (int e = 0; e < R; e++) {
+                const Cplx c = ldg(Gs + e * G + g);
+                Cplx s{0.0, 0.0};
+                if (op == MID_MULADD) s = F::SQS ? S[e * G + g] : ldcg(S + e * G + g);
+                const double re = fma(v[e].re, c.re, fma(-v[e].im, c.im, s.re));
+                const double im = fma(v[e].re, c.im, fma(v[e].im, c.re, s.im));
+                v[e].re = re;
+                v[e].im = im;
+            }
+        } else if (op == MID_STORE) {
+#pragma unroll
+            for (int e = 0; e < R; e++) S[e * G + g] = v[e];
+            continue;
+        } else {
+#pragma unroll
+            for (int e = 0; e < R; e++) {
+                const double re = fma(v[e].re, v[e].re, -(v[e].im * v[e].im));
+                const double im = (v[e].re + v[e].re) * v[e].im;
+                v[e].re = re;
+                v[e].im = im;
+            }
+            if (op == MID_STORE_SQ) {
+#pragma unroll
+                for (int e = 0; e < R; e++) S[e * G + g] = v[e];
+                continue;
+            }
+        }
+        inv_group<R>(v, tw);
+#pragma unroll
+        for (int e = 0; e < R; e++) A[R <= (1 << F::PADL) ? base + e : padx<F>(g * R + e)] = v[e];
+    }
+    cta_sync<F>();
+}
+
+// ---- one candidate's working set -------------------------------------------
+struct View {
+    Cplx *A;       // points, padded
+    Cplx *S;       // a spectrum, [element][group]
+    int *xs;       // limbs of x: [2 e + half][thread]
+    int *bnd;      // carries between warps
+    uint32_t *sc;  // scratch words of the carry scan and of votes
+};
+
+template <class F>
+__device__ __forceinline__ void carve(unsigned char *raw, Cplx *gscratch, View &w) {
+    w.A = reinterpret_cast<Cplx *>(raw);
+    raw += (size_t)F::A_PTS * 16;
+    if (F::SQS) {
+        w.S = reinterpret_cast<Cplx *>(raw);
+        raw += (size_t)F::C * 16;
+    } else {
+        w.S = gscratch;
+    }
+    w.xs = reinterpret_cast<int *>(raw);
+    raw += (size_t)F::C * 8;
+    w.bnd = reinterpret_cast<int *>(raw);
+    raw += (size_t)2 * F::WARPS * F::R1 * 8;
+    w.sc = reinterpret_cast<uint32_t *>(raw);
+}
+
+// First forward pass from the limbs in registers: modulus MOD (0: B^n + 1,
+// 1: M2), into A.
+template <class F, int MOD>
+__device__ __forceinline__ void first_pass(Cplx *A, const int *lo, const int *hi) {
+    Cplx v[F::R1];
+#pragma unroll
+    for (int e = 0; e < F::R1; e++) {
+        const double a = to_double(lo[e]), c = to_double(hi[e]);
+        if (MOD == 0) {
+            v[e].re = a;
+            v[e].im = c;
+        } else {
+            v[e].re = fma(-0.5, c, a);
+            v[e].im = 0.86602540378443864676 * c;
+        }
+    }
+    fwd_group<F::R1>(v, c_first.r[MOD]);
+#pragma unroll
+    for (int e = 0; e < F::R1; e++) A[padx<F>((int)threadIdx.x + e * F::T)] = v[e];
+    cta_sync<F>();
+}
+
+// Carries of every limb to the next one: k in, the neighbour's carry out.
+// Limb order: thread t + T e, then the second half; the carry out of the top
+// limb comes back negated (B^n = -1), modulo M2 at limbs 0 and n/2.
+template <class F, int MOD>
+__device__ __forceinline__ void exchange(int *kl, int *kh, int *buf) {
+    constexpr int R = F::R1;
+    const unsigned FULL = 0xffffffffu;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int pl[R], ph[R];
+    if constexpr (F::WARPS > 1) {
+        if (lane == 31) {
+#pragma unroll
+            for (int e = 0; e < R; e++) {
+                buf[(warp * R + e) * 2] = kl[e];
+                buf[(warp * R + e) * 2 + 1] = kh[e];
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int e = 0; e < R; e++) {
+            pl[e] = __shfl_up_sync(FULL, kl[e], 1);
+            ph[e] = __shfl_up_sync(FULL, kh[e], 1);
+        }
+        if (lane == 0) {
+            const int w = warp ? warp - 1 : F::WARPS - 1;
+#pragma unroll
+            for (int e = 0; e < R; e++) {
+                pl[e] = buf[(w * R + e) * 2];
+                ph[e] = buf[(w * R + e) * 2 + 1];
+            }
+        }
+    } else {
+#pragma unroll
+        for (int e = 0; e < R; e++) {
+            pl[e] = __shfl_sync(FULL, kl[e], (lane + 31) & 31);
+            ph[e] = __shfl_sync(FULL, kh[e], (lane + 31) & 31);
+        }
+    }
+    if (threadIdx.x == 0) {  // the last thread's carries go to the next element
+        const int tl = pl[R - 1], th = ph[R - 1];
+#pragma unroll
+        for (int e = R - 1; e > 0; e--) {
+            pl[e] = pl[e - 1];
+            ph[e] = ph[e - 1];
+        }
+        pl[0] = -th;
+        ph[0] = MOD == 0 ? tl : tl - th;
+    }
+#pragma unroll
+    for (int e = 0; e < R; e++) {
+        kl[e] = pl[e];
+        kh[e] = ph[e];
+    }
+}
+
+// Last inverse pass, rounding and carries: the C points in A to limbs, times
+// two when dbl.  MOD 1: the value found is that of the points divided by R'.
+template <class F, int MOD>
+__device__ __forceinline__ void last_pass(const View &w, int b, int dbl, int *lo, int *hi) {
+    constexpr int R = F::R1;
+    constexpr double S0 = 1.0 / F::C;
+    const int mask = (1 << b) - 1, half = 1 << (b - 1), bs = b - dbl;
+    // 1.5 2^52 + B/2 (B/4 when doubled): the sum's low 51 bits are the rounded
+    // coefficient plus that offset
+    const double magic = 6755399441055744.0 + (double)(half >> dbl);
+    int kl[R], kh[R];
+    {
+        Cplx v[R];
+#pragma unroll
+        for (int e = 0; e < R; e++) v[e] = w.A[padx<F>((int)threadIdx.x + e * F::T)];
+        inv_group<R>(v, c_first.r[MOD]);
+#pragma unroll
+        for (int e = 0; e < R; e++) {
+            long long ql, qh;
+            if (MOD == 0) {
+                ql = bits_of(fma(v[e].re, S0, magic));
+                qh = bits_of(fma(v[e].im, S0, magic));
+            } else {
+                // u + w v = re + i im: v = 2/sqrt(3) im, u = re + v / 2; times
+                // (1 + y) with y^2 = -y - 1: (u - v) + u y
+                const double h = v[e].im * 0.57735026918962576451;  // v / 2
+                ql = bits_of(fma(v[e].re - h, S0, magic));
+                qh = bits_of(fma(v[e].re + h, S0, magic));
+            }
+            ql -= 0x4338000000000000ll;
+            qh -= 0x4338000000000000ll;
+            kl[e] = (int)(ql >> bs);
+            kh[e] = (int)(qh >> bs);
+            lo[e] = (int)(((unsigned)ql << dbl) & (unsigned)mask) - half;
+            hi[e] = (int)(((unsigned)qh << dbl) & (unsigned)mask) - half;
+        }
+    }
+    exchange<F, MOD>(kl, kh, w.bnd);
+#pragma unroll
+    for (int round = 1; round <= 2; round++) {
+#pragma unroll
+        for (int e = 0; e < R; e++) {
+            const int cl = lo[e] + kl[e] + half, ch = hi[e] + kh[e] + half;
+            kl[e] = cl >> b;
+            kh[e] = ch >> b;
+            lo[e] = (cl & mask) - half;
+            hi[e] = (ch & mask) - half;
+        }
+        exchange<F, MOD>(kl, kh, w.bnd + (round & 1) * 2 * F::WARPS * R);
+    }
+#pragma unroll
+    for (int e = 0; e < R; e++) {
+        lo[e] += kl[e];
+        hi[e] += kh[e];
+    }
+}
+
+// The passes between the first and the middle one.
+template <class F>
+__device__ __forceinline__ void fwd_inner(Cplx *A, const Cplx *const *t) {
+    pass<F, F::R2, F::R1, false>(A, t[0]);
+    if constexpr (F::NPASS == 4) pass<F, F::R3, F::R1 * F::R2, false>(A, t[1]);
+}
+template <class F>
+__device__ __forceinline__ void inv_inner(Cplx *A, const Cplx *const *t) {
+    if constexpr (F::NPASS == 4) pass<F, F::R3, F::R1 * F::R2, true>(A, t[1]);
+    pass<F, F::R2, F::R1, true>(A, t[0]);
+}
+
+// One Montgomery step on the limbs (lo, hi) of x:
+//   square: x <- x^2 / R'    else: x <- x / R'    (mod N; times two when dbl)
+// nn, nh: spectra of N'' (modulo B^n + 1) and N (modulo M2).
+template <class F>
+__device__ __forceinline__ void step(const View &w, const Tab &tab, const Cplx *nn, const Cplx *nh, int b,
+                                     bool square, int dbl, int *lo, int *hi) {
+    constexpr int R = F::R1, MT = F::NPASS - 2;
+#pragma unroll
+    for (int e = 0; e < R; e++) {
+        w.xs[(2 * e) * F::T + threadIdx.x] = lo[e];
+        w.xs[(2 * e + 1) * F::T + threadIdx.x] = hi[e];
+    }
+    // phases: 0 spectrum of x (or its square) modulo M2 into S, 1 D, 2 m, 3 U
+#pragma unroll 1
+    for (int ph = 0; ph < 4; ph++) {
+        if (ph == 1 && !square) continue;  // D = x
+        const int mod = (ph == 0 || ph == 3) ? 1 : 0;
+        if (mod) first_pass<F, 1>(w.A, lo, hi);
+        else first_pass<F, 0>(w.A, lo, hi);
+        const Cplx *t[3] = {mod ? tab.t[1][0] : tab.t[0][0], mod ? tab.t[1][1] : tab.t[0][1],
+                            mod ? tab.t[1][2] : tab.t[0][2]};
+        fwd_inner<F>(w.A, t);
+        const int op = ph == 0 ? (square ? MID_STORE_SQ : MID_STORE)
+                               : (ph == 1 ? MID_SQ : (ph == 2 ? MID_MUL : MID_MULADD));
+        mid<F>(w.A, t[MT], op, ph == 2 ? nn : nh, w.S);
+        if (ph == 0) {
+#pragma unroll
+            for (int e = 0; e < R; e++) {
+                lo[e] = w.xs[(2 * e) * F::T + threadIdx.x];
+                hi[e] = w.xs[(2 * e + 1) * F::T + threadIdx.x];
+            }
+            continue;
+        }
+        inv_inner<F>(w.A, t);
+        if (mod) last_pass<F, 1>(w, b, dbl, lo, hi);
+        else last_pass<F, 0>(w, b, 0, lo, hi);
+    }
+}
+
+// lo, hi <- a times the limbs (1 <= a < 2^16), carried locally; |a x| < B^n / 4.
+template <class F>
+__device__ void mul_small(const View &w, int b, uint32_t a, int *lo, int *hi) {
+    constexpr int R = F::R1;
+    const int mask = (1 << b) - 1, half = 1 << (b - 1);
+    int kl[R], kh[R];
+#pragma unroll
+    for (int e = 0; e < R; e++) {
+        const long long ql = (long long)lo[e] * a + half, qh = (long long)hi[e] * a + half;
+        kl[e] = (int)(ql >> b);
+        kh[e] = (int)(qh >> b);
+        lo[e] = (int)(ql & mask) - half;
+        hi[e] = (int)(qh & mask) - half;
+    }
+    cta_sync<F>();
+    exchange<F, 0>(kl, kh, w.bnd);
+#pragma unroll
+    for (int round = 1; round <= 2; round++) {
+#pragma unroll
+        for (int e = 0; e < R; e++) {
+            const int cl = lo[e] + kl[e] + half, ch = hi[e] + kh[e] + half;
+            kl[e] = cl >> b;
+            kh[e] = ch >> b;
+            lo[e] = (cl & mask) - half;
+            hi[e] = (ch & mask) - half;
+        }
+        exchange<F, 0>(kl, kh, w.bnd + (round & 1) * 2 * F::WARPS * R);
+    }
+#pragma unroll
+    for (int e = 0; e < R; e++) {
+        lo[e] += kl[e];
+        hi[e] += kh[e];
+    }
+}
+
+// ---- canonical form --------------------------------------------------------
+// Carry function of a run of limbs, (f(-1), f(0), f(1)) + 1 in two bits each.
+__device__ __forceinline__ uint32_t fn_at(uint32_t f, uint32_t c) { return (f >> (2u * c)) & 3u; }
+__device__ __forceinline__ uint32_t fn_then(uint32_t f, uint32_t g) {  // g after f
+    return fn_at(g, fn_at(f, 0u)) | (fn_at(g, fn_at(f, 1u)) << 2) | (fn_at(g, fn_at(f, 2u)) << 4);
+}
+
+// The n limbs L (each within (-3B/4, 2B)) to digits in [0, B); returns the carry
+// out of the top limb (-1: the number is negative).
+template <class F>
+__device__ int normalize(int *L, int b, uint32_t *sc) {
+    constexpr int W = F::N / F::T;
+    const unsigned FULL = 0xffffffffu;
+    const int mask = (1 << b) - 1, t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    int c = 0;
+    bool zero = true, ones = true;
+    for (int q = 0; q < W; q++) {
+        const int v = L[t * W + q] + c, d = v & mask;
+        c = v >> b;
+        L[t * W + q] = d;
+        zero = zero && d == 0;
+        ones = ones && d == mask;
+    }
+    uint32_t f = (uint32_t)(c + 1 - (zero ? 1 : 0)) | ((uint32_t)(c + 1) << 2) | ((uint32_t)(c + 1 + (ones ? 1 : 0)) << 4);
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t g = __shfl_up_sync(FULL, f, o);
+        if (lane >= o) f = fn_then(g, f);
+    }
+    if (lane == 31) sc[warp] = f;
+    cta_sync<F>();
+    uint32_t cin = 1u;  // carry + 1 into this warp
+    for (int v = 0; v < warp; v++) cin = fn_at(sc[v], cin);
+    uint32_t tot = 1u;
+    for (int v = 0; v < F::WARPS; v++) tot = fn_at(sc[v], tot);
+    const uint32_t before = __shfl_up_sync(FULL, f, 1);
+    int carry = (int)(lane ? fn_at(before, cin) : cin) - 1;
+    for (int q = 0; q < W && carry; q++) {
+        const int v = L[t * W + q] + carry;
+        carry = v >> b;
+        L[t * W + q] = v & mask;
+    }
+    cta_sync<F>();
+    return (int)tot - 1;
+}
+
+// L[0..n) <- the canonical digits (base B) of the value of the limbs modulo
+// N, for a value in (-N, N); nl: N's digits.  L overlays A.
+template <class F>
+__device__ void to_digits(const View &w, int b, const uint32_t *nl, const int *lo, const int *hi, int *L) {
+    cta_sync<F>();
+#pragma unroll
+    for (int e = 0; e < F::R1; e++) {
+        L[threadIdx.x + e * F::T] = lo[e];
+        L[F::C + threadIdx.x + e * F::T] = hi[e];
+    }
+    cta_sync<F>();
+    if (normalize<F>(L, b, w.sc) < 0) {
+        for (int i = threadIdx.x; i < F::N; i += F::T) L[i] += (int)nl[i];
+        cta_sync<F>();
+        normalize<F>(L, b, w.sc);
+    }
+}
+
+// Block-wide AND of a vote.
+template <class F>
+__device__ __forceinline__ bool vote_and(bool v) {
+    return __syncthreads_and(v ? 1 : 0) != 0;
+}
+
+// Balanced limbs (|limb| <= B/2) from canonical digits d, at the positions
+// of this thread; a carry out of the top limb wraps to -1 at limb 0 (B^n =
+// -1; it cannot happen for a number below B^n / 2).
+template <class F>
+__device__ __forceinline__ void balanced(const uint32_t *d, int b, int *lo, int *hi) {
+    const int B = 1 << b, half = B >> 1;
+    auto at = [&](int i) {
+        const int v = (int)d[i];
+        const int top = (int)d[i ? i - 1 : F::N - 1] >= half ? 1 : 0;
+        return (v >= half ? v - B : v) + (i ? top : -top);
+    };
+#pragma unroll
+    for (int e = 0; e < F::R1; e++) {
+        lo[e] = at((int)threadIdx.x + e * F::T);
+        hi[e] = at(F::C + (int)threadIdx.x + e * F::T);
+    }
+}
+
+// out <- the spectrum (modulus mod) of the limbs, [element][group].
+template <class F>
+__device__ void spectrum(const View &w, const Tab &tab, int mod, const int *lo, const int *hi, Cplx *out) {
+    const Cplx *t[3] = {tab.t[mod][0], tab.t[mod][1], tab.t[mod][2]};
+    if (mod) first_pass<F, 1>(w.A, lo, hi);
+    else first_pass<F, 0>(w.A, lo, hi);
+    fwd_inner<F>(w.A, t);
+    mid<F>(w.A, t[F::NPASS - 2], MID_STORE, nullptr, out);
+}
+
+}  // namespace fp
+}  // namespace mr
+}  // namespace pfb

@@ -16,6 +16,7 @@
 #include "common.cuh"
 #include "lucas_host.h"
 #include "mr_device.cuh"
+#include "mr_fft.h"
 #include "mr_tables_host.h"
 #include "pfb_mr.h"
 
@@ -33,6 +34,7 @@ struct pfb_mr {
     uint32_t *d_tw = nullptr;
     uint32_t *d_wide = nullptr;
     Twiddles tw{};
+    fp::Engine fe;
     // persistent-kernel parameters per transform length (pfb_mr_autotune):
     // steps of one candidate per quantum, steps per launch
     int quantum[LOG_LMAX + 1];
@@ -88,6 +90,7 @@ extern "C" int pfb_mr_create(pfb_mr_t **out, int device) {
         if (ce != cudaSuccess) rc = pfb::cuda_fail(ce, "stream", __FILE__, __LINE__);
     }
     if (!rc) rc = build_tables(e);
+    if (!rc) rc = fp::engine_create(e->fe);
     if (!rc) {
         const int mx = (int)std::max(smem_bytes(LOG_LCTA), smem_bytes(LOG_LSEQ));
         ce = cudaFuncSetAttribute(persist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
@@ -98,6 +101,8 @@ extern "C" int pfb_mr_create(pfb_mr_t **out, int device) {
     if (rc) {
         if (e->stream) cudaStreamDestroy(e->stream);
         cudaFree(e->d_tw);
+        cudaFree(e->d_wide);
+        fp::engine_free(e->fe);
         delete e;
         return rc;
     }
@@ -114,6 +119,7 @@ extern "C" void pfb_mr_destroy(pfb_mr_t *e) {
     }
     cudaFree(e->d_tw);
     cudaFree(e->d_wide);
+    fp::engine_free(e->fe);
     delete e;
 }
 
@@ -154,28 +160,104 @@ Layout layout_for(int logl, size_t exp_words, bool lucas = false, bool raw = fal
     return l;
 }
 
-Layout layout_for(const HostPrep &hp, bool lucas) { return layout_for(hp.logl, hp.exp.size(), lucas); }
+// Layout of a candidate of the floating-point engine: n = 2 C digits, spectra
+// of C points (4 words each).
+Layout layout_fp(int cls, size_t exp_words) {
+    const size_t C = (size_t)fp::class_points(cls), n = 2 * C;
+    Layout l{};
+    size_t o = 0;
+    auto take = [&](size_t words) {
+        const size_t at = o;
+        o += (words + 63) & ~(size_t)63;
+        return at;
+    };
+    l.x = take(n);
+    l.res = take(n);
+    l.nn = take(4 * C);
+    l.nh = take(4 * C);
+    l.npl = take(n);
+    l.nl = take(n);
+    l.exp = take(exp_words);
+    l.total = o;
+    return l;
+}
+
+Layout layout_for(const HostPrep &hp, bool lucas) {
+    return hp.fpc ? layout_fp(hp.fpc - 1, hp.exp.size()) : layout_for(hp.logl, hp.exp.size(), lucas);
+}
+
+// Bits of a digit of a candidate's x0, npl, nl and residue.
+int digit_bits(const HostPrep &hp) { return hp.fpc ? hp.fbits : LIMB_BITS; }
+
+// The unfinished candidates by engine: the integer engine's count, and per
+// length class of the floating-point engine a run of `order` (job indices).
+struct ClassRuns {
+    int n_int = 0;
+    int first[fp::kClasses] = {}, count[fp::kClasses] = {};
+    std::vector<int> order;
+    template <class Live, class Fpc>
+    void build(int n, Live live, Fpc fpc) {
+        n_int = 0;
+        order.clear();
+        for (int i = 0; i < n; i++) n_int += live(i) && !fpc(i);
+        for (int c = 0; c < fp::kClasses; c++) {
+            first[c] = (int)order.size();
+            for (int i = 0; i < n; i++)
+                if (live(i) && fpc(i) == c + 1) order.push_back(i);
+            count[c] = (int)order.size() - first[c];
+        }
+    }
+};
+
+// Device scratch (points) of one launch of every class' persistent kernel,
+// and where a class' part begins.
+size_t fp_scratch_points(const pfb_mr *e, const int *count, size_t *begin) {
+    size_t o = 0;
+    for (int c = 0; c < fp::kClasses; c++) {
+        begin[c] = o;
+        if (count[c]) o += fp::scratch_points(c) * fp::persist_launch(e->fe, c, count[c], e->num_sms).grid.x;
+    }
+    return o;
+}
+
+// Quanta of one launch of a class: jobs that each have a CTA of their own run
+// their whole chunk in one quantum.
+void fp_quanta(const pfb_mr *e, int cls, int n, long long chunk, int tuned, int *quantum, unsigned *total) {
+    const int ctas = (int)fp::persist_launch(e->fe, cls, n, e->num_sms).grid.x;
+    *quantum = (int)(n <= ctas ? chunk : std::min<long long>(chunk, tuned));
+    *total = (unsigned)std::min<long long>((long long)n * ((chunk + *quantum - 1) / *quantum), 0x7fffffffll);
+}
 
 // Slot layout of the server: the exponent region sized for the longest
 // modulus of the length class, so that slots of one class are interchangeable.
-Layout slot_layout(int logl) {
-    const size_t H = (size_t)1 << (logl - 1);
-    return layout_for(logl, (LIMB_BITS * H + 31) / 32 + 1);
+// The length class is the transform length's logarithm, or for the
+// floating-point engine kFpKey + its class.
+constexpr int kFpKey = 64;
+int slot_key(const HostPrep &hp) { return hp.fpc ? kFpKey + hp.fpc - 1 : hp.logl; }
+Layout slot_layout(int key) {
+    if (key >= kFpKey) {
+        const int cls = key - kFpKey;
+        return layout_fp(cls, ((size_t)fp::limb_bits(cls) * 2 * fp::class_points(cls) + 31) / 32 + 1);
+    }
+    const size_t H = (size_t)1 << (key - 1);
+    return layout_for(key, (LIMB_BITS * H + 31) / 32 + 1);
 }
 
+// fft: candidates that the floating-point engine can hold are set up for it.
 void prep_all(const pfb_mr_number_t *nums, int n, uint32_t base, int mode, const pfb_mr_number_t *exps,
-              std::vector<HostPrep> &hp) {
+              std::vector<HostPrep> &hp, bool fft) {
     hp.resize(n);
     const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
     const int nt = (int)std::min<unsigned>(hw, (unsigned)std::max(1, n));
     if (nt <= 1 || n < 4) {
-        for (int i = 0; i < n; i++) host_prep(nums[i], base, mode, exps ? exps + i : nullptr, hp[i]);
+        for (int i = 0; i < n; i++) host_prep(nums[i], base, mode, exps ? exps + i : nullptr, hp[i], fft);
         return;
     }
     std::vector<std::thread> th;
     for (int t = 0; t < nt; t++)
         th.emplace_back([&, t]() {
-            for (int i = t; i < n; i += nt) host_prep(nums[i], base, mode, exps ? exps + i : nullptr, hp[i]);
+            for (int i = t; i < n; i += nt)
+                host_prep(nums[i], base, mode, exps ? exps + i : nullptr, hp[i], fft);
         });
     for (auto &x : th) x.join();
 }
@@ -190,7 +272,11 @@ struct pfb_mr_batch {
     uint8_t *d_arena = nullptr;
     JobDev *d_jobs = nullptr;
     int *d_locks = nullptr;           // [n] per-candidate locks of the persistent kernel
-    unsigned int *d_counter = nullptr;  // quanta handed out in the current launch
+    unsigned int *d_counter = nullptr;  // quanta handed out in the current launch: integer engine, then per class
+    ClassRuns runs;
+    int *d_order = nullptr;             // runs.order
+    fp::Cplx *d_scratch = nullptr;      // x^2's spectra, per CTA (classes that need it)
+    size_t scratch_begin[fp::kClasses] = {};
     LucasDev *d_lucas = nullptr;        // [n] (strong Lucas batches only)
     std::vector<HostPrep> hp;
     std::vector<JobDev> jobs;
@@ -225,7 +311,7 @@ int chunk_graph(pfb_mr_batch *b, long long chunk, int quantum, cudaGraphExec_t *
     int *locks = b->d_locks;
     unsigned int *counter = b->d_counter;
     const long long qpj = (chunk + quantum - 1) / quantum;
-    unsigned int total = (unsigned int)std::min<long long>((long long)b->n * qpj, 0x7fffffffll);
+    unsigned int total = (unsigned int)std::min<long long>((long long)b->runs.n_int * qpj, 0x7fffffffll);
     Twiddles tw = b->e->tw;
     void *args[] = {&jobs, &n, &locks, &counter, &total, &q, &tw};
     cudaGraph_t graph = nullptr;
@@ -234,18 +320,40 @@ int chunk_graph(pfb_mr_batch *b, long long chunk, int quantum, cudaGraphExec_t *
     mp.dst = counter;
     mp.value = 0;
     mp.elementSize = sizeof(unsigned int);
-    mp.width = 1;
+    mp.width = 1 + fp::kClasses;
     mp.height = 1;
-    cudaKernelNodeParams kp{};
-    kp.func = (void *)persist_kernel;
-    kp.gridDim = dim3((unsigned)std::min(b->n, std::max(1, b->e->num_sms)));
-    kp.blockDim = dim3(THREADS);
-    kp.sharedMemBytes = (unsigned)smem_bytes(b->maxlog);
-    kp.kernelParams = args;
     cudaGraphNode_t n_mem = nullptr, n_ker = nullptr;
     cudaGraphExec_t exec = nullptr;
     cudaError_t ce = cudaGraphAddMemsetNode(&n_mem, graph, nullptr, 0, &mp);
-    if (ce == cudaSuccess) ce = cudaGraphAddKernelNode(&n_ker, graph, &n_mem, 1, &kp);
+    if (ce == cudaSuccess && b->runs.n_int) {
+        cudaKernelNodeParams kp{};
+        kp.func = (void *)persist_kernel;
+        kp.gridDim = dim3((unsigned)std::min(b->runs.n_int, std::max(1, b->e->num_sms)));
+        kp.blockDim = dim3(THREADS);
+        kp.sharedMemBytes = (unsigned)smem_bytes(b->maxlog);
+        kp.kernelParams = args;
+        ce = cudaGraphAddKernelNode(&n_ker, graph, &n_mem, 1, &kp);
+    }
+    // the length classes' kernels side by side, the longest numbers first
+    for (int c = fp::kClasses - 1; c >= 0 && ce == cudaSuccess; c--) {
+        int nc = b->runs.count[c], qc = 0;
+        if (!nc) continue;
+        unsigned tc = 0;
+        fp_quanta(b->e, c, nc, chunk, quantum, &qc, &tc);
+        const fp::Launch l = fp::persist_launch(b->e->fe, c, nc, b->e->num_sms);
+        const int *order = b->d_order + b->runs.first[c];
+        unsigned int *cnt = counter + 1 + c;
+        fp::Tab tab = b->e->fe.tab[c];
+        fp::Cplx *scratch = b->d_scratch + b->scratch_begin[c];
+        void *fa[] = {&jobs, &order, &nc, &locks, &cnt, &tc, &qc, &tab, &scratch};
+        cudaKernelNodeParams kp{};
+        kp.func = l.func;
+        kp.gridDim = l.grid;
+        kp.blockDim = l.block;
+        kp.sharedMemBytes = (unsigned)l.smem;
+        kp.kernelParams = fa;
+        ce = cudaGraphAddKernelNode(&n_ker, graph, &n_mem, 1, &kp);
+    }
     if (ce == cudaSuccess) ce = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
     if (ce != cudaSuccess) return pfb::cuda_fail(ce, "chunk graph", __FILE__, __LINE__);
@@ -266,21 +374,24 @@ int batch_build(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base, in
     b->e = e;
     b->n = n;
     b->mode = mode;
-    prep_all(nums, n, base, mode, exps, b->hp);
+    prep_all(nums, n, base, mode, exps, b->hp, true);
     std::vector<Layout> lay(n);
     size_t total = 0;
     for (int i = 0; i < n; i++) {
         if (!b->hp[i].ok || b->hp[i].decided >= 0) continue;
         lay[i] = layout_for(b->hp[i], mode == 2);
         total += lay[i].total;
-        b->maxlog = std::max(b->maxlog, b->hp[i].logl);
+        b->maxlog = std::max(b->maxlog, b->hp[i].logl);  // (by size: also for the floating-point engine)
         b->max_steps = std::max(b->max_steps, (long long)b->hp[i].cursor + 2 + b->hp[i].s);
         b->n_ok++;
     }
     const size_t job_bytes = ((size_t)n * sizeof(JobDev) + 255) & ~(size_t)255;
     const size_t lock_bytes = ((size_t)n * sizeof(int) + 256 + 255) & ~(size_t)255;
     const size_t lucas_bytes = mode == 2 ? (((size_t)n * sizeof(LucasDev) + 255) & ~(size_t)255) : 0;
-    const size_t need = job_bytes + lock_bytes + lucas_bytes + total * sizeof(uint32_t);
+    b->runs.build(n, [&](int i) { return b->hp[i].ok && b->hp[i].decided < 0; }, [&](int i) { return b->hp[i].fpc; });
+    const size_t order_bytes = (b->runs.order.size() * sizeof(int) + 255) & ~(size_t)255;
+    const size_t scratch_bytes = fp_scratch_points(e, b->runs.count, b->scratch_begin) * sizeof(fp::Cplx);
+    const size_t need = job_bytes + lock_bytes + lucas_bytes + order_bytes + scratch_bytes + total * sizeof(uint32_t);
     if (cudaMalloc(&b->d_arena, need) != cudaSuccess) {
         cudaGetLastError();
         pfb::set_error("pfb_mr: cannot allocate %zu bytes of device memory", need);
@@ -294,7 +405,9 @@ int batch_build(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base, in
         b->d_lucas = (LucasDev *)(b->d_arena + job_bytes + lock_bytes);
         b->lucas.assign(n, LucasDev{});
     }
-    uint32_t *d_words = (uint32_t *)(b->d_arena + job_bytes + lock_bytes + lucas_bytes);
+    b->d_order = (int *)(b->d_arena + job_bytes + lock_bytes + lucas_bytes);
+    b->d_scratch = (fp::Cplx *)(b->d_arena + job_bytes + lock_bytes + lucas_bytes + order_bytes);
+    uint32_t *d_words = (uint32_t *)(b->d_arena + job_bytes + lock_bytes + lucas_bytes + order_bytes + scratch_bytes);
     if (cudaMemsetAsync(b->d_locks, 0, lock_bytes, e->stream) != cudaSuccess) {
         batch_free(b);
         return pfb::cuda_fail(cudaGetLastError(), "lock reset", __FILE__, __LINE__);
@@ -320,8 +433,10 @@ int batch_build(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base, in
         j.npl = w + l.npl;
         j.nl = w + l.nl;
         j.exp = w + l.exp;
-        if (h.logl > LOG_LCTA) j.ybuf = w + l.yb;
+        if (!h.fpc && h.logl > LOG_LCTA) j.ybuf = w + l.yb;
         j.logl = h.logl;
+        j.fpc = h.fpc;
+        j.fbits = h.fbits;
         j.cursor = h.cursor;
         j.extra = mode >= 1 ? h.s - 1 : 0;
         j.phase = 0;
@@ -358,7 +473,15 @@ int batch_build(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base, in
     if (!rc && ce == cudaSuccess && mode == 2)
         ce = cudaMemcpyAsync(b->d_lucas, b->lucas.data(), n * sizeof(LucasDev), cudaMemcpyHostToDevice, e->stream);
     if (!rc && ce != cudaSuccess) rc = pfb::cuda_fail(ce, "job upload", __FILE__, __LINE__);
-    if (!rc && b->n_ok) {
+    if (!rc && !b->runs.order.empty()) {
+        ce = cudaMemcpyAsync(b->d_order, b->runs.order.data(), b->runs.order.size() * sizeof(int),
+                             cudaMemcpyHostToDevice, e->stream);
+        for (int c = 0; c < fp::kClasses && ce == cudaSuccess; c++)
+            if (b->runs.count[c])
+                ce = fp::prep(e->fe, c, b->d_jobs, b->d_order + b->runs.first[c], b->runs.count[c], e->stream);
+        if (ce != cudaSuccess) rc = pfb::cuda_fail(ce, "fft_prep_kernel", __FILE__, __LINE__);
+    }
+    if (!rc && b->runs.n_int) {
         prep_kernel<<<n, THREADS, smem_bytes(b->maxlog), e->stream>>>(b->d_jobs, nullptr, e->tw);
         ce = cudaGetLastError();
         if (ce != cudaSuccess) rc = pfb::cuda_fail(ce, "prep_kernel", __FILE__, __LINE__);
@@ -433,7 +556,7 @@ int batch_results(pfb_mr_batch *b, int8_t *verdict, uint16_t *residue, int resid
             const size_t H = b->hp[i].x0.size();
             r22.resize(H);
             PFB_CUDA(cudaMemcpy(r22.data(), j.res, H * 4, cudaMemcpyDeviceToHost));
-            pfb::big::Words r = pfb::big::from_limbs(r22.data(), LIMB_BITS, H);
+            pfb::big::Words r = pfb::big::from_limbs(r22.data(), digit_bits(b->hp[i]), H);
             pfb::big::to_u16(r, residue + (size_t)i * residue_stride, (size_t)residue_stride);
         }
     }
@@ -716,6 +839,13 @@ struct pfb_mr_server {
     int *d_list = nullptr;
     uint8_t *d_table_mem = nullptr;
     std::vector<JobDev> jobs;
+    ClassRuns runs;               // resident candidates by engine and class
+    int *d_order = nullptr;       // runs.order
+    bool runs_stale = true;
+    uint8_t *d_scratch = nullptr; // x^2's spectra, per CTA
+    size_t scratch_bytes = 0;
+    cudaStream_t side[fp::kClasses] = {};  // classes run side by side
+    cudaEvent_t fork = nullptr, join[fp::kClasses] = {};
     std::vector<SrvSlot> slots;
     std::map<int, std::vector<uint8_t *>> pool;  // free slot memory by transform length
     size_t bytes_in_use = 0, bytes_owned = 0;
@@ -773,7 +903,7 @@ void srv_prep_worker(pfb_mr_server *s) {
             s->preparing++;
         }
         pfb_mr_number_t num{r.limbs.data(), (int)r.limbs.size()};
-        host_prep(num, s->cfg.base, 1, nullptr, r.hp);
+        host_prep(num, s->cfg.base, 1, nullptr, r.hp, true);
         {
             std::lock_guard<std::mutex> lk(s->mu);
             s->preparing--;
@@ -809,7 +939,7 @@ int srv_admit(pfb_mr_server *s, std::vector<int> &admitted) {
                     break;
                 }
             if (free_slot < 0) break;
-            const int lg = s->prepared.front().hp.logl;
+            const int lg = slot_key(s->prepared.front().hp);
             const size_t need = slot_bytes(lg);
             const bool pooled = !s->pool[lg].empty();
             if (s->cfg.hbm_budget_bytes && !pooled && s->bytes_owned + need > s->cfg.hbm_budget_bytes) {
@@ -905,7 +1035,7 @@ int srv_admit(pfb_mr_server *s, std::vector<int> &admitted) {
         }
         // fill the job and upload its inputs
         const HostPrep &h = sl.req.hp;
-        const Layout l = slot_layout(h.logl);
+        const Layout l = slot_layout(sl.logl);
         uint32_t *w = (uint32_t *)sl.mem;
         JobDev &j = s->jobs[admitted.back()];
         memset(&j, 0, sizeof(j));
@@ -916,8 +1046,10 @@ int srv_admit(pfb_mr_server *s, std::vector<int> &admitted) {
         j.npl = w + l.npl;
         j.nl = w + l.nl;
         j.exp = w + l.exp;
-        if (h.logl > LOG_LCTA) j.ybuf = w + l.yb;
+        if (!h.fpc && h.logl > LOG_LCTA) j.ybuf = w + l.yb;
         j.logl = h.logl;
+        j.fpc = h.fpc;
+        j.fbits = h.fbits;
         j.cursor = h.cursor;
         j.extra = h.s - 1;
         j.phase = 0;
@@ -932,13 +1064,30 @@ int srv_admit(pfb_mr_server *s, std::vector<int> &admitted) {
         PFB_CUDA(cudaStreamSynchronize(s->stream));  // host staging is freed below / reused
     }
     if (!admitted.empty()) {
-        PFB_CUDA(cudaMemcpyAsync(s->d_list, admitted.data(), admitted.size() * sizeof(int), cudaMemcpyHostToDevice,
-                                 s->stream));
+        // d_list: the integer engine's candidates, then each class'
+        ClassRuns adm;
+        adm.build((int)admitted.size(), [](int) { return true; },
+                  [&](int i) { return s->slots[admitted[i]].req.hp.fpc; });
+        std::vector<int> list;
         int maxlog = LOG_LMIN;
-        for (int i : admitted) maxlog = std::max(maxlog, s->slots[i].logl);
-        prep_kernel<<<(int)admitted.size(), THREADS, smem_bytes(maxlog), s->stream>>>(s->d_jobs, s->d_list, s->e->tw);
-        PFB_CUDA(cudaGetLastError());
+        for (int i : admitted)
+            if (!s->slots[i].req.hp.fpc) {
+                list.push_back(i);
+                maxlog = std::max(maxlog, s->slots[i].logl);
+            }
+        for (int i : adm.order) list.push_back(admitted[i]);
+        PFB_CUDA(cudaMemcpyAsync(s->d_list, list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice,
+                                 s->stream));
+        if (adm.n_int) {
+            prep_kernel<<<adm.n_int, THREADS, smem_bytes(maxlog), s->stream>>>(s->d_jobs, s->d_list, s->e->tw);
+            PFB_CUDA(cudaGetLastError());
+        }
+        for (int c = 0; c < fp::kClasses; c++)
+            if (adm.count[c])
+                PFB_CUDA(fp::prep(s->e->fe, c, s->d_jobs, s->d_list + adm.n_int + adm.first[c], adm.count[c],
+                                  s->stream));
         PFB_CUDA(cudaStreamSynchronize(s->stream));
+        s->runs_stale = true;
         for (int i : admitted) {  // the set-up inputs are on the device now
             HostPrep &h = s->slots[i].req.hp;
             std::vector<uint32_t>().swap(h.npl);
@@ -966,7 +1115,7 @@ void srv_retire(pfb_mr_server *s) {
             const size_t H = sl.req.hp.x0.size();
             r22.resize(H);
             if (cudaMemcpy(r22.data(), s->jobs[i].res, H * 4, cudaMemcpyDeviceToHost) == cudaSuccess) {
-                pfb::big::Words r = pfb::big::from_limbs(r22.data(), LIMB_BITS, H);
+                pfb::big::Words r = pfb::big::from_limbs(r22.data(), digit_bits(sl.req.hp), H);
                 pfb::big::to_u16(r, sl.req.residue_out, (size_t)sl.req.residue_cap);
             }
         }
@@ -976,6 +1125,7 @@ void srv_retire(pfb_mr_server *s) {
         s->pool[sl.logl].push_back(sl.mem);
         sl.mem = nullptr;
         sl.busy = false;
+        s->runs_stale = true;
         s->bytes_in_use -= bytes;
         s->resident--;
         s->n_completed++;
@@ -985,6 +1135,81 @@ void srv_retire(pfb_mr_server *s) {
     }
 }
 
+// Enqueues one launch of the persistent kernel per engine and length class
+// with residents, side by side, and joins them on the server's stream.
+int srv_launch(pfb_mr_server *s) {
+    pfb_mr *e = s->e;
+    const int cap = (int)s->slots.size();
+    if (s->runs_stale) {
+        s->runs.build(cap, [&](int i) { return s->slots[i].busy; }, [&](int i) { return s->jobs[i].fpc; });
+        if (!s->runs.order.empty())
+            PFB_CUDA(cudaMemcpyAsync(s->d_order, s->runs.order.data(), s->runs.order.size() * sizeof(int),
+                                     cudaMemcpyHostToDevice, s->stream));
+        s->runs_stale = false;
+    }
+    size_t begin[fp::kClasses];
+    const size_t need = fp_scratch_points(e, s->runs.count, begin) * sizeof(fp::Cplx);
+    if (need > s->scratch_bytes) {
+        PFB_CUDA(cudaStreamSynchronize(s->stream));
+        cudaFree(s->d_scratch);
+        s->d_scratch = nullptr;
+        s->scratch_bytes = 0;
+        PFB_CUDA(cudaMalloc(&s->d_scratch, need));
+        s->scratch_bytes = need;
+    }
+    PFB_CUDA(cudaMemsetAsync(s->d_counter, 0, (1 + fp::kClasses) * sizeof(unsigned int), s->stream));
+    const int quantum = std::min(64, s->cfg.chunk_steps);
+    bool forked = false;
+    if (s->runs.n_int) {
+        const long long qpj = (s->cfg.chunk_steps + quantum - 1) / quantum;
+        int maxlog = LOG_LMIN;
+        for (auto &sl : s->slots)
+            if (sl.busy && sl.logl < kFpKey) maxlog = std::max(maxlog, sl.logl);
+        if (!s->runs.order.empty()) {
+            PFB_CUDA(cudaEventRecord(s->fork, s->stream));
+            forked = true;
+        }
+        persist_kernel<<<std::min(s->runs.n_int, std::max(1, e->num_sms)), THREADS, smem_bytes(maxlog), s->stream>>>(
+            s->d_jobs, cap, s->d_locks, s->d_counter, (unsigned int)(s->runs.n_int * qpj), quantum, e->tw);
+        PFB_CUDA(cudaGetLastError());
+    }
+    int classes = 0;
+    for (int c = 0; c < fp::kClasses; c++) classes += s->runs.count[c] > 0;
+    if (classes > 1 && !forked) {
+        PFB_CUDA(cudaEventRecord(s->fork, s->stream));
+        forked = true;
+    }
+    for (int c = fp::kClasses - 1; c >= 0; c--) {
+        int nc = s->runs.count[c], qc = 0;
+        if (!nc) continue;
+        cudaStream_t st = s->stream;
+        if (forked) {
+            if (!s->side[c]) {
+                PFB_CUDA(cudaStreamCreateWithFlags(&s->side[c], cudaStreamNonBlocking));
+                PFB_CUDA(cudaEventCreateWithFlags(&s->join[c], cudaEventDisableTiming));
+            }
+            st = s->side[c];
+            PFB_CUDA(cudaStreamWaitEvent(st, s->fork, 0));
+        }
+        unsigned tc = 0;
+        fp_quanta(e, c, nc, s->cfg.chunk_steps, quantum, &qc, &tc);
+        const fp::Launch l = fp::persist_launch(e->fe, c, nc, e->num_sms);
+        const int *order = s->d_order + s->runs.first[c];
+        unsigned int *cnt = s->d_counter + 1 + c;
+        fp::Tab tab = e->fe.tab[c];
+        fp::Cplx *scratch = (fp::Cplx *)s->d_scratch + begin[c];
+        void *fa[] = {&s->d_jobs, &order, &nc, &s->d_locks, &cnt, &tc, &qc, &tab, &scratch};
+        PFB_CUDA(cudaLaunchKernel(l.func, l.grid, l.block, fa, l.smem, st));
+    }
+    if (forked)
+        for (int c = 0; c < fp::kClasses; c++)
+            if (s->runs.count[c]) {
+                PFB_CUDA(cudaEventRecord(s->join[c], s->side[c]));
+                PFB_CUDA(cudaStreamWaitEvent(s->stream, s->join[c], 0));
+            }
+    return PFB_OK;
+}
+
 void srv_driver(pfb_mr_server *s) {
     if (cudaSetDevice(s->e->device) != cudaSuccess) {
         s->error = PFB_E_CUDA;
@@ -992,7 +1217,6 @@ void srv_driver(pfb_mr_server *s) {
     }
     std::vector<int> admitted;
     const int cap = (int)s->slots.size();
-    const int grid_max = std::max(1, s->e->num_sms);
     while (true) {
         {
             std::unique_lock<std::mutex> lk(s->mu);
@@ -1011,16 +1235,9 @@ void srv_driver(pfb_mr_server *s) {
             res_now = s->resident;
         }
         if (res_now == 0) continue;
-        // one launch: every resident candidate advances about chunk_steps steps
-        const int quantum = std::min(64, s->cfg.chunk_steps);
-        const long long qpj = (s->cfg.chunk_steps + quantum - 1) / quantum;
-        int maxlog = LOG_LMIN;
-        for (auto &sl : s->slots)
-            if (sl.busy) maxlog = std::max(maxlog, sl.logl);
-        cudaMemsetAsync(s->d_counter, 0, sizeof(unsigned int), s->stream);
-        persist_kernel<<<std::min(res_now, grid_max), THREADS, smem_bytes(maxlog), s->stream>>>(
-            s->d_jobs, cap, s->d_locks, s->d_counter, (unsigned int)(res_now * qpj), quantum, s->e->tw);
-        if (cudaGetLastError() != cudaSuccess ||
+        // one launch per engine and class: every resident candidate advances
+        // about chunk_steps steps
+        if (srv_launch(s) != PFB_OK ||
             cudaMemcpyAsync(s->jobs.data(), s->d_jobs, cap * sizeof(JobDev), cudaMemcpyDeviceToHost, s->stream) !=
                 cudaSuccess ||
             cudaStreamSynchronize(s->stream) != cudaSuccess) {
@@ -1057,7 +1274,7 @@ extern "C" int pfb_mr_server_create(pfb_mr_t *e, const pfb_mr_server_config_t *c
     PFB_CUDA(cudaSetDevice(e->device));
     const size_t job_bytes = ((size_t)cap * sizeof(JobDev) + 255) & ~(size_t)255;
     const size_t int_bytes = ((size_t)cap * sizeof(int) + 255) & ~(size_t)255;
-    if (cudaMalloc(&s->d_table_mem, job_bytes + 2 * int_bytes + 256) != cudaSuccess) {
+    if (cudaMalloc(&s->d_table_mem, job_bytes + 3 * int_bytes + 256) != cudaSuccess) {
         cudaGetLastError();
         delete s;
         pfb::set_error("pfb_mr_server_create: cannot allocate the job table");
@@ -1066,17 +1283,20 @@ extern "C" int pfb_mr_server_create(pfb_mr_t *e, const pfb_mr_server_config_t *c
     s->d_jobs = (JobDev *)s->d_table_mem;
     s->d_locks = (int *)(s->d_table_mem + job_bytes);
     s->d_list = (int *)(s->d_table_mem + job_bytes + int_bytes);
-    s->d_counter = (unsigned int *)(s->d_table_mem + job_bytes + 2 * int_bytes);
+    s->d_order = (int *)(s->d_table_mem + job_bytes + 2 * int_bytes);
+    s->d_counter = (unsigned int *)(s->d_table_mem + job_bytes + 3 * int_bytes);
     s->jobs.assign(cap, JobDev{});
     for (auto &j : s->jobs) j.phase = 3;
     s->slots.resize(cap);
     int rc = PFB_OK;
     cudaError_t ce = cudaStreamCreateWithFlags(&s->stream, cudaStreamNonBlocking);
+    if (ce == cudaSuccess) ce = cudaEventCreateWithFlags(&s->fork, cudaEventDisableTiming);
     if (ce == cudaSuccess) ce = cudaMemcpy(s->d_jobs, s->jobs.data(), cap * sizeof(JobDev), cudaMemcpyHostToDevice);
     if (ce == cudaSuccess) ce = cudaMemset(s->d_locks, 0, int_bytes);
     if (ce != cudaSuccess) rc = pfb::cuda_fail(ce, "server set-up", __FILE__, __LINE__);
     if (rc) {
         cudaFree(s->d_table_mem);
+        if (s->fork) cudaEventDestroy(s->fork);
         if (s->stream) cudaStreamDestroy(s->stream);
         delete s;
         return rc;
@@ -1175,6 +1395,12 @@ extern "C" void pfb_mr_server_destroy(pfb_mr_server_t *s) {
         if (sl.mem) cudaFree(sl.mem);
     for (auto &kv : s->pool)
         for (uint8_t *m : kv.second) cudaFree(m);
+    cudaFree(s->d_scratch);
+    cudaEventDestroy(s->fork);
+    for (int c = 0; c < fp::kClasses; c++) {
+        if (s->side[c]) cudaStreamDestroy(s->side[c]);
+        if (s->join[c]) cudaEventDestroy(s->join[c]);
+    }
     cudaFree(s->d_table_mem);
     cudaStreamDestroy(s->stream);
     delete s;
@@ -1249,7 +1475,7 @@ extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs
     std::vector<pfb_mr_number_t> nums(n_batch);
     for (int i = 0; i < n_batch; i++) nums[i] = pfb_mr_number_t{n16.data() + (size_t)i * n_limbs, n_limbs};
     // base 2 sizes R > 64 N: products of two reduced operands stay below 2N after REDC
-    prep_all(nums.data(), n_batch, 2u, 1, nullptr, c->hp);
+    prep_all(nums.data(), n_batch, 2u, 1, nullptr, c->hp, false);
     std::vector<Layout> lay(n_batch);
     size_t words = 0;
     for (int i = 0; i < n_batch; i++) {

@@ -9,40 +9,12 @@
 
 #include "common.cuh"
 #include "mr_device.cuh"
+#include "mr_job.cuh"
 
 namespace pfb {
 namespace mr {
 
 __constant__ CrtConsts c_crt;
-
-// State of one candidate in device memory.
-struct JobDev {
-    uint32_t *x;          // H limbs: Montgomery residue (working value)
-    uint32_t *res;        // H limbs: canonical residue a^E mod N (output)
-    uint32_t *nn;         // [2][H] negacyclic NTT_H(N''), N'' = -N^-1 mod (B^H + 1)
-    uint32_t *nh;         // [2][H] NTT_H(N)
-    const uint32_t *npl;  // H limbs of N'' (set-up input)
-    const uint32_t *nl;   // H limbs of N
-    const uint32_t *exp;  // exponent, 32-bit words, little-endian
-    uint32_t *ybuf;       // H + H/32 words (L = 2^15 only: the residue Y, padded)
-    struct LucasDev *lucas;  // strong Lucas test (mode 2) only
-    int logl;
-    int cursor;   // next exponent bit (MSB first); phase 0 while >= 0
-    int extra;    // squarings left in phase 2 (s - 1 for a strong test)
-    int phase;    // 0 exponent loop, 1 first check, 2 squarings r < s, 3 done
-    uint32_t base;
-    int mode;     // 0 modular power only, 1 strong test, 2 strong Lucas test
-    int verdict;  // 1 probable prime, 0 composite
-    int steps;    // steps taken (diagnostics)
-};
-
-// Strong Lucas state of one candidate: H limbs each, Montgomery form: V_k,
-// V_(k+1), Q^k, a product, R mod N; gy the [2][L] spectrum of V_(k+1).
-struct LucasDev {
-    uint32_t *lv0, *lv1, *lqk, *lt, *lone, *gy;
-    int q;        // Selfridge Q = (1 - D) / 4
-    uint32_t lb;  // every stored value is < lb * N
-};
 
 // Shared memory: up to L = 2^LOG_LCTA both primes' length-L transforms (A0,
 // A1), the residue X and a second residue Y; at L = 2^15 three buffers of H
@@ -127,7 +99,7 @@ __device__ void prep_t(const Smem &sm, const JobDev &jb, const Twiddles &tw) {
 __global__ void __launch_bounds__(THREADS, 1) prep_kernel(JobDev *jobs, const int *list, Twiddles tw) {
     PFB_DYNAMIC_SMEM(uint32_t, raw);
     const JobDev jb = jobs[list ? list[blockIdx.x] : (int)blockIdx.x];
-    if (jb.phase == 3) return;
+    if (jb.phase == 3 || jb.fpc) return;
     Smem sm;
     uint32_t *Y;
     carve(raw, jb.logl, sm, Y, jb.ybuf);
@@ -427,7 +399,7 @@ persist_kernel(JobDev *jobs, int n, int *locks, unsigned int *counter, unsigned 
             if (q < total) {
                 for (int probe = 0; probe < n; probe++) {
                     const int j = (int)((q + (unsigned int)probe) % (unsigned int)n);
-                    if (__ldcg(&jobs[j].phase) == 3) continue;
+                    if (__ldcg(&jobs[j].phase) == 3 || __ldcg(&jobs[j].fpc)) continue;
                     if (atomicCAS(&locks[j], 0, 1) != 0) continue;
                     __threadfence();
                     if (__ldcg(&jobs[j].phase) != 3) {

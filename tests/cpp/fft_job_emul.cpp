@@ -1,0 +1,205 @@
+// Runs the floating-point Montgomery engine (fft_device.cuh, fft_kernels.cuh)
+// unchanged on the CPU, one candidate per CTA of cooperative fibers
+// (tests/cpp/emul/), with the engine's own host set-up (mr_prep_host.h) and
+// roots (fft_tables_host.h).  Input lines:
+//
+//   job mode base N [E]        whole test (mode 1) or base^E mod N (mode 0)
+//                              -> class bits verdict residue
+//   step cls bits dbl kind N   one squaring of limbs of a pattern: kind 0
+//                              all B/2 + 40, 1 all -(B/2 + 40), 2 alternating,
+//                              3 random signs, 4 random limbs (the top limbs
+//                              zero so that |x| < N)
+//                              -> x, result (signed hexadecimal), largest |limb|
+#include <functional>
+#include <iostream>
+#include <random>
+#include <sstream>
+#include <string>
+#include <vector>
+
+#include "mr_kernels.cuh"
+
+#include "fft_kernels.cuh"
+#include "fft_tables_host.h"
+#include "mr_prep_host.h"
+
+using namespace pfb::mr;
+using pfb::big::Words;
+
+static Words from_hex(const std::string &h) {
+    Words w;
+    size_t end = h.size();
+    while (end > 0) {
+        const size_t start = end >= 16 ? end - 16 : 0;
+        w.push_back(std::stoull(h.substr(start, end - start), nullptr, 16));
+        end = start;
+    }
+    pfb::big::trim(w);
+    return w;
+}
+
+static std::string to_hex(Words t) {
+    pfb::big::trim(t);
+    if (t.empty()) return "0";
+    std::string s;
+    char buf[24];
+    snprintf(buf, sizeof buf, "%llx", (unsigned long long)t.back());
+    s += buf;
+    for (size_t i = t.size() - 1; i-- > 0;) {
+        snprintf(buf, sizeof buf, "%016llx", (unsigned long long)t[i]);
+        s += buf;
+    }
+    return s;
+}
+
+// Signed value of limbs of b bits.
+static std::string limbs_hex(const std::vector<int> &l, int b) {
+    std::vector<uint32_t> d(l.size());
+    long long c = 0;
+    auto digits = [&](int sign) {
+        c = 0;
+        for (size_t i = 0; i < l.size(); i++) {
+            const long long v = (long long)sign * l[i] + c;
+            d[i] = (uint32_t)(v & ((1ll << b) - 1));
+            c = v >> b;
+        }
+    };
+    digits(1);
+    const bool neg = c < 0;
+    if (neg) digits(-1);
+    return (neg ? "-" : "") + to_hex(pfb::big::from_limbs(d.data(), b, d.size()));
+}
+
+template <class F>
+static fp::Tab tables(std::vector<fp::Cplx> &mem) {
+    size_t off[2][3] = {};
+    mem = fp::class_roots<F>(off);
+    fp::Tab t{};
+    for (int m = 0; m < 2; m++)
+        for (int p = 0; p < 3; p++) t.t[m][p] = mem.data() + off[m][p];
+    return t;
+}
+
+template <class F>
+static void run_job_cls(JobDev &j) {
+    std::vector<fp::Cplx> mem, scratch(F::SQS ? 1 : F::C);
+    const fp::Tab tab = tables<F>(mem);
+    const int list[1] = {0};
+    emu::run_grid(1, 1, F::T, [&] { fp::fft_prep_kernel<F>(&j, list, tab); }, F::smem());
+    int locks[1] = {0};
+    unsigned counter = 0;
+    for (int launch = 0; j.phase != 3 && launch < 1 << 20; launch++) {
+        counter = 0;
+        emu::run_grid(1, 1, F::T,
+                      [&] { fp::fft_persist_kernel<F>(&j, list, 1, locks, &counter, 8u, 64, tab, scratch.data()); },
+                      F::smem());
+    }
+}
+
+template <class F>
+static void run_step(int b, int dbl, int kind, const Words &N) {
+    const size_t n = F::N;
+    std::vector<fp::Cplx> mem, scratch(F::C), nn(F::C), nh(F::C);
+    const fp::Tab tab = tables<F>(mem);
+    Words inv;
+    if (!neg_inv_radix(N, n * b, inv)) {
+        std::cout << "none" << std::endl;
+        return;
+    }
+    std::vector<uint32_t> npl(n), nl(n);
+    pfb::big::to_limbs(inv, b, npl.data(), n);
+    pfb::big::to_limbs(N, b, nl.data(), n);
+    std::mt19937_64 rng(kind + 17);
+    std::vector<int> x(n, 0), y(n);
+    const int ext = (1 << (b - 1)) + 40;
+    const size_t used = pfb::big::bit_length(N) / b;  // |x| < N
+    for (size_t i = 0; i + 1 < used; i++)
+        x[i] = kind == 0 ? ext : kind == 1 ? -ext : kind == 2 ? (i & 1 ? ext : -ext)
+             : kind == 3 ? (rng() & 1 ? ext : -ext) : (int)(rng() % (2 * ext + 1)) - ext;
+    emu::run_grid(1, 1, F::T, [&] {
+        PFB_DYNAMIC_SMEM(unsigned char, raw);
+        fp::View w;
+        fp::carve<F>(raw, scratch.data(), w);
+        int lo[F::R1], hi[F::R1];
+        fp::balanced<F>(npl.data(), b, lo, hi);
+        fp::spectrum<F>(w, tab, 0, lo, hi, nn.data());
+        fp::balanced<F>(nl.data(), b, lo, hi);
+        fp::spectrum<F>(w, tab, 1, lo, hi, nh.data());
+        for (int e = 0; e < F::R1; e++) {
+            lo[e] = x[threadIdx.x + e * F::T];
+            hi[e] = x[F::C + threadIdx.x + e * F::T];
+        }
+        fp::step<F>(w, tab, nn.data(), nh.data(), b, true, dbl, lo, hi);
+        for (int e = 0; e < F::R1; e++) {
+            y[threadIdx.x + e * F::T] = lo[e];
+            y[F::C + threadIdx.x + e * F::T] = hi[e];
+        }
+    }, F::smem());
+    int big = 0;
+    for (int v : y) big = std::max(big, v < 0 ? -v : v);
+    std::cout << limbs_hex(x, b) << " " << limbs_hex(y, b) << " " << big << std::endl;
+}
+
+int main() {
+    fp::c_first = fp::first_roots();
+    std::string line;
+    while (std::getline(std::cin, line)) {
+        std::istringstream in(line);
+        std::string op, sn, se;
+        in >> op;
+        if (op == "step") {
+            int cls, b, dbl, kind;
+            in >> cls >> b >> dbl >> kind >> sn;
+            const Words N = from_hex(sn);
+            switch (cls) {
+#define PFB_CLS(F) \
+    case fp::F::ID: run_step<fp::F>(b, dbl, kind, N); break;
+                PFB_FP_CLASSES(PFB_CLS)
+#undef PFB_CLS
+            }
+            continue;
+        }
+        int mode = 1;
+        uint32_t base = 2;
+        in >> mode >> base >> sn >> se;
+        const Words N = from_hex(sn), E = from_hex(se);
+        std::vector<uint16_t> limbs(std::max<size_t>(1, (pfb::big::bit_length(N) + 15) / 16));
+        pfb::big::to_u16(N, limbs.data(), limbs.size());
+        std::vector<uint16_t> el(std::max<size_t>(1, (pfb::big::bit_length(E) + 15) / 16));
+        pfb::big::to_u16(E, el.data(), el.size());
+        const pfb_mr_number_t num{limbs.data(), (int)limbs.size()}, ex{el.data(), (int)el.size()};
+        HostPrep hp;
+        host_prep(num, base, mode, mode ? nullptr : &ex, hp, true);
+        if (!hp.ok || !hp.fpc) {
+            std::cout << hp.fpc << " 0 -1 0" << std::endl;
+            continue;
+        }
+        const size_t n = hp.x0.size();
+        std::vector<uint32_t> x = hp.x0, res(n), npl = hp.npl, nl = hp.nl, e = hp.exp;
+        std::vector<fp::Cplx> nn(n / 2), nh(n / 2);
+        JobDev j{};
+        j.x = x.data();
+        j.res = res.data();
+        j.nn = reinterpret_cast<uint32_t *>(nn.data());
+        j.nh = reinterpret_cast<uint32_t *>(nh.data());
+        j.npl = npl.data();
+        j.nl = nl.data();
+        j.exp = e.data();
+        j.logl = hp.logl;
+        j.fpc = hp.fpc;
+        j.fbits = hp.fbits;
+        j.cursor = hp.cursor;
+        j.extra = mode >= 1 ? hp.s - 1 : 0;
+        j.base = base;
+        j.mode = mode;
+        switch (hp.fpc - 1) {
+#define PFB_CLS(F) \
+    case fp::F::ID: run_job_cls<fp::F>(j); break;
+            PFB_FP_CLASSES(PFB_CLS)
+#undef PFB_CLS
+        }
+        std::cout << hp.fpc - 1 << " " << hp.fbits << " " << (j.phase == 3 ? j.verdict : -2) << " "
+                  << to_hex(pfb::big::from_limbs(res.data(), hp.fbits, n)) << std::endl;
+    }
+    return 0;
+}
