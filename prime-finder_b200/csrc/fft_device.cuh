@@ -54,42 +54,66 @@ struct alignas(16) Cplx {
 };
 
 // ---- length classes --------------------------------------------------------
-// C complex points, passes of radix R1, R2, R3, R4 (R4 = 1: three passes),
-// T = C / R1 threads: a thread holds one group of the first pass, and the
-// last inverse pass, the carries and the next first pass stay in registers.
-// SQS: x^2's spectrum waits in shared memory (else in global memory); PADL:
-// one unused point per 2^PADL in shared memory against bank conflicts of the
-// last pass.
-template <int ID_, int C_, int R1_, int R2_, int R3_, int R4_, bool SQS_, int MINB_>
+// C = 2^k or 3 2^k complex points, passes of radix R1 (with the factor 3), R2,
+// R3, R4 (R4 = 1: three passes), T threads.  Each holds one group of the first
+// pass (T = T1 = C / R1; the second half of a warp repeats the first when T1 =
+// 16): the last inverse pass, the carries and the next first pass stay in
+// registers.  SQS: x^2's spectrum waits in
+// shared memory, XSS: so do x's limbs (else both in global memory); PADL: one
+// unused point per 2^PADL in shared memory against bank conflicts of the last
+// pass.
+constexpr int kResident = 1024;
+template <int ID_, int C_, int R1_, int R2_, int R3_, int R4_, int T_, bool SQS_, bool XSS_, int MINB_>
 struct Cls {
-    static constexpr int ID = ID_, C = C_, R1 = R1_, R2 = R2_, R3 = R3_, R4 = R4_, T = C_ / R1_, N = 2 * C_;
-    static constexpr bool SQS = SQS_;
+    static constexpr int ID = ID_, C = C_, R1 = R1_, R2 = R2_, R3 = R3_, R4 = R4_, T = T_, T1 = C_ / R1_, N = 2 * C_;
+    static constexpr bool SQS = SQS_, XSS = XSS_;
     static constexpr int MINB = MINB_;
     static constexpr int NPASS = R4_ > 1 ? 4 : 3;
     static constexpr int RM = R4_ > 1 ? R4_ : R3_;  // radix of the middle sweep
     static constexpr int PADL = RM >= 16 ? 4 : 3;
     static constexpr int WARPS = T / 32;
-    static_assert(R1_ * R2_ * R3_ * R4_ == C_ && T % 32 == 0, "pass radices");
-    // bytes: points (padded), x limbs, boundary carries, flags, x^2's spectrum
+    // short numbers, whose steps are a chain of latencies: the roots and the
+    // spectra of N'' and N are copied to shared memory for a quantum
+    static constexpr bool RES = C_ <= kResident;
+    static constexpr int ROOTS = 2 * (R2_ / 2 * R1_ + R3_ / 2 * R1_ * R2_ + (R4_ > 1 ? R4_ / 2 * R1_ * R2_ * R3_ : 0));
+    static_assert(R1_ * R2_ * R3_ * R4_ == C_ && T % 32 == 0 && N % T == 0, "passes");
+    static_assert(T1 == T || (T1 == 16 && T == 32), "one group of the first pass per thread");
+    // shared memory: points (padded), x^2's spectrum, x's limbs, carries
+    // between warps, scratch words
     static constexpr int A_PTS = C_ + (C_ >> PADL);
     static constexpr size_t smem() {
-        return (size_t)A_PTS * 16 + (size_t)C_ * 8 + (size_t)2 * WARPS * R1_ * 8 + 256 + (SQS_ ? (size_t)C_ * 16 : 0);
+        return (size_t)A_PTS * 16 + (SQS_ ? (size_t)C_ * 16 : 0) + (XSS_ ? (size_t)C_ * 8 : 0) +
+               (size_t)2 * WARPS * R1_ * 8 + 256 + (RES ? (size_t)(2 * C_ + ROOTS) * 16 : 0);
     }
+    // points of global scratch per CTA
+    static constexpr size_t scratch() { return (SQS_ ? 0 : C_) + (XSS_ ? 0 : C_ / 2); }
 };
 
-constexpr int kClasses = 8;
-using Cls0 = Cls<0, 64, 2, 4, 8, 1, true, 8>;
-using Cls1 = Cls<1, 128, 4, 4, 8, 1, true, 8>;
-using Cls2 = Cls<2, 256, 4, 8, 8, 1, true, 8>;
-using Cls3 = Cls<3, 512, 8, 8, 8, 1, true, 6>;
-using Cls4 = Cls<4, 1024, 8, 16, 8, 1, true, 3>;
-using Cls5 = Cls<5, 2048, 16, 16, 8, 1, true, 2>;
-using Cls6 = Cls<6, 4096, 16, 16, 16, 1, true, 1>;
-using Cls7 = Cls<7, 8192, 16, 8, 8, 8, false, 1>;
-#define PFB_FP_CLASSES(F) F(Cls0) F(Cls1) F(Cls2) F(Cls3) F(Cls4) F(Cls5) F(Cls6) F(Cls7)
+constexpr int kClasses = 16;
+using Cls0 = Cls<0, 64, 2, 4, 8, 1, 32, true, true, 8>;
+using Cls1 = Cls<1, 96, 3, 4, 8, 1, 32, true, true, 8>;
+using Cls2 = Cls<2, 128, 4, 4, 8, 1, 32, true, true, 8>;
+using Cls3 = Cls<3, 192, 3, 8, 8, 1, 64, true, true, 8>;
+using Cls4 = Cls<4, 256, 4, 8, 8, 1, 64, true, true, 8>;
+using Cls5 = Cls<5, 384, 6, 8, 8, 1, 64, true, true, 6>;
+using Cls6 = Cls<6, 512, 8, 8, 8, 1, 64, true, true, 6>;
+using Cls7 = Cls<7, 768, 6, 16, 8, 1, 128, true, true, 4>;
+using Cls8 = Cls<8, 1024, 8, 16, 8, 1, 128, true, true, 3>;
+using Cls9 = Cls<9, 1536, 12, 8, 16, 1, 128, true, true, 2>;
+using Cls10 = Cls<10, 2048, 16, 16, 8, 1, 128, true, true, 2>;
+using Cls11 = Cls<11, 3072, 12, 16, 16, 1, 256, true, true, 1>;
+using Cls12 = Cls<12, 4096, 16, 16, 16, 1, 256, true, true, 1>;
+using Cls13 = Cls<13, 6144, 24, 16, 16, 1, 256, false, true, 1>;
+using Cls14 = Cls<14, 8192, 16, 8, 8, 8, 512, false, true, 1>;
+using Cls15 = Cls<15, 12288, 24, 8, 8, 8, 512, false, false, 1>;
+#define PFB_FP_CLASSES(F)                                                                                     \
+    F(Cls0) F(Cls1) F(Cls2) F(Cls3) F(Cls4) F(Cls5) F(Cls6) F(Cls7) F(Cls8) F(Cls9) F(Cls10) F(Cls11) F(Cls12) \
+        F(Cls13) F(Cls14) F(Cls15)
 
 inline int class_points(int cls) {
-    static const int c[kClasses] = {64, 128, 256, 512, 1024, 2048, 4096, 8192};
+#define PFB_CLS(F) F::C,
+    static const int c[kClasses] = {PFB_FP_CLASSES(PFB_CLS)};
+#undef PFB_CLS
     return c[cls];
 }
 
@@ -116,8 +140,11 @@ struct Tab {
 
 // The first pass' roots, the same for every length: entry q of a radix-16
 // group at the root of the tree.
+// (tree of binary levels), and for a radix 3 r group the root r and r^2 of
+// the ternary level, then for each child the roots of a radix-8 group.
 struct First {
     Cplx r[2][8];
+    Cplx t[2][2 + 3 * 4];
 };
 __constant__ First c_first;
 
@@ -229,10 +256,63 @@ __device__ __forceinline__ void inv_group(Cplx *v, const Cplx *tw) {
     }
 }
 
-template <int R>
+// A group of the first pass, radix 2^k or 3 2^k.  The ternary level takes
+// y^(3m) - r^3 to y^m - r, y^m - r z, y^m - r z^2, z = e^(2 pi i / 3).
+template <int R, int MOD>
+__device__ __forceinline__ void fwd_first(Cplx *v) {
+    if constexpr (R % 3 == 0) {
+        constexpr int Q = R / 3;
+        constexpr double H = 0.86602540378443864676;
+        const Cplx *w = c_first.t[MOD];
+#pragma unroll
+        for (int e = 0; e < Q; e++) {
+            const Cplx f = v[e], g = v[e + Q], h = v[e + 2 * Q];
+            const Cplx b{fma(w[0].re, g.re, -(w[0].im * g.im)), fma(w[0].re, g.im, w[0].im * g.re)};
+            const Cplx s{fma(-w[1].im, h.im, fma(w[1].re, h.re, b.re)), fma(w[1].re, h.im, fma(w[1].im, h.re, b.im))};
+            const Cplx d{fma(2.0, b.re, -s.re), fma(2.0, b.im, -s.im)};  // b - c
+            const double tr = fma(-0.5, s.re, f.re), ti = fma(-0.5, s.im, f.im);
+            v[e] = Cplx{f.re + s.re, f.im + s.im};
+            v[e + Q] = Cplx{fma(-H, d.im, tr), fma(H, d.re, ti)};
+            v[e + 2 * Q] = Cplx{fma(H, d.im, tr), fma(-H, d.re, ti)};
+        }
+        if constexpr (Q > 1) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) fwd_group<Q>(v + k * Q, w + 2 + 4 * k);
+        }
+    } else {
+        fwd_group<R>(v, c_first.r[MOD]);
+    }
+}
+
+template <int R, int MOD>
+__device__ __forceinline__ void inv_last(Cplx *v) {
+    if constexpr (R % 3 == 0) {
+        constexpr int Q = R / 3;
+        constexpr double H = 0.86602540378443864676;
+        const Cplx *w = c_first.t[MOD];
+        if constexpr (Q > 1) {
+#pragma unroll
+            for (int k = 0; k < 3; k++) inv_group<Q>(v + k * Q, w + 2 + 4 * k);
+        }
+#pragma unroll
+        for (int e = 0; e < Q; e++) {
+            const Cplx f = v[e], g = v[e + Q], h = v[e + 2 * Q];
+            const Cplx s{g.re + h.re, g.im + h.im}, d{g.re - h.re, g.im - h.im};
+            const double tr = fma(-0.5, s.re, f.re), ti = fma(-0.5, s.im, f.im);
+            v[e] = Cplx{f.re + s.re, f.im + s.im};
+            const Cplx b{fma(H, d.im, tr), fma(-H, d.re, ti)}, c{fma(-H, d.im, tr), fma(H, d.re, ti)};
+            v[e + Q] = Cplx{fma(b.re, w[0].re, b.im * w[0].im), fma(b.im, w[0].re, -(b.re * w[0].im))};
+            v[e + 2 * Q] = Cplx{fma(c.re, w[1].re, c.im * w[1].im), fma(c.im, w[1].re, -(c.re * w[1].im))};
+        }
+    } else {
+        inv_group<R>(v, c_first.r[MOD]);
+    }
+}
+
+template <class F, int R>
 __device__ __forceinline__ void load_roots(Cplx *tw, const Cplx *tab, int nodes, int node) {
 #pragma unroll
-    for (int q = 0; q < R / 2; q++) tw[q] = ldg(tab + q * nodes + node);
+    for (int q = 0; q < R / 2; q++) tw[q] = F::RES ? tab[q * nodes + node] : ldg(tab + q * nodes + node);
 }
 
 // One pass of radix R over the C points in A: NODES nodes of C / NODES
@@ -244,7 +324,7 @@ __device__ __forceinline__ void pass(Cplx *A, const Cplx *tab) {
     for (int g = threadIdx.x; g < G; g += F::T) {
         const int node = g / SUB, j0 = g % SUB, base = node * (R * SUB) + j0;
         Cplx tw[R / 2], v[R];
-        load_roots<R>(tw, tab, NODES, node);
+        load_roots<F, R>(tw, tab, NODES, node);
 #pragma unroll
         for (int e = 0; e < R; e++) v[e] = A[padx<F>(base + e * SUB)];
         if constexpr (INV) inv_group<R>(v, tw);
@@ -255,29 +335,31 @@ __device__ __forceinline__ void pass(Cplx *A, const Cplx *tab) {
     cta_sync<F>();
 }
 
-enum MidOp { MID_STORE_SQ, MID_STORE, MID_SQ, MID_MUL, MID_MULADD };
+enum MidOp { MID_STORE_SQ, MID_STORE_MUL, MID_STORE, MID_SQ, MID_MUL, MID_MULADD };
 
 // The last forward pass, the pointwise operation and the first inverse pass
 // on groups of RM consecutive points.  Spectra outside A are laid out
 // [element][group], so a warp reads and writes them contiguously, and S is
 // read back by the thread that wrote it.
-//   MID_STORE_SQ, MID_STORE: S <- v^2, S <- v, no inverse
+// G may have been written earlier in the launch, by the same thread; res: it
+// is in shared memory.
+//   MID_STORE_SQ, MID_STORE_MUL, MID_STORE: S <- v^2, v G, v; no inverse
 //   MID_SQ: v^2    MID_MUL: v G    MID_MULADD: v G + S
 template <class F>
-__device__ __forceinline__ void mid(Cplx *A, const Cplx *tab, int op, const Cplx *Gs, Cplx *S) {
+__device__ __forceinline__ void mid(Cplx *A, const Cplx *tab, int op, const Cplx *Gs, Cplx *S, bool res = false) {
     constexpr int R = F::RM, G = F::C / R;
 #pragma unroll 1
     for (int g = threadIdx.x; g < G; g += F::T) {
         Cplx tw[R / 2], v[R];
-        load_roots<R>(tw, tab, G, g);
+        load_roots<F, R>(tw, tab, G, g);
         const int base = padx<F>(g * R);
 #pragma unroll
         for (int e = 0; e < R; e++) v[e] = A[R <= (1 << F::PADL) ? base + e : padx<F>(g * R + e)];
         fwd_group<R>(v, tw);
-        if (op == MID_MUL || op == MID_MULADD) {
+        if (op == MID_MUL || op == MID_MULADD || op == MID_STORE_MUL) {
 #pragma unroll
             for (int e = 0; e < R; e++) {
-                const Cplx c = ldg(Gs + e * G + g);
+                const Cplx c = res ? Gs[e * G + g] : ldcg(Gs + e * G + g);
                 Cplx s{0.0, 0.0};
                 if (op == MID_MULADD) s = F::SQS ? S[e * G + g] : ldcg(S + e * G + g);
                 const double re = fma(v[e].re, c.re, fma(-v[e].im, c.im, s.re));
@@ -297,11 +379,11 @@ __device__ __forceinline__ void mid(Cplx *A, const Cplx *tab, int op, const Cplx
                 v[e].re = re;
                 v[e].im = im;
             }
-            if (op == MID_STORE_SQ) {
+        }
+        if (op == MID_STORE_SQ || op == MID_STORE_MUL) {
 #pragma unroll
-                for (int e = 0; e < R; e++) S[e * G + g] = v[e];
-                continue;
-            }
+            for (int e = 0; e < R; e++) S[e * G + g] = v[e];
+            continue;
         }
         inv_group<R>(v, tw);
 #pragma unroll
@@ -314,9 +396,10 @@ __device__ __forceinline__ void mid(Cplx *A, const Cplx *tab, int op, const Cplx
 struct View {
     Cplx *A;       // points, padded
     Cplx *S;       // a spectrum, [element][group]
-    int *xs;       // limbs of x: [2 e + half][thread]
+    int *xs;       // limbs of x: [2 e + half][thread], each thread's own
     int *bnd;      // carries between warps
     uint32_t *sc;  // scratch words of the carry scan and of votes
+    Cplx *res;     // RES: roots, then the spectra of N'' and N
 };
 
 template <class F>
@@ -329,11 +412,44 @@ __device__ __forceinline__ void carve(unsigned char *raw, Cplx *gscratch, View &
     } else {
         w.S = gscratch;
     }
-    w.xs = reinterpret_cast<int *>(raw);
-    raw += (size_t)F::C * 8;
+    w.res = reinterpret_cast<Cplx *>(raw);
+    if (F::RES) raw += (size_t)(2 * F::C + F::ROOTS) * 16;
+    if (F::XSS) {
+        w.xs = reinterpret_cast<int *>(raw);
+        raw += (size_t)F::C * 8;
+    } else {
+        w.xs = reinterpret_cast<int *>(gscratch + (F::SQS ? 0 : F::C));
+    }
     w.bnd = reinterpret_cast<int *>(raw);
     raw += (size_t)2 * F::WARPS * F::R1 * 8;
     w.sc = reinterpret_cast<uint32_t *>(raw);
+}
+
+// This thread's group of the first pass.
+template <class F>
+__device__ __forceinline__ int tid1() {
+    return F::T1 == F::T ? (int)threadIdx.x : (int)threadIdx.x & (F::T1 - 1);
+}
+
+// The roots (and with nn, nh the spectra) in shared memory, where the class
+// keeps them there: tab, nn and nh then point to the copies.
+template <class F>
+__device__ __forceinline__ void resident(const View &w, Tab &tab, const Cplx *&nn, const Cplx *&nh) {
+    if (!F::RES) return;
+    const Cplx *src = tab.t[0][0];
+    for (int i = threadIdx.x; i < F::ROOTS; i += F::T) w.res[i] = ldg(src + i);
+    if (nn)
+        for (int i = threadIdx.x; i < F::C; i += F::T) {
+            w.res[F::ROOTS + i] = ldg(nn + i);
+            w.res[F::ROOTS + F::C + i] = ldg(nh + i);
+        }
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int p = 0; p < 3; p++) tab.t[m][p] = w.res + (tab.t[m][p] - src);
+    nn = w.res + F::ROOTS;
+    nh = nn + F::C;
+    cta_sync<F>();
 }
 
 // First forward pass from the limbs in registers: modulus MOD (0: B^n + 1,
@@ -352,21 +468,20 @@ __device__ __forceinline__ void first_pass(Cplx *A, const int *lo, const int *hi
             v[e].im = 0.86602540378443864676 * c;
         }
     }
-    fwd_group<F::R1>(v, c_first.r[MOD]);
+    fwd_first<F::R1, MOD>(v);
 #pragma unroll
-    for (int e = 0; e < F::R1; e++) A[padx<F>((int)threadIdx.x + e * F::T)] = v[e];
+    for (int e = 0; e < F::R1; e++) A[padx<F>(tid1<F>() + e * F::T1)] = v[e];
     cta_sync<F>();
 }
 
 // Carries of every limb to the next one: k in, the neighbour's carry out.
-// Limb order: thread t + T e, then the second half; the carry out of the top
+// Limb order: thread t + T1 e, then the second half; the carry out of the top
 // limb comes back negated (B^n = -1), modulo M2 at limbs 0 and n/2.
 template <class F, int MOD>
 __device__ __forceinline__ void exchange(int *kl, int *kh, int *buf) {
     constexpr int R = F::R1;
     const unsigned FULL = 0xffffffffu;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int pl[R], ph[R];
     if constexpr (F::WARPS > 1) {
         if (lane == 31) {
 #pragma unroll
@@ -376,40 +491,61 @@ __device__ __forceinline__ void exchange(int *kl, int *kh, int *buf) {
             }
         }
         __syncthreads();
-#pragma unroll
-        for (int e = 0; e < R; e++) {
-            pl[e] = __shfl_up_sync(FULL, kl[e], 1);
-            ph[e] = __shfl_up_sync(FULL, kh[e], 1);
-        }
-        if (lane == 0) {
-            const int w = warp ? warp - 1 : F::WARPS - 1;
-#pragma unroll
-            for (int e = 0; e < R; e++) {
-                pl[e] = buf[(w * R + e) * 2];
-                ph[e] = buf[(w * R + e) * 2 + 1];
-            }
-        }
-    } else {
-#pragma unroll
-        for (int e = 0; e < R; e++) {
-            pl[e] = __shfl_sync(FULL, kl[e], (lane + 31) & 31);
-            ph[e] = __shfl_sync(FULL, kh[e], (lane + 31) & 31);
-        }
     }
-    if (threadIdx.x == 0) {  // the last thread's carries go to the next element
-        const int tl = pl[R - 1], th = ph[R - 1];
+    [[maybe_unused]] const int wl = kl[R - 1], wh = kh[R - 1];  // the top limbs' carries
+    // descending e: the first thread takes the last thread's carry of e - 1
 #pragma unroll
-        for (int e = R - 1; e > 0; e--) {
-            pl[e] = pl[e - 1];
-            ph[e] = ph[e - 1];
+    for (int e = R - 1; e >= 0; e--) {
+        int pl, ph;
+        if constexpr (F::WARPS > 1) {
+            pl = __shfl_up_sync(FULL, kl[e], 1);
+            ph = __shfl_up_sync(FULL, kh[e], 1);
+            if (lane == 0) {
+                const int at = warp ? (warp - 1) * R + e : (F::WARPS - 1) * R + (e ? e - 1 : R - 1);
+                pl = buf[at * 2];
+                ph = buf[at * 2 + 1];
+            }
+        } else {
+            constexpr int M = F::T1 - 1;  // T1 = 32 or 16 lanes in a ring
+            const int from = (lane & ~M) | ((lane + M) & M);
+            pl = (lane & M) != M ? kl[e] : (e ? kl[e ? e - 1 : 0] : wl);
+            ph = (lane & M) != M ? kh[e] : (e ? kh[e ? e - 1 : 0] : wh);
+            pl = __shfl_sync(FULL, pl, from);
+            ph = __shfl_sync(FULL, ph, from);
         }
-        pl[0] = -th;
-        ph[0] = MOD == 0 ? tl : tl - th;
+        if (e == 0 && tid1<F>() == 0) {
+            const int tl = pl, th = ph;
+            pl = -th;
+            ph = MOD == 0 ? tl : tl - th;
+        }
+        kl[e] = pl;
+        kh[e] = ph;
+    }
+}
+
+// Two more local carry steps after the carries k of the first split: limbs
+// of at most B/2 + 40 in magnitude.
+template <class F, int MOD>
+__device__ __forceinline__ void settle(const View &w, int b, int *kl, int *kh, int *lo, int *hi) {
+    constexpr int R = F::R1;
+    const int mask = (1 << b) - 1, half = 1 << (b - 1);
+    exchange<F, MOD>(kl, kh, w.bnd);
+#pragma unroll
+    for (int turn = 1; turn <= 2; turn++) {
+#pragma unroll
+        for (int e = 0; e < R; e++) {
+            const int cl = lo[e] + kl[e] + half, ch = hi[e] + kh[e] + half;
+            kl[e] = cl >> b;
+            kh[e] = ch >> b;
+            lo[e] = (cl & mask) - half;
+            hi[e] = (ch & mask) - half;
+        }
+        exchange<F, MOD>(kl, kh, w.bnd + (turn & 1) * 2 * F::WARPS * R);
     }
 #pragma unroll
     for (int e = 0; e < R; e++) {
-        kl[e] = pl[e];
-        kh[e] = ph[e];
+        lo[e] += kl[e];
+        hi[e] += kh[e];
     }
 }
 
@@ -427,8 +563,8 @@ __device__ __forceinline__ void last_pass(const View &w, int b, int dbl, int *lo
     {
         Cplx v[R];
 #pragma unroll
-        for (int e = 0; e < R; e++) v[e] = w.A[padx<F>((int)threadIdx.x + e * F::T)];
-        inv_group<R>(v, c_first.r[MOD]);
+        for (int e = 0; e < R; e++) v[e] = w.A[padx<F>(tid1<F>() + e * F::T1)];
+        inv_last<R, MOD>(v);
 #pragma unroll
         for (int e = 0; e < R; e++) {
             long long ql, qh;
@@ -450,24 +586,7 @@ __device__ __forceinline__ void last_pass(const View &w, int b, int dbl, int *lo
             hi[e] = (int)(((unsigned)qh << dbl) & (unsigned)mask) - half;
         }
     }
-    exchange<F, MOD>(kl, kh, w.bnd);
-#pragma unroll
-    for (int round = 1; round <= 2; round++) {
-#pragma unroll
-        for (int e = 0; e < R; e++) {
-            const int cl = lo[e] + kl[e] + half, ch = hi[e] + kh[e] + half;
-            kl[e] = cl >> b;
-            kh[e] = ch >> b;
-            lo[e] = (cl & mask) - half;
-            hi[e] = (ch & mask) - half;
-        }
-        exchange<F, MOD>(kl, kh, w.bnd + (round & 1) * 2 * F::WARPS * R);
-    }
-#pragma unroll
-    for (int e = 0; e < R; e++) {
-        lo[e] += kl[e];
-        hi[e] += kh[e];
-    }
+    settle<F, MOD>(w, b, kl, kh, lo, hi);
 }
 
 // The passes between the first and the middle one.
@@ -482,19 +601,30 @@ __device__ __forceinline__ void inv_inner(Cplx *A, const Cplx *const *t) {
     pass<F, F::R2, F::R1, true>(A, t[0]);
 }
 
-// One Montgomery step on the limbs (lo, hi) of x:
-//   square: x <- x^2 / R'    else: x <- x / R'    (mod N; times two when dbl)
-// nn, nh: spectra of N'' (modulo B^n + 1) and N (modulo M2).
+// x's limbs as the last step found them.
+template <class F>
+__device__ __forceinline__ void load_x(const View &w, int *lo, int *hi) {
+#pragma unroll
+    for (int e = 0; e < F::R1; e++) {
+        lo[e] = w.xs[(2 * e) * F::T1 + tid1<F>()];
+        hi[e] = w.xs[(2 * e + 1) * F::T1 + tid1<F>()];
+    }
+}
+
+// One Montgomery step on the limbs (lo, hi) of x (mod N; times two when dbl):
+//   square: x <- x^2 / R', or x y / R' given y's spectra (2 C points: modulo
+//   B^n + 1, then M2)    else: x <- x / R'
+// nn, nh: spectra of N'' (modulo B^n + 1) and N (modulo M2), from resident().
 template <class F>
 __device__ __forceinline__ void step(const View &w, const Tab &tab, const Cplx *nn, const Cplx *nh, int b,
-                                     bool square, int dbl, int *lo, int *hi) {
+                                     bool square, int dbl, int *lo, int *hi, const Cplx *y = nullptr) {
     constexpr int R = F::R1, MT = F::NPASS - 2;
 #pragma unroll
     for (int e = 0; e < R; e++) {
-        w.xs[(2 * e) * F::T + threadIdx.x] = lo[e];
-        w.xs[(2 * e + 1) * F::T + threadIdx.x] = hi[e];
+        w.xs[(2 * e) * F::T1 + tid1<F>()] = lo[e];
+        w.xs[(2 * e + 1) * F::T1 + tid1<F>()] = hi[e];
     }
-    // phases: 0 spectrum of x (or its square) modulo M2 into S, 1 D, 2 m, 3 U
+    // phases: 0 spectrum of x (of its square, of x y) modulo M2 into S, 1 D, 2 m, 3 U
 #pragma unroll 1
     for (int ph = 0; ph < 4; ph++) {
         if (ph == 1 && !square) continue;  // D = x
@@ -504,15 +634,12 @@ __device__ __forceinline__ void step(const View &w, const Tab &tab, const Cplx *
         const Cplx *t[3] = {mod ? tab.t[1][0] : tab.t[0][0], mod ? tab.t[1][1] : tab.t[0][1],
                             mod ? tab.t[1][2] : tab.t[0][2]};
         fwd_inner<F>(w.A, t);
-        const int op = ph == 0 ? (square ? MID_STORE_SQ : MID_STORE)
-                               : (ph == 1 ? MID_SQ : (ph == 2 ? MID_MUL : MID_MULADD));
-        mid<F>(w.A, t[MT], op, ph == 2 ? nn : nh, w.S);
+        const int op = ph == 0 ? (!square ? MID_STORE : (y ? MID_STORE_MUL : MID_STORE_SQ))
+                               : (ph == 1 ? (y ? MID_MUL : MID_SQ) : (ph == 2 ? MID_MUL : MID_MULADD));
+        mid<F>(w.A, t[MT], op, ph == 0 ? y + F::C : (ph == 1 ? y : (ph == 2 ? nn : nh)), w.S,
+               F::RES && ph >= 2);
         if (ph == 0) {
-#pragma unroll
-            for (int e = 0; e < R; e++) {
-                lo[e] = w.xs[(2 * e) * F::T + threadIdx.x];
-                hi[e] = w.xs[(2 * e + 1) * F::T + threadIdx.x];
-            }
+            load_x<F>(w, lo, hi);
             continue;
         }
         inv_inner<F>(w.A, t);
@@ -521,38 +648,32 @@ __device__ __forceinline__ void step(const View &w, const Tab &tab, const Cplx *
     }
 }
 
-// lo, hi <- a times the limbs (1 <= a < 2^16), carried locally; |a x| < B^n / 4.
+// lo, hi <- limbs + c (ylo, yhi), carried locally; |c| < 2^16, and the value
+// stays below B^n / 4.
 template <class F>
-__device__ void mul_small(const View &w, int b, uint32_t a, int *lo, int *hi) {
+__device__ void add_mul(const View &w, int b, int c, const int *ylo, const int *yhi, int *lo, int *hi) {
     constexpr int R = F::R1;
     const int mask = (1 << b) - 1, half = 1 << (b - 1);
     int kl[R], kh[R];
 #pragma unroll
     for (int e = 0; e < R; e++) {
-        const long long ql = (long long)lo[e] * a + half, qh = (long long)hi[e] * a + half;
+        const long long ql = lo[e] + (long long)c * ylo[e] + half, qh = hi[e] + (long long)c * yhi[e] + half;
         kl[e] = (int)(ql >> b);
         kh[e] = (int)(qh >> b);
         lo[e] = (int)(ql & mask) - half;
         hi[e] = (int)(qh & mask) - half;
     }
     cta_sync<F>();
-    exchange<F, 0>(kl, kh, w.bnd);
+    settle<F, 0>(w, b, kl, kh, lo, hi);
+}
+
+// This thread's limbs from an array of n words written earlier in the launch.
+template <class F>
+__device__ __forceinline__ void get_limbs(const uint32_t *src, int *lo, int *hi) {
 #pragma unroll
-    for (int round = 1; round <= 2; round++) {
-#pragma unroll
-        for (int e = 0; e < R; e++) {
-            const int cl = lo[e] + kl[e] + half, ch = hi[e] + kh[e] + half;
-            kl[e] = cl >> b;
-            kh[e] = ch >> b;
-            lo[e] = (cl & mask) - half;
-            hi[e] = (ch & mask) - half;
-        }
-        exchange<F, 0>(kl, kh, w.bnd + (round & 1) * 2 * F::WARPS * R);
-    }
-#pragma unroll
-    for (int e = 0; e < R; e++) {
-        lo[e] += kl[e];
-        hi[e] += kh[e];
+    for (int e = 0; e < F::R1; e++) {
+        lo[e] = (int)__ldcg(src + tid1<F>() + e * F::T1);
+        hi[e] = (int)__ldcg(src + F::C + tid1<F>() + e * F::T1);
     }
 }
 
@@ -601,16 +722,22 @@ __device__ int normalize(int *L, int b, uint32_t *sc) {
     return (int)tot - 1;
 }
 
+// This thread's limbs to and from an array of n words.
+template <class F, class W>
+__device__ __forceinline__ void put_limbs(W *L, const int *lo, const int *hi) {
+#pragma unroll
+    for (int e = 0; e < F::R1; e++) {
+        L[tid1<F>() + e * F::T1] = (W)lo[e];
+        L[F::C + tid1<F>() + e * F::T1] = (W)hi[e];
+    }
+}
+
 // L[0..n) <- the canonical digits (base B) of the value of the limbs modulo
 // N, for a value in (-N, N); nl: N's digits.  L overlays A.
 template <class F>
 __device__ void to_digits(const View &w, int b, const uint32_t *nl, const int *lo, const int *hi, int *L) {
     cta_sync<F>();
-#pragma unroll
-    for (int e = 0; e < F::R1; e++) {
-        L[threadIdx.x + e * F::T] = lo[e];
-        L[F::C + threadIdx.x + e * F::T] = hi[e];
-    }
+    put_limbs<F>(L, lo, hi);
     cta_sync<F>();
     if (normalize<F>(L, b, w.sc) < 0) {
         for (int i = threadIdx.x; i < F::N; i += F::T) L[i] += (int)nl[i];
@@ -625,21 +752,21 @@ __device__ __forceinline__ bool vote_and(bool v) {
     return __syncthreads_and(v ? 1 : 0) != 0;
 }
 
-// Balanced limbs (|limb| <= B/2) from canonical digits d, at the positions
+// Balanced limbs (|limb| <= B/2) from canonical digits d(i), at the positions
 // of this thread; a carry out of the top limb wraps to -1 at limb 0 (B^n =
 // -1; it cannot happen for a number below B^n / 2).
-template <class F>
-__device__ __forceinline__ void balanced(const uint32_t *d, int b, int *lo, int *hi) {
+template <class F, class Digit>
+__device__ __forceinline__ void balanced(Digit d, int b, int *lo, int *hi) {
     const int B = 1 << b, half = B >> 1;
     auto at = [&](int i) {
-        const int v = (int)d[i];
-        const int top = (int)d[i ? i - 1 : F::N - 1] >= half ? 1 : 0;
+        const int v = (int)d(i);
+        const int top = (int)d(i ? i - 1 : F::N - 1) >= half ? 1 : 0;
         return (v >= half ? v - B : v) + (i ? top : -top);
     };
 #pragma unroll
     for (int e = 0; e < F::R1; e++) {
-        lo[e] = at((int)threadIdx.x + e * F::T);
-        hi[e] = at(F::C + (int)threadIdx.x + e * F::T);
+        lo[e] = at(tid1<F>() + e * F::T1);
+        hi[e] = at(F::C + tid1<F>() + e * F::T1);
     }
 }
 

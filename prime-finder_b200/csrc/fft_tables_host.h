@@ -15,7 +15,7 @@ namespace fp {
 
 // Angles are kept as integers in units of a full turn / kTurn, which every
 // halving below divides exactly.
-constexpr long long kTurn = 3ll << 40;
+constexpr long long kTurn = 36ll << 34;
 
 // e^(2 pi i num / kTurn), each part correctly rounded but for the rare tie
 // of the extended-precision value; the argument is reduced to an eighth turn.
@@ -48,18 +48,27 @@ inline long long node_angle(long long phi0, int lv, long long node) {
 // Root angle of the moduli: y^C = i (B^n + 1), y^C = e^(2 pi i / 3) (M2).
 inline long long top_angle(int mod) { return mod ? kTurn / 3 : kTurn / 4; }
 
-// The roots of a radix-R group at node `node` of level `lv`.
-inline Cplx group_root(int mod, int lv, long long node, int q) {
+// The roots of a radix-R group at node `node` of (binary) level `lv` under
+// the angle phi0.
+inline Cplx group_root(long long phi0, int lv, long long node, int q) {
     int s = 0;
     while (q >= (1 << s)) s++;  // q = 0: level 0; else q in [2^(s-1), 2^s): level s
     const int u = s ? q - (1 << (s - 1)) : 0;
-    return unit_root(node_angle(top_angle(mod), lv + s, (node << s) + 2 * u));
+    return unit_root(node_angle(phi0, lv + s, (node << s) + 2 * u));
 }
+
+// Angle of child k of the ternary level at the root of the tree.
+inline long long child_angle(int mod, int k) { return top_angle(mod) / 3 + kTurn / 3 * k; }
 
 inline First first_roots() {
     First f{};
-    for (int mod = 0; mod < 2; mod++)
-        for (int q = 0; q < 8; q++) f.r[mod][q] = group_root(mod, 0, 0, q);
+    for (int mod = 0; mod < 2; mod++) {
+        for (int q = 0; q < 8; q++) f.r[mod][q] = group_root(top_angle(mod), 0, 0, q);
+        f.t[mod][0] = unit_root(child_angle(mod, 0));
+        f.t[mod][1] = unit_root(2 * child_angle(mod, 0));
+        for (int k = 0; k < 3; k++)
+            for (int q = 0; q < 4; q++) f.t[mod][2 + 4 * k + q] = group_root(child_angle(mod, k), 0, 0, q);
+    }
     return f;
 }
 
@@ -79,7 +88,14 @@ std::vector<Cplx> class_roots(size_t off[2][3]) {
         for (int p = 1; p < F::NPASS; p++) {
             off[mod][p - 1] = v.size();
             for (int q = 0; q < radix[p] / 2; q++)
-                for (int nd = 0; nd < nodes; nd++) v.push_back(group_root(mod, ilog2(nodes), nd, q));
+                for (int nd = 0; nd < nodes; nd++) {
+                    if (nodes % 3 == 0) {
+                        const int sub = nodes / 3;
+                        v.push_back(group_root(child_angle(mod, nd / sub), ilog2(sub), nd % sub, q));
+                    } else {
+                        v.push_back(group_root(top_angle(mod), ilog2(nodes), nd, q));
+                    }
+                }
             nodes *= radix[p];
         }
     }

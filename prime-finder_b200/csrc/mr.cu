@@ -15,31 +15,12 @@
 #include "bigint_host.h"
 #include "common.cuh"
 #include "lucas_host.h"
-#include "mr_device.cuh"
-#include "mr_fft.h"
+#include "mr_engine.h"
+#include "mr_prep_host.h"
 #include "mr_tables_host.h"
 #include "pfb_mr.h"
 
-#include "mr_ctx_kernels.cuh"
-#include "mr_kernels.cuh"
-#include "radix_probe.cuh"
-#include "mr_prep_host.h"
-
 using namespace pfb::mr;
-
-struct pfb_mr {
-    int device = 0;
-    int num_sms = 0;
-    cudaStream_t stream = nullptr;
-    uint32_t *d_tw = nullptr;
-    uint32_t *d_wide = nullptr;
-    Twiddles tw{};
-    fp::Engine fe;
-    // persistent-kernel parameters per transform length (pfb_mr_autotune):
-    // steps of one candidate per quantum, steps per launch
-    int quantum[LOG_LMAX + 1];
-    int chunk[LOG_LMAX + 1];
-};
 
 static int build_tables(pfb_mr *e) {
     const int half = 1 << (LOG_LMAX - 1);
@@ -54,14 +35,13 @@ static int build_tables(pfb_mr *e) {
         e->tw.wish[pr] = base + 3 * half;
     }
     const CrtConsts cc = crt_consts();
-    PFB_CUDA(cudaMemcpyToSymbol(c_crt, &cc, sizeof(cc)));
     WideTabs wt{};
     const std::vector<uint32_t> wide = wide_tables(h, wt);
     PFB_CUDA(cudaMalloc(&e->d_wide, wide.size() * sizeof(uint32_t)));
     PFB_CUDA(cudaMemcpy(e->d_wide, wide.data(), wide.size() * sizeof(uint32_t), cudaMemcpyHostToDevice));
     wt.base = (const uint4 *)e->d_wide;
-    PFB_CUDA(cudaMemcpyToSymbol(c_wide, &wt, sizeof(wt)));
-    return PFB_OK;
+    e->wt = wt;
+    return int_setup(cc, wt);
 }
 
 extern "C" int pfb_mr_device(const pfb_mr_t *e) { return e ? e->device : -1; }
@@ -91,13 +71,6 @@ extern "C" int pfb_mr_create(pfb_mr_t **out, int device) {
     }
     if (!rc) rc = build_tables(e);
     if (!rc) rc = fp::engine_create(e->fe);
-    if (!rc) {
-        const int mx = (int)std::max(smem_bytes(LOG_LCTA), smem_bytes(LOG_LSEQ));
-        ce = cudaFuncSetAttribute(persist_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-        if (ce == cudaSuccess) ce = cudaFuncSetAttribute(prep_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-        if (ce == cudaSuccess) ce = cudaFuncSetAttribute(ctx_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, mx);
-        if (ce != cudaSuccess) rc = pfb::cuda_fail(ce, "smem attribute", __FILE__, __LINE__);
-    }
     if (rc) {
         if (e->stream) cudaStreamDestroy(e->stream);
         cudaFree(e->d_tw);
@@ -127,7 +100,7 @@ namespace {
 
 // Per-candidate device layout inside the arena (32-bit words).
 struct Layout {
-    size_t x, res, nn, nh, npl, nl, exp, yb, lv0, lv1, lqk, lt, lone, gy, raw, total;
+    size_t x, res, nn, nh, npl, nl, exp, yb, lv0, lv1, lqk, lt, lone, gy, raw, ys, total;
 };
 
 Layout layout_for(int logl, size_t exp_words, bool lucas = false, bool raw = false) {
@@ -161,8 +134,9 @@ Layout layout_for(int logl, size_t exp_words, bool lucas = false, bool raw = fal
 }
 
 // Layout of a candidate of the floating-point engine: n = 2 C digits, spectra
-// of C points (4 words each).
-Layout layout_fp(int cls, size_t exp_words) {
+// of C points (4 words each).  ctx_logl: a modulus of a context instead, with
+// the buffers of the integer engine's raw products at that transform length.
+Layout layout_fp(int cls, size_t exp_words, bool lucas, int ctx_logl = 0) {
     const size_t C = (size_t)fp::class_points(cls), n = 2 * C;
     Layout l{};
     size_t o = 0;
@@ -171,19 +145,34 @@ Layout layout_fp(int cls, size_t exp_words) {
         o += (words + 63) & ~(size_t)63;
         return at;
     };
-    l.x = take(n);
-    l.res = take(n);
     l.nn = take(4 * C);
     l.nh = take(4 * C);
     l.npl = take(n);
     l.nl = take(n);
-    l.exp = take(exp_words);
+    if (ctx_logl) {
+        const size_t L = (size_t)1 << ctx_logl;
+        l.lt = take(L / 2);
+        l.gy = take(2 * L);
+        l.raw = take(2 * L);
+        l.ys = take(8 * C);
+    } else {
+        l.x = take(n);
+        l.res = take(n);
+        l.exp = take(exp_words);
+    }
+    if (lucas) {
+        l.lv0 = take(n);
+        l.lv1 = take(n);
+        l.lqk = take(n);
+        l.lt = take(n);
+        l.lone = take(n);
+    }
     l.total = o;
     return l;
 }
 
 Layout layout_for(const HostPrep &hp, bool lucas) {
-    return hp.fpc ? layout_fp(hp.fpc - 1, hp.exp.size()) : layout_for(hp.logl, hp.exp.size(), lucas);
+    return hp.fpc ? layout_fp(hp.fpc - 1, hp.exp.size(), lucas) : layout_for(hp.logl, hp.exp.size(), lucas);
 }
 
 // Bits of a digit of a candidate's x0, npl, nl and residue.
@@ -211,19 +200,20 @@ struct ClassRuns {
 
 // Device scratch (points) of one launch of every class' persistent kernel,
 // and where a class' part begins.
-size_t fp_scratch_points(const pfb_mr *e, const int *count, size_t *begin) {
+size_t fp_scratch_points(const pfb_mr *e, bool lucas, const int *count, size_t *begin) {
     size_t o = 0;
     for (int c = 0; c < fp::kClasses; c++) {
         begin[c] = o;
-        if (count[c]) o += fp::scratch_points(c) * fp::persist_launch(e->fe, c, count[c], e->num_sms).grid.x;
+        if (count[c])
+            o += fp::scratch_points(c, lucas) * fp::persist_launch(e->fe, lucas, c, count[c], e->num_sms).grid.x;
     }
     return o;
 }
 
 // Quanta of one launch of a class: jobs that each have a CTA of their own run
 // their whole chunk in one quantum.
-void fp_quanta(const pfb_mr *e, int cls, int n, long long chunk, int tuned, int *quantum, unsigned *total) {
-    const int ctas = (int)fp::persist_launch(e->fe, cls, n, e->num_sms).grid.x;
+void fp_quanta(const pfb_mr *e, bool lucas, int cls, int n, long long chunk, int tuned, int *quantum, unsigned *total) {
+    const int ctas = (int)fp::persist_launch(e->fe, lucas, cls, n, e->num_sms).grid.x;
     *quantum = (int)(n <= ctas ? chunk : std::min<long long>(chunk, tuned));
     *total = (unsigned)std::min<long long>((long long)n * ((chunk + *quantum - 1) / *quantum), 0x7fffffffll);
 }
@@ -237,11 +227,13 @@ int slot_key(const HostPrep &hp) { return hp.fpc ? kFpKey + hp.fpc - 1 : hp.logl
 Layout slot_layout(int key) {
     if (key >= kFpKey) {
         const int cls = key - kFpKey;
-        return layout_fp(cls, ((size_t)fp::limb_bits(cls) * 2 * fp::class_points(cls) + 31) / 32 + 1);
+        return layout_fp(cls, ((size_t)fp::limb_bits(cls) * 2 * fp::class_points(cls) + 31) / 32 + 1, false);
     }
     const size_t H = (size_t)1 << (key - 1);
     return layout_for(key, (LIMB_BITS * H + 31) / 32 + 1);
 }
+
+size_t slot_bytes(int key) { return slot_layout(key).total * sizeof(uint32_t); }
 
 // fft: candidates that the floating-point engine can hold are set up for it.
 void prep_all(const pfb_mr_number_t *nums, int n, uint32_t base, int mode, const pfb_mr_number_t *exps,
@@ -327,7 +319,7 @@ int chunk_graph(pfb_mr_batch *b, long long chunk, int quantum, cudaGraphExec_t *
     cudaError_t ce = cudaGraphAddMemsetNode(&n_mem, graph, nullptr, 0, &mp);
     if (ce == cudaSuccess && b->runs.n_int) {
         cudaKernelNodeParams kp{};
-        kp.func = (void *)persist_kernel;
+        kp.func = int_persist_func();
         kp.gridDim = dim3((unsigned)std::min(b->runs.n_int, std::max(1, b->e->num_sms)));
         kp.blockDim = dim3(THREADS);
         kp.sharedMemBytes = (unsigned)smem_bytes(b->maxlog);
@@ -339,8 +331,8 @@ int chunk_graph(pfb_mr_batch *b, long long chunk, int quantum, cudaGraphExec_t *
         int nc = b->runs.count[c], qc = 0;
         if (!nc) continue;
         unsigned tc = 0;
-        fp_quanta(b->e, c, nc, chunk, quantum, &qc, &tc);
-        const fp::Launch l = fp::persist_launch(b->e->fe, c, nc, b->e->num_sms);
+        fp_quanta(b->e, b->mode == 2, c, nc, chunk, quantum, &qc, &tc);
+        const fp::Launch l = fp::persist_launch(b->e->fe, b->mode == 2, c, nc, b->e->num_sms);
         const int *order = b->d_order + b->runs.first[c];
         unsigned int *cnt = counter + 1 + c;
         fp::Tab tab = b->e->fe.tab[c];
@@ -362,8 +354,8 @@ int chunk_graph(pfb_mr_batch *b, long long chunk, int quantum, cudaGraphExec_t *
     return PFB_OK;
 }
 
-int batch_build(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base, int mode,
-                const pfb_mr_number_t *exps, pfb_mr_batch **out) {
+int batch_build_on(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base, int mode,
+                   const pfb_mr_number_t *exps, bool fft, pfb_mr_batch **out) {
     *out = nullptr;
     if (!e || !nums || n <= 0 || base < 2 || base > 0xFFFFu) {
         pfb::set_error("pfb_mr: bad argument (n=%d base=%u)", n, base);
@@ -374,7 +366,7 @@ int batch_build(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base, in
     b->e = e;
     b->n = n;
     b->mode = mode;
-    prep_all(nums, n, base, mode, exps, b->hp, true);
+    prep_all(nums, n, base, mode, exps, b->hp, fft);
     std::vector<Layout> lay(n);
     size_t total = 0;
     for (int i = 0; i < n; i++) {
@@ -390,7 +382,7 @@ int batch_build(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base, in
     const size_t lucas_bytes = mode == 2 ? (((size_t)n * sizeof(LucasDev) + 255) & ~(size_t)255) : 0;
     b->runs.build(n, [&](int i) { return b->hp[i].ok && b->hp[i].decided < 0; }, [&](int i) { return b->hp[i].fpc; });
     const size_t order_bytes = (b->runs.order.size() * sizeof(int) + 255) & ~(size_t)255;
-    const size_t scratch_bytes = fp_scratch_points(e, b->runs.count, b->scratch_begin) * sizeof(fp::Cplx);
+    const size_t scratch_bytes = fp_scratch_points(e, mode == 2, b->runs.count, b->scratch_begin) * sizeof(fp::Cplx);
     const size_t need = job_bytes + lock_bytes + lucas_bytes + order_bytes + scratch_bytes + total * sizeof(uint32_t);
     if (cudaMalloc(&b->d_arena, need) != cudaSuccess) {
         cudaGetLastError();
@@ -451,15 +443,22 @@ int batch_build(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base, in
             lc.lqk = w + l.lqk;
             lc.lt = w + l.lt;
             lc.lone = w + l.lone;
-            lc.gy = w + l.gy;
+            if (!h.fpc) lc.gy = w + l.gy;
             lc.q = h.q;
             lc.lb = h.lb;
             j.lucas = b->d_lucas + i;
-            // V_0 = 2, V_1 = P = 1, Q^0 = 1, and 1 itself, in Montgomery form
-            if (ce == cudaSuccess) ce = cudaMemcpyAsync(lc.lv0, h.v0.data(), H * 4, cudaMemcpyHostToDevice, e->stream);
-            if (ce == cudaSuccess) ce = cudaMemcpyAsync(lc.lv1, h.x0.data(), H * 4, cudaMemcpyHostToDevice, e->stream);
-            if (ce == cudaSuccess) ce = cudaMemcpyAsync(lc.lqk, h.x0.data(), H * 4, cudaMemcpyHostToDevice, e->stream);
-            if (ce == cudaSuccess) ce = cudaMemcpyAsync(lc.lone, h.x0.data(), H * 4, cudaMemcpyHostToDevice, e->stream);
+            // V_0 = 2, V_1 = P = 1, Q^0 = 1, and 1 itself, in Montgomery form (the
+            // floating-point engine's set-up kernel makes them from x0)
+            if (!h.fpc) {
+                if (ce == cudaSuccess)
+                    ce = cudaMemcpyAsync(lc.lv0, h.v0.data(), H * 4, cudaMemcpyHostToDevice, e->stream);
+                if (ce == cudaSuccess)
+                    ce = cudaMemcpyAsync(lc.lv1, h.x0.data(), H * 4, cudaMemcpyHostToDevice, e->stream);
+                if (ce == cudaSuccess)
+                    ce = cudaMemcpyAsync(lc.lqk, h.x0.data(), H * 4, cudaMemcpyHostToDevice, e->stream);
+                if (ce == cudaSuccess)
+                    ce = cudaMemcpyAsync(lc.lone, h.x0.data(), H * 4, cudaMemcpyHostToDevice, e->stream);
+            }
         }
         if (ce == cudaSuccess) ce = cudaMemcpyAsync((void *)j.npl, h.npl.data(), H * 4, cudaMemcpyHostToDevice, e->stream);
         if (ce == cudaSuccess) ce = cudaMemcpyAsync((void *)j.nl, h.nl.data(), H * 4, cudaMemcpyHostToDevice, e->stream);
@@ -482,8 +481,7 @@ int batch_build(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base, in
         if (ce != cudaSuccess) rc = pfb::cuda_fail(ce, "fft_prep_kernel", __FILE__, __LINE__);
     }
     if (!rc && b->runs.n_int) {
-        prep_kernel<<<n, THREADS, smem_bytes(b->maxlog), e->stream>>>(b->d_jobs, nullptr, e->tw);
-        ce = cudaGetLastError();
+        ce = int_prep(b->d_jobs, nullptr, n, b->maxlog, e->tw, e->stream);
         if (ce != cudaSuccess) rc = pfb::cuda_fail(ce, "prep_kernel", __FILE__, __LINE__);
     }
     // host staging must outlive the copies; later work may use other streams
@@ -497,6 +495,15 @@ int batch_build(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base, in
     }
     *out = b;
     return PFB_OK;
+}
+
+// A batch on the floating-point engine, whose spectra take up to half as much
+// memory again as the integer engine's; where the device cannot hold that,
+// the whole batch on the integer engine.
+int batch_build(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base, int mode,
+                const pfb_mr_number_t *exps, pfb_mr_batch **out) {
+    const int rc = batch_build_on(e, nums, n, base, mode, exps, true, out);
+    return rc == PFB_E_NOMEM ? batch_build_on(e, nums, n, base, mode, exps, false, out) : rc;
 }
 
 // Enqueues about `steps` steps of every unfinished candidate: launches of the
@@ -875,7 +882,6 @@ double now_s(const pfb_mr_server *s) {
     return std::chrono::duration<double>(Clock::now() - s->t0).count();
 }
 
-size_t slot_bytes(int logl) { return slot_layout(logl).total * sizeof(uint32_t); }
 
 // Slot memory; a failure injected from the host (a test hook) is reported as
 // cudaErrorMemoryAllocation without calling cudaMalloc.
@@ -904,6 +910,10 @@ void srv_prep_worker(pfb_mr_server *s) {
         }
         pfb_mr_number_t num{r.limbs.data(), (int)r.limbs.size()};
         host_prep(num, s->cfg.base, 1, nullptr, r.hp, true);
+        // a budget below one slot of the floating-point engine: the integer
+        // engine's slots are smaller
+        if (r.hp.ok && r.hp.fpc && s->cfg.hbm_budget_bytes && slot_bytes(slot_key(r.hp)) > s->cfg.hbm_budget_bytes)
+            host_prep(num, s->cfg.base, 1, nullptr, r.hp, false);
         {
             std::lock_guard<std::mutex> lk(s->mu);
             s->preparing--;
@@ -1079,8 +1089,7 @@ int srv_admit(pfb_mr_server *s, std::vector<int> &admitted) {
         PFB_CUDA(cudaMemcpyAsync(s->d_list, list.data(), list.size() * sizeof(int), cudaMemcpyHostToDevice,
                                  s->stream));
         if (adm.n_int) {
-            prep_kernel<<<adm.n_int, THREADS, smem_bytes(maxlog), s->stream>>>(s->d_jobs, s->d_list, s->e->tw);
-            PFB_CUDA(cudaGetLastError());
+            PFB_CUDA(int_prep(s->d_jobs, s->d_list, adm.n_int, maxlog, s->e->tw, s->stream));
         }
         for (int c = 0; c < fp::kClasses; c++)
             if (adm.count[c])
@@ -1148,7 +1157,7 @@ int srv_launch(pfb_mr_server *s) {
         s->runs_stale = false;
     }
     size_t begin[fp::kClasses];
-    const size_t need = fp_scratch_points(e, s->runs.count, begin) * sizeof(fp::Cplx);
+    const size_t need = fp_scratch_points(e, false, s->runs.count, begin) * sizeof(fp::Cplx);
     if (need > s->scratch_bytes) {
         PFB_CUDA(cudaStreamSynchronize(s->stream));
         cudaFree(s->d_scratch);
@@ -1169,9 +1178,12 @@ int srv_launch(pfb_mr_server *s) {
             PFB_CUDA(cudaEventRecord(s->fork, s->stream));
             forked = true;
         }
-        persist_kernel<<<std::min(s->runs.n_int, std::max(1, e->num_sms)), THREADS, smem_bytes(maxlog), s->stream>>>(
-            s->d_jobs, cap, s->d_locks, s->d_counter, (unsigned int)(s->runs.n_int * qpj), quantum, e->tw);
-        PFB_CUDA(cudaGetLastError());
+        int n = cap, q = quantum;
+        unsigned int *counter = s->d_counter, total = (unsigned int)(s->runs.n_int * qpj);
+        Twiddles tw = e->tw;
+        void *args[] = {&s->d_jobs, &n, &s->d_locks, &counter, &total, &q, &tw};
+        PFB_CUDA(cudaLaunchKernel(int_persist_func(), dim3(std::min(s->runs.n_int, std::max(1, e->num_sms))),
+                                  dim3(THREADS), args, smem_bytes(maxlog), s->stream));
     }
     int classes = 0;
     for (int c = 0; c < fp::kClasses; c++) classes += s->runs.count[c] > 0;
@@ -1192,8 +1204,8 @@ int srv_launch(pfb_mr_server *s) {
             PFB_CUDA(cudaStreamWaitEvent(st, s->fork, 0));
         }
         unsigned tc = 0;
-        fp_quanta(e, c, nc, s->cfg.chunk_steps, quantum, &qc, &tc);
-        const fp::Launch l = fp::persist_launch(e->fe, c, nc, e->num_sms);
+        fp_quanta(e, false, c, nc, s->cfg.chunk_steps, quantum, &qc, &tc);
+        const fp::Launch l = fp::persist_launch(e->fe, false, c, nc, e->num_sms);
         const int *order = s->d_order + s->runs.first[c];
         unsigned int *cnt = s->d_counter + 1 + c;
         fp::Tab tab = e->fe.tab[c];
@@ -1416,6 +1428,13 @@ struct pfb_mr_ctx {
     JobDev *d_jobs = nullptr;
     CtxExtra *d_ex = nullptr;
     uint64_t *d_one = nullptr, *d_nm1 = nullptr, *d_tmp = nullptr, *d_n = nullptr;  // [n][n16] each
+    // moduli of the floating-point engine (transform lengths up to 2^LOG_LCTA)
+    // by class; the others, and all raw products, on the integer engine
+    ClassRuns runs;
+    int *d_order = nullptr;
+    fp::Cplx *d_scratch = nullptr;
+    int *d_slots = nullptr;  // scratch regions in use
+    int n_slots = 0;
     std::vector<HostPrep> hp;
 };
 
@@ -1445,9 +1464,14 @@ int ctx_launch(pfb_mr_ctx *c, const uint64_t *a, const uint64_t *b, uint64_t *ou
     // NULL: the legacy default stream, ordered with the caller's other
     // default-stream work (the reference's methods run there)
     cudaStream_t st = stream ? (cudaStream_t)stream : cudaStreamLegacy;
-    ctx_kernel<<<c->n, THREADS, smem_bytes(c->maxlog), st>>>(c->d_jobs, c->d_ex, a, b ? b : a, out, c->n16,
-                                                              out_stride, op, c->e->tw);
-    PFB_CUDA(cudaGetLastError());
+    if (op != CTX_RAW_SQ && op != CTX_RAW_MUL) {
+        for (int k = 0; k < fp::kClasses; k++)
+            if (c->runs.count[k])
+                PFB_CUDA(fp::ctx(c->e->fe, k, c->d_jobs, c->d_order + c->runs.first[k], c->runs.count[k], a,
+                                 b ? b : a, out, c->n16, op, c->d_scratch, c->d_slots, c->n_slots, c->d_ex, st));
+        if (!c->runs.n_int) return PFB_OK;
+    }
+    PFB_CUDA(int_ctx(c->d_jobs, c->d_ex, c->n, c->maxlog, a, b ? b : a, out, c->n16, out_stride, op, c->e->tw, st));
     return PFB_OK;
 }
 
@@ -1483,14 +1507,28 @@ extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs
             pfb::set_error("pfb_mr_ctx_create: modulus %d is not odd, > 1 and at most %d bits", i, PFB_MR_MAX_BITS);
             return ctx_fail(c, PFB_E_ARG);
         }
-        lay[i] = layout_for(c->hp[i].logl, 1, true, true);  // gy [2][L], spare H-word buffers, raw coefficients
+        HostPrep &h = c->hp[i];
+        for (int k = 0; k < fp::kClasses && h.logl <= LOG_LCTA; k++)
+            if (fp::class_points(k) == 1 << (h.logl - 1)) h.fpc = k + 1;
+        lay[i] = h.fpc ? layout_fp(h.fpc - 1, 0, false, h.logl)
+                       : layout_for(h.logl, 1, true, true);  // gy [2][L], spare H-word buffers, raw coefficients
         words += lay[i].total;
         c->maxlog = std::max(c->maxlog, c->hp[i].logl);
     }
     const size_t job_bytes = ((size_t)n_batch * sizeof(JobDev) + 255) & ~(size_t)255;
     const size_t ex_bytes = ((size_t)n_batch * sizeof(CtxExtra) + 255) & ~(size_t)255;
     const size_t v_bytes = (((size_t)n_batch * n_limbs * sizeof(uint64_t)) + 255) & ~(size_t)255;
-    const size_t need = job_bytes + ex_bytes + 4 * v_bytes + words * sizeof(uint32_t);
+    c->runs.build(n_batch, [](int) { return true; }, [&](int i) { return c->hp[i].fpc; });
+    const size_t order_bytes = ((size_t)n_batch * sizeof(int) + 255) & ~(size_t)255;
+    size_t region = 0;  // the largest class' scratch
+    for (int k = 0; k < fp::kClasses; k++)
+        if (c->runs.count[k] && fp::scratch_points(k, false)) {
+            region = std::max(region, fp::scratch_points(k, false));
+            c->n_slots = e->num_sms * std::max(1, e->fe.ctx_per_sm[k]);
+        }
+    const size_t slot_ints = ((size_t)c->n_slots * sizeof(int) + 255) & ~(size_t)255;
+    const size_t fp_bytes = order_bytes + slot_ints + region * c->n_slots * sizeof(fp::Cplx);
+    const size_t need = job_bytes + ex_bytes + 4 * v_bytes + fp_bytes + words * sizeof(uint32_t);
     if (cudaMalloc(&c->d_arena, need) != cudaSuccess) {
         cudaGetLastError();
         pfb::set_error("pfb_mr_ctx_create: cannot allocate %zu bytes of device memory", need);
@@ -1502,7 +1540,11 @@ extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs
     c->d_nm1 = (uint64_t *)(c->d_arena + job_bytes + ex_bytes + v_bytes);
     c->d_tmp = (uint64_t *)(c->d_arena + job_bytes + ex_bytes + 2 * v_bytes);
     c->d_n = (uint64_t *)(c->d_arena + job_bytes + ex_bytes + 3 * v_bytes);
-    uint32_t *d_words = (uint32_t *)(c->d_arena + job_bytes + ex_bytes + 4 * v_bytes);
+    uint8_t *d_fp = c->d_arena + job_bytes + ex_bytes + 4 * v_bytes;
+    c->d_order = (int *)d_fp;
+    c->d_slots = (int *)(d_fp + order_bytes);
+    c->d_scratch = (fp::Cplx *)(d_fp + order_bytes + slot_ints);
+    uint32_t *d_words = (uint32_t *)(d_fp + fp_bytes);
     std::vector<JobDev> jobs(n_batch);
     std::vector<CtxExtra> ex(n_batch);
     std::vector<uint64_t> one((size_t)n_batch * n_limbs), nm1((size_t)n_batch * n_limbs);
@@ -1517,17 +1559,35 @@ extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs
         j.nh = w + l.nh;
         j.npl = w + l.npl;
         j.nl = w + l.nl;
-        j.x = w + l.x;
-        j.res = w + l.res;
-        if (h.logl > LOG_LCTA) j.ybuf = w + l.yb;
+        if (!h.fpc) {
+            j.x = w + l.x;
+            j.res = w + l.res;
+            if (h.logl > LOG_LCTA) j.ybuf = w + l.yb;
+        }
         j.logl = h.logl;
+        j.fpc = h.fpc;
+        j.fbits = h.fpc ? LIMB_BITS / 2 : 0;
         j.phase = 0;
         ex[i].gy = w + l.gy;
         ex[i].yl = w + l.lt;
         ex[i].raw = (unsigned long long *)(w + l.raw);
+        ex[i].ys = h.fpc ? w + l.ys : nullptr;
         const size_t H = h.nl.size();
-        PFB_CUDA(cudaMemcpy((void *)j.npl, h.npl.data(), H * 4, cudaMemcpyHostToDevice));
-        PFB_CUDA(cudaMemcpy((void *)j.nl, h.nl.data(), H * 4, cudaMemcpyHostToDevice));
+        std::vector<uint32_t> npl = h.npl, nl = h.nl;
+        if (h.fpc) {  // two digits of 11 bits per limb: the radix R' is the same
+            auto split = [](const std::vector<uint32_t> &v) {
+                std::vector<uint32_t> d;
+                for (uint32_t x : v) {
+                    d.push_back(x & ((1u << LIMB_BITS / 2) - 1u));
+                    d.push_back(x >> LIMB_BITS / 2);
+                }
+                return d;
+            };
+            npl = split(h.npl);
+            nl = split(h.nl);
+        }
+        PFB_CUDA(cudaMemcpy((void *)j.npl, npl.data(), npl.size() * 4, cudaMemcpyHostToDevice));
+        PFB_CUDA(cudaMemcpy((void *)j.nl, nl.data(), nl.size() * 4, cudaMemcpyHostToDevice));
         // working forms of 1 and N - 1: R mod N and N - (R mod N)
         const pfb::big::Words N = pfb::big::from_u16(nums[i].limbs, (size_t)n_limbs);
         const pfb::big::Words r = pfb::big::from_limbs(h.x0.data(), LIMB_BITS, H);
@@ -1542,8 +1602,15 @@ extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs
     PFB_CUDA(cudaMemcpy(c->d_nm1, nm1.data(), nm1.size() * 8, cudaMemcpyHostToDevice));
     const std::vector<uint64_t> nall(n16.begin(), n16.end());
     PFB_CUDA(cudaMemcpy(c->d_n, nall.data(), nall.size() * 8, cudaMemcpyHostToDevice));
-    prep_kernel<<<n_batch, THREADS, smem_bytes(c->maxlog), e->stream>>>(c->d_jobs, nullptr, e->tw);
-    cudaError_t ce = cudaGetLastError();
+    cudaError_t ce = cudaSuccess;
+    if (c->n_slots) ce = cudaMemsetAsync(c->d_slots, 0, (size_t)c->n_slots * sizeof(int), e->stream);
+    if (ce == cudaSuccess && !c->runs.order.empty())
+        ce = cudaMemcpyAsync(c->d_order, c->runs.order.data(), c->runs.order.size() * sizeof(int),
+                             cudaMemcpyHostToDevice, e->stream);
+    for (int k = 0; k < fp::kClasses && ce == cudaSuccess; k++)
+        if (c->runs.count[k])
+            ce = fp::prep(e->fe, k, c->d_jobs, c->d_order + c->runs.first[k], c->runs.count[k], e->stream);
+    if (ce == cudaSuccess && c->runs.n_int) ce = int_prep(c->d_jobs, nullptr, n_batch, c->maxlog, e->tw, e->stream);
     if (ce == cudaSuccess) ce = cudaStreamSynchronize(e->stream);
     if (ce != cudaSuccess) return ctx_fail(c, pfb::cuda_fail(ce, "pfb_mr_ctx_create", __FILE__, __LINE__));
     *out = c;
@@ -1610,8 +1677,7 @@ extern "C" int pfb_mr_ctx_check_passed(pfb_mr_ctx_t *c, const uint64_t *d_r, uin
     }
     PFB_CUDA(cudaSetDevice(c->e->device));
     cudaStream_t st = stream ? (cudaStream_t)stream : cudaStreamLegacy;
-    ctx_check_kernel<<<c->n, 256, 0, st>>>(d_r, c->d_one, c->d_nm1, d_passed, c->n16);
-    PFB_CUDA(cudaGetLastError());
+    PFB_CUDA(int_ctx_check(d_r, c->d_one, c->d_nm1, d_passed, c->n, c->n16, st));
     return PFB_OK;
 }
 
@@ -1631,123 +1697,4 @@ extern "C" int pfb_mr_ctx_sq_raw(pfb_mr_ctx_t *c, const uint64_t *d_a, uint64_t 
 extern "C" int pfb_mr_ctx_mul_raw(pfb_mr_ctx_t *c, const uint64_t *d_a, const uint64_t *d_b, uint64_t *d_out,
                                   void *stream) {
     return ctx_launch(c, d_a, d_b, d_out, c ? 2 * c->n16 + 16 : 0, CTX_RAW_MUL, stream);
-}
-
-// ---------------------------------------------------------------------------
-// Measurement: two forms of one radix-16 pass (radix_probe.cuh).
-
-extern "C" int pfb_mr_radix16_forms(pfb_mr_t *e, int ctas, int reps, double *ms_butterfly, double *ms_tensor,
-                                    long long *mismatches, int *tensor_error) {
-    if (!e || ctas <= 0 || reps <= 0 || !ms_butterfly || !ms_tensor || !mismatches || !tensor_error) {
-        pfb::set_error("pfb_mr_radix16_forms: bad argument");
-        return PFB_E_ARG;
-    }
-    PFB_CUDA(cudaSetDevice(e->device));
-    const uint32_t P[2] = {P1, P2};
-    // host tables: the operand image of the byte planes of F, omega_n^t, floor(2^64 / p)
-    std::vector<uint8_t> fa(RP_OPND, 0);
-    std::vector<uint32_t> wn(4 * (size_t)RP_N);
-    RpTables t{};
-    for (int pr = 0; pr < 2; pr++) {
-        const uint64_t p = P[pr];
-        uint64_t om = 1, b = 3, ex = (p - 1) >> LOG_LMAX;  // order 2^15
-        for (; ex; ex >>= 1, b = b * b % p)
-            if (ex & 1) om = om * b % p;
-        const uint64_t wn1 = om * om % p;  // order 2^14
-        uint64_t w16 = 1;
-        for (int i = 0; i < RP_N / 16; i++) w16 = w16 * wn1 % p;  // order 16
-        uint32_t *wv = wn.data() + (size_t)(2 * pr) * RP_N, *ws = wv + RP_N;
-        uint64_t a = 1;
-        for (int i = 0; i < RP_N; i++, a = a * wn1 % p) {
-            wv[i] = (uint32_t)a;
-            ws[i] = (uint32_t)(((uint64_t)a << 32) / p);
-        }
-        for (int k = 0; k < 16; k++) {
-            uint64_t wk = 1;
-            for (int i = 0; i < k; i++) wk = wk * w16 % p;
-            uint64_t f = 1;
-            for (int m = 0; m < 16; m++, f = f * wk % p)
-                for (int byte = 0; byte < 4; byte++) fa[rp_off(pr * 64 + k * 4 + byte, m)] = (uint8_t)(f >> (8 * byte));
-        }
-        t.mu[pr] = ~0ull / p;
-    }
-    const size_t nx = (size_t)ctas * RP_N;
-    uint32_t *d_x = nullptr, *d_yb = nullptr, *d_yt = nullptr, *d_wn = nullptr;
-    uint8_t *d_fa = nullptr;
-    int *d_err = nullptr;
-    cudaError_t ce = cudaMalloc(&d_x, nx * 4);
-    if (ce == cudaSuccess) ce = cudaMalloc(&d_yb, 2 * nx * 4);
-    if (ce == cudaSuccess) ce = cudaMalloc(&d_yt, 2 * nx * 4);
-    if (ce == cudaSuccess) ce = cudaMalloc(&d_wn, wn.size() * 4);
-    if (ce == cudaSuccess) ce = cudaMalloc(&d_fa, fa.size());
-    if (ce == cudaSuccess) ce = cudaMalloc(&d_err, sizeof(int));
-    auto release = [&]() {
-        cudaFree(d_x);
-        cudaFree(d_yb);
-        cudaFree(d_yt);
-        cudaFree(d_wn);
-        cudaFree(d_fa);
-        cudaFree(d_err);
-    };
-    if (ce != cudaSuccess) {
-        release();
-        return pfb::cuda_fail(ce, "pfb_mr_radix16_forms: allocation", __FILE__, __LINE__);
-    }
-    std::vector<uint32_t> hx(nx);
-    uint64_t st = 0x9E3779B97F4A7C15ull;
-    for (auto &v : hx) {
-        st = st * 6364136223846793005ull + 1442695040888963407ull;
-        v = (uint32_t)(st >> 40) & LIMB_MASK;
-    }
-    float ms_b = 0.f, ms_t = 0.f;
-    cudaEvent_t e0 = nullptr, e1 = nullptr;
-    do {
-        if ((ce = cudaMemcpy(d_x, hx.data(), nx * 4, cudaMemcpyHostToDevice)) != cudaSuccess) break;
-        if ((ce = cudaMemcpy(d_wn, wn.data(), wn.size() * 4, cudaMemcpyHostToDevice)) != cudaSuccess) break;
-        if ((ce = cudaMemcpy(d_fa, fa.data(), fa.size(), cudaMemcpyHostToDevice)) != cudaSuccess) break;
-        if ((ce = cudaMemset(d_err, 0, sizeof(int))) != cudaSuccess) break;
-        t.fa = d_fa;
-        for (int pr = 0; pr < 2; pr++) {
-            t.wn[pr] = d_wn + (size_t)(2 * pr) * RP_N;
-            t.wnsh[pr] = t.wn[pr] + RP_N;
-        }
-        const int smem_b = (int)(2 * (RP_N + RP_N / 32) * sizeof(uint32_t));
-        if ((ce = cudaFuncSetAttribute(rp_butterfly_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem_b)) !=
-            cudaSuccess)
-            break;
-        if ((ce = cudaFuncSetAttribute(rp_tensor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, RP_SMEM)) !=
-            cudaSuccess)
-            break;
-        if ((ce = cudaEventCreate(&e0)) != cudaSuccess || (ce = cudaEventCreate(&e1)) != cudaSuccess) break;
-        cudaStream_t s = e->stream;
-        for (int form = 0; form < 2 && ce == cudaSuccess; form++) {
-            for (int r = -1; r < reps; r++) {  // one untimed launch first
-                if (r == 0) cudaEventRecord(e0, s);
-                if (form == 0) rp_butterfly_kernel<<<ctas, THREADS, smem_b, s>>>(d_x, d_yb, e->tw);
-                else rp_tensor_kernel<<<ctas, THREADS, RP_SMEM, s>>>(d_x, d_yt, t, d_err);
-            }
-            cudaEventRecord(e1, s);
-            if ((ce = cudaEventSynchronize(e1)) != cudaSuccess) break;
-            if ((ce = cudaGetLastError()) != cudaSuccess) break;
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, e0, e1);
-            (form == 0 ? ms_b : ms_t) = ms / reps;
-        }
-        if (ce != cudaSuccess) break;
-        std::vector<uint32_t> yb(2 * nx), yt(2 * nx);
-        if ((ce = cudaMemcpy(yb.data(), d_yb, yb.size() * 4, cudaMemcpyDeviceToHost)) != cudaSuccess) break;
-        if ((ce = cudaMemcpy(yt.data(), d_yt, yt.size() * 4, cudaMemcpyDeviceToHost)) != cudaSuccess) break;
-        if ((ce = cudaMemcpy(tensor_error, d_err, sizeof(int), cudaMemcpyDeviceToHost)) != cudaSuccess) break;
-        long long bad = 0;
-        for (size_t i = 0; i < yb.size(); i++) bad += yb[i] != yt[i];
-        *mismatches = bad;
-    } while (0);
-    int rc = PFB_OK;
-    if (ce != cudaSuccess) rc = pfb::cuda_fail(ce, "pfb_mr_radix16_forms", __FILE__, __LINE__);
-    if (e0) cudaEventDestroy(e0);
-    if (e1) cudaEventDestroy(e1);
-    release();
-    *ms_butterfly = ms_b;
-    *ms_tensor = ms_t;
-    return rc;
 }

@@ -16,22 +16,6 @@
 namespace pfb {
 namespace mr {
 
-enum CtxOp : int {
-    CTX_MODSQ = 0,    // out = REDC(A^2)         (working form in, working form out)
-    CTX_MODMUL = 1,   // out = REDC(A B)
-    CTX_RAW_SQ = 2,   // out = A^2, n_sum limbs  (no reduction)
-    CTX_RAW_MUL = 3,  // out = A B, n_sum limbs
-    CTX_FROM = 4,     // out = A R^-1 mod N      (working form -> plain residue)
-};
-
-// Per-modulus buffers beyond the engine's own (JobDev: spectra of N' and N,
-// limbs of N, spill buffers of the longest transform).
-struct CtxExtra {
-    uint32_t *gy;              // [2][L] spectrum of the second factor
-    uint32_t *yl;              // H limbs of the second factor
-    unsigned long long *raw;   // L coefficients of a raw product
-};
-
 // 16-bit limbs (one per uint64, the reference's Data64 layout) -> H limbs of
 // 22 bits; limbs past n16 are zero.  dst is padded (shared-memory layout)
 // when PAD.
@@ -123,6 +107,7 @@ ctx_kernel(const JobDev *jobs, const CtxExtra *ex, const uint64_t *A, const uint
     PFB_DYNAMIC_SMEM(uint32_t, raw);
     const JobDev jb = jobs[blockIdx.x];
     if (jb.phase == 3) return;  // not a valid modulus: nothing to compute
+    if (jb.fpc && op != CTX_RAW_SQ && op != CTX_RAW_MUL) return;  // the floating-point engine's
     Smem sm;
     uint32_t *Y;
     carve(raw, jb.logl, sm, Y, jb.ybuf);

@@ -429,56 +429,6 @@ __device__ __forceinline__ void product_from(uint32_t *A0, uint32_t *A1, const T
     dit_from<TWO, PR, LOGN, M, NEG>(A0, A1, tw);
 }
 
-#define PFB_LOGN_CASES(F) \
-    F(7) F(8) F(9) F(10) F(11) F(12) F(13) F(14) F(15)
-
-__device__ void dif(uint32_t *A0, uint32_t *A1, int logn, const Twiddles &tw) {
-    switch (logn) {
-#define PFB_CASE(n)                                  \
-    case n:                                          \
-        dif_from<true, 0, n, n>(A0, A1, tw);         \
-        return;
-        PFB_LOGN_CASES(PFB_CASE)
-#undef PFB_CASE
-    }
-}
-
-__device__ void dit(uint32_t *A0, uint32_t *A1, int logn, const Twiddles &tw) {
-    switch (logn) {
-#define PFB_CASE(n)                                  \
-    case n:                                          \
-        dit_from<true, 0, n, 0>(A0, A1, tw);         \
-        return;
-        PFB_LOGN_CASES(PFB_CASE)
-#undef PFB_CASE
-    }
-}
-
-// Single-prime transforms: all threads of the CTA work on prime PR.
-template <int PR>
-__device__ void dif1(uint32_t *A, int logn, const Twiddles &tw) {
-    switch (logn) {
-#define PFB_CASE(n)                                  \
-    case n:                                          \
-        dif_from<false, PR, n, n>(A, nullptr, tw);   \
-        return;
-        PFB_LOGN_CASES(PFB_CASE)
-#undef PFB_CASE
-    }
-}
-
-template <int PR>
-__device__ void dit1(uint32_t *A, int logn, const Twiddles &tw) {
-    switch (logn) {
-#define PFB_CASE(n)                                  \
-    case n:                                          \
-        dit_from<false, PR, n, 0>(A, nullptr, tw);   \
-        return;
-        PFB_LOGN_CASES(PFB_CASE)
-#undef PFB_CASE
-    }
-}
-
 // Scratch of the carry-lookahead scan.
 struct CarrySmem {
     unsigned long long wc[THREADS / 32];
@@ -574,45 +524,6 @@ __device__ __forceinline__ unsigned long long crt(uint32_t r1, uint32_t r2, int 
     t = red2(t, 2u * P2);
     t = red2(t, P2);
     return (unsigned long long)c1 + (unsigned long long)P1 * t;
-}
-
-// Pointwise Montgomery product of a transform in shared memory with a stored
-// spectrum in global memory (16-byte loads, 4 consecutive points per thread).
-template <int PR, bool CG = false>
-__device__ __forceinline__ void pointwise1(uint32_t *A, const uint32_t *__restrict__ C, int n, const CrtConsts &cc) {
-    constexpr uint32_t p = PR ? P2 : P1;
-    const uint4 *C4 = reinterpret_cast<const uint4 *>(C);
-    for (int i4 = threadIdx.x; i4 < (n >> 2); i4 += blockDim.x) {
-        const uint4 c = CG ? __ldcg(C4 + i4) : __ldg(C4 + i4);
-        const int i = 4 * i4;
-        A[pad(i)] = mont(A[pad(i)], c.x, p, cc.pinv[PR]);
-        A[pad(i + 1)] = mont(A[pad(i + 1)], c.y, p, cc.pinv[PR]);
-        A[pad(i + 2)] = mont(A[pad(i + 2)], c.z, p, cc.pinv[PR]);
-        A[pad(i + 3)] = mont(A[pad(i + 3)], c.w, p, cc.pinv[PR]);
-    }
-    __syncthreads();
-}
-
-// CG: the operand was written earlier in the same launch (L2-coherent loads).
-template <bool CG = false>
-__device__ __forceinline__ void pointwise2(uint32_t *A0, uint32_t *A1, const uint32_t *__restrict__ C0,
-                                           const uint32_t *__restrict__ C1, int n, const CrtConsts &cc) {
-    const uint4 *C04 = reinterpret_cast<const uint4 *>(C0);
-    const uint4 *C14 = reinterpret_cast<const uint4 *>(C1);
-    for (int i4 = threadIdx.x; i4 < (n >> 2); i4 += blockDim.x) {
-        const uint4 c = CG ? __ldcg(C04 + i4) : __ldg(C04 + i4);
-        const uint4 d = CG ? __ldcg(C14 + i4) : __ldg(C14 + i4);
-        const int i = 4 * i4;
-        A0[pad(i)] = mont(A0[pad(i)], c.x, P1, cc.pinv[0]);
-        A0[pad(i + 1)] = mont(A0[pad(i + 1)], c.y, P1, cc.pinv[0]);
-        A0[pad(i + 2)] = mont(A0[pad(i + 2)], c.z, P1, cc.pinv[0]);
-        A0[pad(i + 3)] = mont(A0[pad(i + 3)], c.w, P1, cc.pinv[0]);
-        A1[pad(i)] = mont(A1[pad(i)], d.x, P2, cc.pinv[1]);
-        A1[pad(i + 1)] = mont(A1[pad(i + 1)], d.y, P2, cc.pinv[1]);
-        A1[pad(i + 2)] = mont(A1[pad(i + 2)], d.z, P2, cc.pinv[1]);
-        A1[pad(i + 3)] = mont(A1[pad(i + 3)], d.w, P2, cc.pinv[1]);
-    }
-    __syncthreads();
 }
 
 // Per-CTA view of one candidate.
@@ -823,6 +734,18 @@ __device__ void mont_step(const Smem &sm, const Cand &cd, bool square, uint32_t 
     } else if (a > 2u) {
         carry_pass<true>(H, 0ull, [&](int i) { return (unsigned long long)X[pad(i)] * (a >> 1); }, X, cs);
     }
+}
+
+// Shared memory: up to L = 2^LOG_LCTA both primes' length-L transforms (A0,
+// A1), the residue X and a second residue Y; at L = 2^15 three buffers of H
+// padded words (A0, A1, X; every product there is of length H) and Y in the
+// candidate's global ybuf.
+__host__ __device__ inline size_t smem_words(int logl) {
+    const size_t L = (size_t)1 << logl, H = L / 2;
+    return logl <= LOG_LCTA ? 2 * (L + L / 32) + 2 * (H + H / 32) : 3 * (H + H / 32);
+}
+inline size_t smem_bytes(int logl) {
+    return smem_words(logl) * sizeof(uint32_t) + sizeof(CarrySmem) + 16;
 }
 
 }  // namespace mr

@@ -14,6 +14,12 @@ namespace fp {
 
 namespace {
 
+// Contexts have the integer engine's lengths: powers of two from 2^7 on.
+template <class F>
+constexpr bool in_ctx() {
+    return F::C >= 128 && (F::C & (F::C - 1)) == 0;
+}
+
 template <class F>
 int setup_class(Engine &e, std::vector<Cplx> &all) {
     size_t off[2][3] = {};
@@ -24,7 +30,18 @@ int setup_class(Engine &e, std::vector<Cplx> &all) {
     all.insert(all.end(), v.begin(), v.end());
     PFB_CUDA(cudaFuncSetAttribute(fft_persist_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::smem()));
     PFB_CUDA(cudaFuncSetAttribute(fft_prep_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::smem()));
-    PFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e.per_sm[F::ID], fft_persist_kernel<F>, F::T, F::smem()));
+    PFB_CUDA(cudaFuncSetAttribute(fft_persist_kernel<F, true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                  (int)F::smem()));
+    PFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e.per_sm[0][F::ID], fft_persist_kernel<F>, F::T,
+                                                           F::smem()));
+    PFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e.per_sm[1][F::ID], fft_persist_kernel<F, true>, F::T,
+                                                           F::smem()));
+    e.ctx_per_sm[F::ID] = 0;
+    if constexpr (in_ctx<F>()) {
+        PFB_CUDA(cudaFuncSetAttribute(fft_ctx_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::smem()));
+        PFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e.ctx_per_sm[F::ID], fft_ctx_kernel<F>, F::T,
+                                                               F::smem()));
+    }
     return PFB_OK;
 }
 
@@ -54,22 +71,25 @@ void engine_free(Engine &e) {
     e.mem = nullptr;
 }
 
-size_t scratch_points(int cls) {
+size_t scratch_points(int cls, bool lucas) {
     switch (cls) {
 #define PFB_CLS(F) \
-    case F::ID: return F::SQS ? 0 : (size_t)F::C;
+    case F::ID: return F::scratch() + (lucas ? 2 * (size_t)F::C : 0);
         PFB_FP_CLASSES(PFB_CLS)
 #undef PFB_CLS
     }
     return 0;
 }
 
-Launch persist_launch(const Engine &e, int cls, int n, int sms) {
+Launch persist_launch(const Engine &e, bool lucas, int cls, int n, int sms) {
     Launch l{};
-    const int grid = std::max(1, std::min(n, sms * std::max(1, e.per_sm[cls])));
+    const int grid = std::max(1, std::min(n, sms * std::max(1, e.per_sm[lucas][cls])));
     switch (cls) {
-#define PFB_CLS(F) \
-    case F::ID: l = Launch{(void *)fft_persist_kernel<F>, dim3(grid), dim3(F::T), F::smem()}; break;
+#define PFB_CLS(F)                                                                                    \
+    case F::ID:                                                                                       \
+        l = Launch{lucas ? (void *)fft_persist_kernel<F, true> : (void *)fft_persist_kernel<F, false>, \
+                   dim3(grid), dim3(F::T), F::smem()};                                                \
+        break;
         PFB_FP_CLASSES(PFB_CLS)
 #undef PFB_CLS
     }
@@ -80,6 +100,22 @@ cudaError_t prep(const Engine &e, int cls, JobDev *jobs, const int *d_list, int 
     switch (cls) {
 #define PFB_CLS(F)                                                                    \
     case F::ID: fft_prep_kernel<F><<<n, F::T, F::smem(), st>>>(jobs, d_list, e.tab[F::ID]); break;
+        PFB_FP_CLASSES(PFB_CLS)
+#undef PFB_CLS
+    }
+    return cudaGetLastError();
+}
+
+cudaError_t ctx(const Engine &e, int cls, const JobDev *jobs, const int *d_list, int n, const uint64_t *a,
+                const uint64_t *b, uint64_t *out, int n16, int op, Cplx *scratch, int *slots, int n_slots,
+                const CtxExtra *ex, cudaStream_t st) {
+    switch (cls) {
+#define PFB_CLS(F)                                                                                           \
+    case F::ID:                                                                                              \
+        if constexpr (in_ctx<F>())                                                                           \
+            fft_ctx_kernel<F><<<n, F::T, F::smem(), st>>>(jobs, d_list, a, b, out, n16, op, e.tab[F::ID], scratch, \
+                                                          slots, n_slots, ex);                               \
+        break;
         PFB_FP_CLASSES(PFB_CLS)
 #undef PFB_CLS
     }

@@ -13,14 +13,16 @@ namespace fp {
 struct Engine {
     Cplx *mem = nullptr;     // roots of all classes
     Tab tab[kClasses];
-    int per_sm[kClasses];    // resident CTAs per SM
+    int per_sm[2][kClasses];   // resident CTAs per SM: strong tests, Lucas tests
+    int ctx_per_sm[kClasses];  // and of a context's operations
 };
 
 int engine_create(Engine &e);
 void engine_free(Engine &e);
 
-// Points of device scratch the persistent kernel of a class needs per CTA.
-size_t scratch_points(int cls);
+// Points of device scratch a class needs per CTA (lucas: of the Lucas tests'
+// persistent kernel, else of the others).
+size_t scratch_points(int cls, bool lucas);
 
 // Arguments and launch shape of one launch of the persistent kernel.
 struct Launch {
@@ -28,7 +30,11 @@ struct Launch {
     dim3 grid, block;
     size_t smem;
 };
-Launch persist_launch(const Engine &e, int cls, int n, int sms);
+Launch persist_launch(const Engine &e, bool lucas, int cls, int n, int sms);
+
+cudaError_t ctx(const Engine &e, int cls, const JobDev *jobs, const int *d_list, int n, const uint64_t *a,
+                const uint64_t *b, uint64_t *out, int n16, int op, Cplx *scratch, int *slots, int n_slots,
+                const CtxExtra *ex, cudaStream_t st);
 
 cudaError_t prep(const Engine &e, int cls, JobDev *jobs, const int *d_list, int n, cudaStream_t st);
 

@@ -39,5 +39,23 @@ struct LucasDev {
     uint32_t lb;  // every stored value is < lb * N
 };
 
+// Operations of the modular context (pfb_mr_ctx_*).
+enum CtxOp : int {
+    CTX_MODSQ = 0,    // out = REDC(A^2)         (working form in, working form out)
+    CTX_MODMUL = 1,   // out = REDC(A B)
+    CTX_RAW_SQ = 2,   // out = A^2, n_sum limbs  (no reduction)
+    CTX_RAW_MUL = 3,  // out = A B, n_sum limbs
+    CTX_FROM = 4,     // out = A R^-1 mod N      (working form -> plain residue)
+};
+
+// Per-modulus buffers beyond the engine's own (JobDev: spectra of N' and N,
+// limbs of N, spill buffers of the longest transform).
+struct CtxExtra {
+    uint32_t *gy;              // [2][L] spectrum of the second factor
+    uint32_t *yl;              // H limbs of the second factor
+    unsigned long long *raw;   // L coefficients of a raw product
+    uint32_t *ys;              // floating-point engine: spectra of the second factor, 2 C points
+};
+
 }  // namespace mr
 }  // namespace pfb

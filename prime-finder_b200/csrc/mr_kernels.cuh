@@ -16,18 +16,6 @@ namespace mr {
 
 __constant__ CrtConsts c_crt;
 
-// Shared memory: up to L = 2^LOG_LCTA both primes' length-L transforms (A0,
-// A1), the residue X and a second residue Y; at L = 2^15 three buffers of H
-// padded words (A0, A1, X; every product there is of length H) and Y in the
-// candidate's global ybuf.
-__host__ __device__ inline size_t smem_words(int logl) {
-    const size_t L = (size_t)1 << logl, H = L / 2;
-    return logl <= LOG_LCTA ? 2 * (L + L / 32) + 2 * (H + H / 32) : 3 * (H + H / 32);
-}
-inline size_t smem_bytes(int logl) {
-    return smem_words(logl) * sizeof(uint32_t) + sizeof(CarrySmem) + 16;
-}
-
 __device__ __forceinline__ void carve(uint32_t *raw, int logl, Smem &sm, uint32_t *&Y, uint32_t *ybuf) {
     const int L = 1 << logl, H = L >> 1;
     const int BA = logl <= LOG_LCTA ? L + L / 32 : H + H / 32, BX = H + H / 32;

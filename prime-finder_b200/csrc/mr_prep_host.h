@@ -70,8 +70,8 @@ inline bool choose_fp(size_t nbits, uint32_t base, int &cls, int &bits) {
 }
 
 // mode 1: exponent d of N - 1 = 2^s d; mode 0: exponent given; mode 2: the
-// strong Lucas test, exponent d of N + 1 = 2^s d.  fft: modes 0 and 1 take
-// the floating-point engine where it can hold the number.
+// strong Lucas test, exponent d of N + 1 = 2^s d.  fft: take the
+// floating-point engine where it can hold the number.
 inline void host_prep(const pfb_mr_number_t &num, uint32_t base, int mode, const pfb_mr_number_t *ex,
                       HostPrep &hp, bool fft = false) {
     using namespace pfb::big;
@@ -105,7 +105,7 @@ inline void host_prep(const pfb_mr_number_t &num, uint32_t base, int mode, const
     size_t H = 0, rbits = 0;
     unsigned lbits = LIMB_BITS;
     int cls = 0, fb = 0;
-    if (fft && mode != 2 && choose_fp(nb, base, cls, fb))
+    if (fft && choose_fp(nb, base, cls, fb))
         for (; fb <= fp::limb_bits(cls) && !hp.fpc; fb++)
             if (neg_inv_radix(N, 2 * (size_t)fp::class_points(cls) * fb, inv)) {
                 hp.fpc = cls + 1;

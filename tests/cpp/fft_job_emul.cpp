@@ -3,8 +3,11 @@
 // (tests/cpp/emul/), with the engine's own host set-up (mr_prep_host.h) and
 // roots (fft_tables_host.h).  Input lines:
 //
-//   job mode base N [E]        whole test (mode 1) or base^E mod N (mode 0)
+//   job mode base N [E]        whole test (mode 1: strong test, 2: strong Lucas
+//                              test) or base^E mod N (mode 0)
 //                              -> class bits verdict residue
+//   ctx cls op N a b           an operation of a modular context (mr_job.cuh:
+//                              CtxOp) on plain numbers -> result
 //   step cls bits dbl kind N   one squaring of limbs of a pattern: kind 0
 //                              all B/2 + 40, 1 all -(B/2 + 40), 2 alternating,
 //                              3 random signs, 4 random limbs (the top limbs
@@ -82,7 +85,7 @@ static fp::Tab tables(std::vector<fp::Cplx> &mem) {
 
 template <class F>
 static void run_job_cls(JobDev &j) {
-    std::vector<fp::Cplx> mem, scratch(F::SQS ? 1 : F::C);
+    std::vector<fp::Cplx> mem, scratch(F::scratch() + (j.mode == 2 ? 2 * F::C : 0) + 1);
     const fp::Tab tab = tables<F>(mem);
     const int list[1] = {0};
     emu::run_grid(1, 1, F::T, [&] { fp::fft_prep_kernel<F>(&j, list, tab); }, F::smem());
@@ -90,17 +93,20 @@ static void run_job_cls(JobDev &j) {
     unsigned counter = 0;
     for (int launch = 0; j.phase != 3 && launch < 1 << 20; launch++) {
         counter = 0;
-        emu::run_grid(1, 1, F::T,
-                      [&] { fp::fft_persist_kernel<F>(&j, list, 1, locks, &counter, 8u, 64, tab, scratch.data()); },
-                      F::smem());
+        emu::run_grid(1, 1, F::T, [&] {
+            if (j.mode == 2)
+                fp::fft_persist_kernel<F, true>(&j, list, 1, locks, &counter, 8u, 64, tab, scratch.data());
+            else
+                fp::fft_persist_kernel<F>(&j, list, 1, locks, &counter, 8u, 64, tab, scratch.data());
+        }, F::smem());
     }
 }
 
 template <class F>
 static void run_step(int b, int dbl, int kind, const Words &N) {
     const size_t n = F::N;
-    std::vector<fp::Cplx> mem, scratch(F::C), nn(F::C), nh(F::C);
-    const fp::Tab tab = tables<F>(mem);
+    std::vector<fp::Cplx> mem, scratch(F::scratch() + 1), nn(F::C), nh(F::C);
+    const fp::Tab gtab = tables<F>(mem);
     Words inv;
     if (!neg_inv_radix(N, n * b, inv)) {
         std::cout << "none" << std::endl;
@@ -120,24 +126,69 @@ static void run_step(int b, int dbl, int kind, const Words &N) {
         PFB_DYNAMIC_SMEM(unsigned char, raw);
         fp::View w;
         fp::carve<F>(raw, scratch.data(), w);
+        fp::Tab tab = gtab;
+        const fp::Cplx *sn = nullptr, *sh = nullptr;
+        fp::resident<F>(w, tab, sn, sh);
         int lo[F::R1], hi[F::R1];
-        fp::balanced<F>(npl.data(), b, lo, hi);
+        fp::balanced<F>([&](int i) { return npl[i]; }, b, lo, hi);
         fp::spectrum<F>(w, tab, 0, lo, hi, nn.data());
-        fp::balanced<F>(nl.data(), b, lo, hi);
+        fp::balanced<F>([&](int i) { return nl[i]; }, b, lo, hi);
         fp::spectrum<F>(w, tab, 1, lo, hi, nh.data());
         for (int e = 0; e < F::R1; e++) {
-            lo[e] = x[threadIdx.x + e * F::T];
-            hi[e] = x[F::C + threadIdx.x + e * F::T];
+            lo[e] = x[fp::tid1<F>() + e * F::T1];
+            hi[e] = x[F::C + fp::tid1<F>() + e * F::T1];
         }
-        fp::step<F>(w, tab, nn.data(), nh.data(), b, true, dbl, lo, hi);
-        for (int e = 0; e < F::R1; e++) {
-            y[threadIdx.x + e * F::T] = lo[e];
-            y[F::C + threadIdx.x + e * F::T] = hi[e];
-        }
+        __syncthreads();  // the spectra are complete
+        tab = gtab;
+        sn = nn.data();
+        sh = nh.data();
+        fp::resident<F>(w, tab, sn, sh);
+        fp::step<F>(w, tab, sn, sh, b, true, dbl, lo, hi);
+        fp::put_limbs<F>(y.data(), lo, hi);
     }, F::smem());
     int big = 0;
     for (int v : y) big = std::max(big, v < 0 ? -v : v);
     std::cout << limbs_hex(x, b) << " " << limbs_hex(y, b) << " " << big << std::endl;
+}
+
+template <class F>
+static void run_ctx(int op, const Words &N, const Words &a, const Words &b) {
+    const size_t n = F::N;
+    const int n16 = (int)((pfb::big::bit_length(N) + 15) / 16);
+    std::vector<fp::Cplx> mem, scratch(2 * F::scratch() + 1), nn(F::C), nh(F::C), ys(2 * F::C);
+    const fp::Tab tab = tables<F>(mem);
+    Words inv;
+    if (!neg_inv_radix(N, n * fp::kCtxBits, inv)) {
+        std::cout << "none" << std::endl;
+        return;
+    }
+    std::vector<uint32_t> npl(n), nl(n);
+    pfb::big::to_limbs(inv, fp::kCtxBits, npl.data(), n);
+    pfb::big::to_limbs(N, fp::kCtxBits, nl.data(), n);
+    JobDev j{};
+    j.nn = reinterpret_cast<uint32_t *>(nn.data());
+    j.nh = reinterpret_cast<uint32_t *>(nh.data());
+    j.npl = npl.data();
+    j.nl = nl.data();
+    j.fpc = F::ID + 1;
+    j.fbits = fp::kCtxBits;
+    CtxExtra ex{};
+    ex.ys = reinterpret_cast<uint32_t *>(ys.data());
+    auto wide = [&](const Words &w) {
+        std::vector<uint16_t> t(n16);
+        pfb::big::to_u16(w, t.data(), n16);
+        return std::vector<uint64_t>(t.begin(), t.end());
+    };
+    const std::vector<uint64_t> A = wide(a), B = wide(b);
+    std::vector<uint64_t> out(n16);
+    const int list[1] = {0};
+    int slots[2] = {1, 0};  // the first region is taken
+    emu::run_grid(1, 1, F::T, [&] { fp::fft_prep_kernel<F>(&j, list, tab); }, F::smem());
+    emu::run_grid(1, 1, F::T, [&] {
+        fp::fft_ctx_kernel<F>(&j, list, A.data(), B.data(), out.data(), n16, op, tab, scratch.data(), slots, 2, &ex);
+    }, F::smem());
+    std::vector<uint16_t> o(out.begin(), out.end());
+    std::cout << to_hex(pfb::big::from_u16(o.data(), o.size())) << " " << slots[0] << slots[1] << std::endl;
 }
 
 int main() {
@@ -159,6 +210,18 @@ int main() {
             }
             continue;
         }
+        if (op == "ctx") {
+            int cls, o;
+            std::string sa, sb;
+            in >> cls >> o >> sn >> sa >> sb;
+            switch (cls) {
+#define PFB_CLS(F) \
+    case fp::F::ID: run_ctx<fp::F>(o, from_hex(sn), from_hex(sa), from_hex(sb)); break;
+                PFB_FP_CLASSES(PFB_CLS)
+#undef PFB_CLS
+            }
+            continue;
+        }
         int mode = 1;
         uint32_t base = 2;
         in >> mode >> base >> sn >> se;
@@ -170,8 +233,8 @@ int main() {
         const pfb_mr_number_t num{limbs.data(), (int)limbs.size()}, ex{el.data(), (int)el.size()};
         HostPrep hp;
         host_prep(num, base, mode, mode ? nullptr : &ex, hp, true);
-        if (!hp.ok || !hp.fpc) {
-            std::cout << hp.fpc << " 0 -1 0" << std::endl;
+        if (!hp.ok || hp.decided >= 0 || !hp.fpc) {
+            std::cout << "- 0 " << (hp.ok && hp.decided >= 0 ? hp.decided : -1) << " 0" << std::endl;
             continue;
         }
         const size_t n = hp.x0.size();
@@ -192,6 +255,18 @@ int main() {
         j.extra = mode >= 1 ? hp.s - 1 : 0;
         j.base = base;
         j.mode = mode;
+        std::vector<uint32_t> lv0(n), lv1(n), lqk(n), lt(n), lone(n);
+        LucasDev lc{};
+        if (mode == 2) {
+            lc.lv0 = lv0.data();
+            lc.lv1 = lv1.data();
+            lc.lqk = lqk.data();
+            lc.lt = lt.data();
+            lc.lone = lone.data();
+            lc.q = hp.q;
+            lc.lb = hp.lb;
+            j.lucas = &lc;
+        }
         switch (hp.fpc - 1) {
 #define PFB_CLS(F) \
     case fp::F::ID: run_job_cls<fp::F>(j); break;

@@ -13,11 +13,13 @@ import subprocess
 
 import pytest
 
+import lucas
 import oracle
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 # complex points and widest limb of every class
-CLASSES = [(64, 19), (128, 18), (256, 17), (512, 17), (1024, 16), (2048, 16), (4096, 15), (8192, 15)]
+CLASSES = [(64, 19), (96, 18), (128, 18), (192, 18), (256, 17), (384, 17), (512, 17), (768, 16), (1024, 16),
+           (1536, 16), (2048, 16), (3072, 15), (4096, 15), (6144, 15), (8192, 15), (12288, 14)]
 
 
 def _build(exe, *flags):
@@ -88,11 +90,50 @@ def test_modular_powers_of_every_class(emul):
     assert {int(o[0]) for o in out} == set(range(len(CLASSES)))
 
 
+def test_strong_lucas_tests(emul):
+    rng = random.Random(12)
+    ns = [5459, 5777, 10877, 16109, 18971, 3, 5, 7, 11, 13, 25, 49, 1000003, 1000001, (1 << 61) - 1, (1 << 127) - 1]
+    ns += [rng.getrandbits(b) | 1 | (1 << (b - 1)) for b in (30, 50, 70)]
+    for D in (5, -7, -11, 13, -15, 17, -19, -23):  # one composite and one prime per Q
+        for want_prime in (False, True):
+            while True:
+                n = rng.getrandbits(100) | (1 << 99) | 1
+                n = oracle.nextprime(n) if want_prime else n
+                if lucas.selfridge_d(n) == D:
+                    break
+            ns.append(n)
+    assert [int(o[2]) for o in emul(["job 2 2 %x" % n for n in ns])] == [lucas.strong_lucas(n) for n in ns]
+
+
+@pytest.mark.parametrize("cls", [c for c, (C, _) in enumerate(CLASSES) if C >= 128 and C & (C - 1) == 0])
+def test_context_operations(emul, cls):
+    """Fully reduced results in the integer engine's radix, 2^(22 C) + 1, with
+    operands up to N - 1 and moduli that fill the length or are short."""
+    rng = random.Random(40 + cls)
+    C = CLASSES[cls][0]
+    ri = None
+    lines, want = [], []
+    for bits in (22 * C - 6, 22 * C - 37, max(20, 11 * C - 3)):
+        N = rng.getrandbits(bits) | 1 | (1 << (bits - 1))
+        try:
+            ri = pow((1 << (22 * C)) + 1, -1, N)
+        except ValueError:
+            continue
+        for a, b in ((rng.randrange(N), rng.randrange(N)), (N - 1, N - 1), (0, 1), (1, N - 2)):
+            for op, r in ((0, a * a * ri % N), (1, a * b * ri % N), (4, a * ri % N)):
+                lines.append("ctx %d %d %x %x %x" % (cls, op, N, a, b))
+                want.append(r)
+    out = emul(lines)
+    for line, o, r in zip(lines, out, want):
+        assert int(o[0], 16) == r and o[1] == "10", line[:20]
+
+
 def test_in_bounds_under_address_sanitizer(tmp_path):
     exe = str(tmp_path / "fft_job_asan")
     _build(exe, "-O1", "-g", "-fsanitize=address")
     rng = random.Random(3)
     lines = ["job 1 2 %x" % n for n in (3, 561, (1 << 89) - 1)] + ["job 1 7 %x" % 1000003]
+    lines += ["job 2 2 %x" % n for n in (5459, (1 << 61) - 1)] + ["ctx 14 1 %x 5 7" % ((1 << 900) - 1)]
     for cls, (C, b) in enumerate(CLASSES):
         lines.append("step %d %d 1 4 %x" % (cls, b, rng.getrandbits(2 * C * b - 7) | 1 | (1 << (2 * C * b - 8))))
     r = subprocess.run([exe], input="\n".join(lines) + "\n", capture_output=True, text=True, timeout=900,
