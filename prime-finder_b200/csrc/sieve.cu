@@ -205,11 +205,10 @@ int enqueue_sieve(pfb_sieve *s, int n_abc, int K, uint32_t *d_mask, cudaStream_t
         small_setup_kernel<<<g1, 128, 0, st>>>(s->d_tiny, s->d_small, s->d_counts, s->d_abc, n_abc, K, cap,
                                                s->d_rec);
         PFB_CUDA(cudaGetLastError());
-        const uint32_t tiles = ((uint32_t)K + kTileRows - 1u) / kTileRows;
-        const uint32_t max_rows = (uint32_t)K < (uint32_t)kTileRows ? (uint32_t)K : (uint32_t)kTileRows;
-        const size_t smem = tile_smem_bytes(max_rows, K);
-        dim3 g2(tiles, (unsigned)n_abc);
-        small_tile_kernel<<<g2, kBlockTile, smem, st>>>(s->d_rec, s->d_counts, cap, s->d_abc, K, d_mask, wpt);
+        const uint32_t rows = tile_rows(K, n_abc, s->max_grid / 16);
+        dim3 g2(((uint32_t)K + rows - 1u) / rows, (unsigned)n_abc);
+        small_tile_kernel<<<g2, kBlockTile, tile_smem_bytes(rows, K), st>>>(s->d_rec, s->d_counts, cap, s->d_abc, K,
+                                                                             d_mask, wpt, rows);
         PFB_CUDA(cudaGetLastError());
     }
     if (s->n_primes)
@@ -596,10 +595,9 @@ extern "C" int pfb_sieve_run_noalloc(const uint32_t *d_primes, uint32_t n_primes
         dim3 g1((2u * cap + 127u) / 128u, 1u);
         small_setup_kernel<<<g1, 128, 0, st>>>(sc->tiny, sc->small, sc->counts, sc->abc, 1, K, 2u * cap, sc->rec);
         PFB_CUDA(cudaGetLastError());
-        const uint32_t tiles = ((uint32_t)K + kTileRows - 1u) / kTileRows;
-        const uint32_t rows = (uint32_t)K < (uint32_t)kTileRows ? (uint32_t)K : (uint32_t)kTileRows;
-        small_tile_kernel<<<dim3(tiles, 1u), kBlockTile, tile_smem_bytes(rows, K), st>>>(
-            sc->rec, sc->counts, 2u * cap, sc->abc, K, d_mask, wpt);
+        const uint32_t rows = tile_rows(K, 1, sms);
+        small_tile_kernel<<<dim3(((uint32_t)K + rows - 1u) / rows, 1u), kBlockTile, tile_smem_bytes(rows, K), st>>>(
+            sc->rec, sc->counts, 2u * cap, sc->abc, K, d_mask, wpt, rows);
         PFB_CUDA(cudaGetLastError());
         PFB_CUDA(enqueue_large(d_primes, n_primes, lim, sc->abc, 1, K, d_mask, wpt, sms, st));
     }

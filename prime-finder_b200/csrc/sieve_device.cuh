@@ -13,9 +13,10 @@ namespace {
 using pfb::Mod32;
 
 constexpr uint32_t kTinyLimit = 512;      // primes below: one warp per (prime,row)
-constexpr int kTileRows = 64;             // rows of the (k,j) grid per shared-memory tile
+constexpr int kTileRows = 64;             // most rows of the (k,j) grid per shared-memory tile
 constexpr int kBlockTile = 512;
 constexpr int kBlockLarge = 256;
+constexpr int kDirectK = 256;             // grids up to this K: rows one by one, no lattice walk
 
 __host__ __device__ inline int ndigits(int x) { return x < 10 ? 1 : x < 100 ? 2 : x < 1000 ? 3 : 4; }
 __host__ __device__ inline uint32_t pow10i(int d) {
@@ -36,6 +37,12 @@ __device__ __forceinline__ uint32_t rev_digits(uint32_t x, int l) {
 // and end inside a word, hence the two extra words.
 inline size_t tile_smem_bytes(uint32_t rows, int K) {
     return (((size_t)rows * (size_t)K + 31u) / 32u + 2u) * sizeof(uint32_t);
+}
+
+// Rows per tile: enough CTAs for every SM to hold several.
+inline uint32_t tile_rows(int K, int n_abc, int sms) {
+    const long long r = (long long)K * n_abc / ((long long)sms * 8);
+    return (uint32_t)(r < 1 ? 1 : r > kTileRows ? kTileRows : r);
 }
 
 inline uint32_t small_limit(int K) {
@@ -534,16 +541,16 @@ __device__ __forceinline__ void small_rows(const SmallRec *rt, uint32_t n_tiny, 
     }
 }
 
-// Row-tile sieve of the small primes.  grid = (tiles, triples).
+// Row-tile sieve of the small primes.  grid = (tiles of tile_rows rows, triples).
 __global__ void __launch_bounds__(kBlockTile)
 small_tile_kernel(const SmallRec *__restrict__ rec, const uint32_t *__restrict__ counts, uint32_t cap,
                   const long long *__restrict__ abc, int K, uint32_t *__restrict__ mask,
-                  size_t words_per_triple) {
+                  size_t words_per_triple, uint32_t tile_rows = kTileRows) {
     PFB_DYNAMIC_SMEM(uint32_t, tile);
     const int t = blockIdx.y;
-    const uint32_t k0 = 1u + blockIdx.x * kTileRows;
+    const uint32_t k0 = 1u + blockIdx.x * tile_rows;
     if (k0 > (uint32_t)K) return;
-    const uint32_t k1 = min((uint32_t)K + 1u, k0 + kTileRows);
+    const uint32_t k1 = min((uint32_t)K + 1u, k0 + tile_rows);
     const uint32_t rows = k1 - k0;
     const uint32_t bit_lo = (k0 - 1u) * (uint32_t)K;
     const uint32_t bit_hi = (k1 - 1u) * (uint32_t)K;
@@ -641,6 +648,54 @@ __device__ __forceinline__ void large_lines(const Mont32 &M, const LineCoeffsM &
         });
 }
 
+// Hits of one prime on both lines of a small grid (K <= kDirectK), row by
+// row: the residue of the next row is one subtraction away.  Rev rows with
+// D = 3: x = 10 x' for the k of one or two digits (x' = rev_2(k)), then the
+// K - 99 rows of three digits by one product each.  A prime has a hit in few
+// rows (K / p of them), so four rows share one test.
+template <int D>
+__device__ __forceinline__ void direct_lines(const Mont32 &M, const LineCoeffsM &lc, uint32_t kmax, uint32_t jmax,
+                                             int K, uint32_t *m) {
+    constexpr uint32_t X = D == 1 ? 9u : D == 2 ? 99u : 999u, XS = D == 1 ? 9u : 99u;
+    const uint32_t KK = (uint32_t)K;
+    {
+        uint32_t u = M.sub(lc.an, 1u);  // j - 1 of row 0
+        for (uint32_t k = 1; k <= KK; k += 4) {
+            uint32_t r[4];
+#pragma unroll
+            for (int q = 0; q < 4; q++) r[q] = u = M.sub(u, lc.bn);
+            if (min(min(r[0], r[1]), min(r[2], r[3])) < KK) {
+#pragma unroll
+                for (int q = 0; q < 4; q++)
+                    if (r[q] < KK && k + q <= KK) mark_global(m, K, k + q, r[q] + 1u);
+            }
+        }
+    }
+    if (!kmax || !jmax) return;
+    auto rev_hit = [&](uint32_t x, uint32_t u) {
+        if (u >= X) return;
+        const uint32_t k = rev_digits(x, D), j = rev_digits(u + 1u, D);
+        if (k <= kmax && j <= jmax) mark_global(m, K, k, j);
+    };
+    const uint32_t step = D == 3 ? M.mul(lc.brm, 10u) : lc.br, u0 = M.sub(lc.ar, 1u);
+    uint32_t u = u0;
+    for (uint32_t x = 1; x <= XS; x += 4) {
+        uint32_t r[4];
+#pragma unroll
+        for (int q = 0; q < 4; q++) r[q] = u = M.sub(u, step);
+        if (min(min(r[0], r[1]), min(r[2], r[3])) < X) {
+#pragma unroll
+            for (int q = 0; q < 4; q++)
+                if (x + q <= XS) rev_hit(D == 3 ? 10u * (x + q) : x + q, r[q]);
+        }
+    }
+    if (D == 3)
+        for (uint32_t k = 100; k <= kmax; k++) {
+            const uint32_t x = rev_digits(k, 3);
+            rev_hit(x, M.sub(u0, M.mul(lc.brm, x)));
+        }
+}
+
 // Primes in [p_med, inf): one thread per prime, whole lines.  At most about
 // 2 K^2 / p_med hits per thread.
 template <int D>
@@ -660,7 +715,8 @@ large_kernel(const uint32_t *__restrict__ primes, uint32_t n, uint32_t p_med,
         M.init(p);
         LineCoeffsM lc;
         line_coeffs_m(M, a, b, c, D, lc);
-        large_lines<D>(M, lc, 1u, (uint32_t)K, 1u, X, kmax, jmax, K, m);
+        if (D <= 3 && K <= kDirectK) direct_lines<D <= 3 ? D : 3>(M, lc, kmax, jmax, K, m);
+        else large_lines<D>(M, lc, 1u, (uint32_t)K, 1u, X, kmax, jmax, K, m);
     }
 }
 
