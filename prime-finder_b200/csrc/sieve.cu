@@ -21,7 +21,8 @@
 //  * Large primes (p >= S) hit each row at most once.  Their two lines are
 //    enumerated by lattice walks (O(log p) per line plus O(1) per hit): a
 //    warp per prime below (K^2 + X^2) / 12288 (lanes split the range of x),
-//    a thread per prime above; hits are OR-ed into global memory.
+//    a thread per prime above; hits are OR-ed into global memory.  On grids
+//    up to K = kDirectK a thread steps through its prime's rows instead.
 #include <cuda_runtime.h>
 #include <stdarg.h>
 #include <stdint.h>

@@ -648,52 +648,99 @@ __device__ __forceinline__ void large_lines(const Mont32 &M, const LineCoeffsM &
         });
 }
 
-// Hits of one prime on both lines of a small grid (K <= kDirectK), row by
-// row: the residue of the next row is one subtraction away.  Rev rows with
-// D = 3: x = 10 x' for the k of one or two digits (x' = rev_2(k)), then the
-// K - 99 rows of three digits by one product each.  A prime has a hit in few
-// rows (K / p of them), so four rows share one test.
-template <int D>
-__device__ __forceinline__ void direct_lines(const Mont32 &M, const LineCoeffsM &lc, uint32_t kmax, uint32_t jmax,
-                                             int K, uint32_t *m) {
-    constexpr uint32_t X = D == 1 ? 9u : D == 2 ? 99u : 999u, XS = D == 1 ? 9u : 99u;
-    const uint32_t KK = (uint32_t)K;
-    {
-        uint32_t u = M.sub(lc.an, 1u);  // j - 1 of row 0
-        for (uint32_t k = 1; k <= KK; k += 4) {
-            uint32_t r[4];
+// Rows of a small grid (K <= kDirectK) one by one.  Both lines in the form
+// u_r = u_0 - r s (mod p) with the same slope s = 10^(b-c): j - 1 at row r = k
+// of the N line, and x - 1 at row r = y of the rev line read the other way
+// round (x == (10^a - 1) 10^(b+D-a) - y 10^(b-c)); a row is hit when u_r is
+// below the line's width.
+//
+// The rows are first tested on fractions f = u 2^32 / p, which wrap at 2^32 by
+// themselves: one subtraction a row and one minimum, eight rows to a branch,
+// where the residue needs a compare and a select a row as well.  f_0 and the
+// slope's fraction are within 2 of their true values, so row r <= n is within
+// 2 n + 2 < E; hit(r) confirms the few rows that pass on the residue itself.
+template <class Hit>
+__device__ __forceinline__ void scan_rows(uint32_t f0, uint32_t g, uint32_t width, uint32_t n, Hit hit) {
+    const uint32_t E = 2u * n + 8u, lim = width + 2u * E;
+    uint32_t f = f0 + E;
+    for (uint32_t r = 1; r <= n; r += 8) {
+        uint32_t v[8];
 #pragma unroll
-            for (int q = 0; q < 4; q++) r[q] = u = M.sub(u, lc.bn);
-            if (min(min(r[0], r[1]), min(r[2], r[3])) < KK) {
+        for (int q = 0; q < 8; q++) v[q] = f - (uint32_t)(q + 1) * g;
+        f = v[7];
+        const uint32_t m = min(min(min(v[0], v[1]), min(v[2], v[3])), min(min(v[4], v[5]), min(v[6], v[7])));
+        if (m <= lim) {
 #pragma unroll
-                for (int q = 0; q < 4; q++)
-                    if (r[q] < KK && k + q <= KK) mark_global(m, K, k + q, r[q] + 1u);
-            }
+            for (int q = 0; q < 8; q++)
+                if (v[q] <= lim && r + q <= n) hit(r + q);
         }
     }
+}
+
+// The coefficients of that form: an - 1, (10^a - 1) 10^(b+D-a) - 1, and the
+// slope plain and in Montgomery form: four powers on the two squaring chains
+// of line_coeffs_m, the chain of 10^-1 as long as its exponents need.
+struct DirectCoeffs {
+    uint32_t un, ur, s, sm;
+};
+
+__device__ void direct_coeffs(const Mont32 &M, long long a, long long b, long long c, int D, DirectCoeffs &o) {
+    const uint32_t p = M.p;
+    const uint32_t one = (0u - p) % p;  // R mod p
+    const uint32_t r2 = M.add(one, one), r4 = M.add(r2, r2), r8 = M.add(r4, r4);
+    uint32_t x10 = M.add(r8, r2);
+    const uint32_t pd = p % 10u, pi = pd == 1 ? 1u : pd == 3 ? 7u : pd == 7 ? 3u : 9u;  // p^-1 mod 10
+    const uint32_t k = ((10u - one % 10u) % 10u) * pi % 10u;
+    uint32_t xi = (uint32_t)(((unsigned long long)one + (unsigned long long)k * p) / 10ull);
+    const long long e[4] = {a, -c, b - c, b + D - a};
+    uint32_t acc[4];
+    unsigned long long m[4], mp = 0, mn = 0;  // bits left in the exponents of 10 and of 10^-1
+#pragma unroll
+    for (int q = 0; q < 4; q++) {
+        m[q] = (unsigned long long)(e[q] < 0 ? -e[q] : e[q]);
+        (e[q] < 0 ? mn : mp) |= m[q];
+        acc[q] = one;
+    }
+    for (; mp | mn; mp >>= 1, mn >>= 1) {
+#pragma unroll
+        for (int q = 0; q < 4; q++) {
+            if (m[q] & 1ull) acc[q] = M.mul(acc[q], e[q] < 0 ? xi : x10);
+            m[q] >>= 1;
+        }
+        if (mp > 1ull) x10 = M.mul(x10, x10);
+        if (mn > 1ull) xi = M.mul(xi, xi);
+    }
+    const uint32_t ram1 = M.sub(acc[0], one);  // (10^a - 1) R
+    o.un = M.sub(M.mul(M.mul(ram1, acc[1]), 1u), 1u);
+    o.ur = M.sub(M.mul(M.mul(ram1, acc[3]), 1u), 1u);
+    o.sm = acc[2];
+    o.s = M.mul(acc[2], 1u);
+}
+
+// Hits of one prime on both lines.  Rev rows: with D = 3 the j of one or two
+// digits are y = 10 y' (y' = rev_2(j)), those of three digits come one by one.
+template <int D>
+__device__ __forceinline__ void direct_lines(const Mont32 &M, const DirectCoeffs &o, uint32_t kmax, uint32_t jmax,
+                                             int K, uint32_t *m) {
+    constexpr uint32_t X = D == 1 ? 9u : D == 2 ? 99u : 999u, YS = D == 1 ? 9u : 99u;
+    const uint32_t KK = (uint32_t)K;
+    const double rp = 4294967296.0 / (double)M.p;
+    auto frac = [&](uint32_t u) { return (uint32_t)((double)u * rp); };
+    scan_rows(frac(o.un), frac(o.s), frac(KK) + 1u, KK, [&](uint32_t k) {
+        const uint32_t u = M.sub(o.un, M.mul(o.sm, k));
+        if (u < KK) mark_global(m, K, k, u + 1u);
+    });
     if (!kmax || !jmax) return;
-    auto rev_hit = [&](uint32_t x, uint32_t u) {
+    auto rev_row = [&](uint32_t y) {
+        const uint32_t u = M.sub(o.ur, M.mul(o.sm, y));
         if (u >= X) return;
-        const uint32_t k = rev_digits(x, D), j = rev_digits(u + 1u, D);
+        const uint32_t k = rev_digits(u + 1u, D), j = rev_digits(y, D);
         if (k <= kmax && j <= jmax) mark_global(m, K, k, j);
     };
-    const uint32_t step = D == 3 ? M.mul(lc.brm, 10u) : lc.br, u0 = M.sub(lc.ar, 1u);
-    uint32_t u = u0;
-    for (uint32_t x = 1; x <= XS; x += 4) {
-        uint32_t r[4];
-#pragma unroll
-        for (int q = 0; q < 4; q++) r[q] = u = M.sub(u, step);
-        if (min(min(r[0], r[1]), min(r[2], r[3])) < X) {
-#pragma unroll
-            for (int q = 0; q < 4; q++)
-                if (x + q <= XS) rev_hit(D == 3 ? 10u * (x + q) : x + q, r[q]);
-        }
-    }
+    const uint32_t s1 = D == 3 ? M.mul(o.sm, 10u) : o.s;
+    scan_rows(frac(o.ur), frac(s1), frac(X) + 1u, YS, [&](uint32_t y) { rev_row(D == 3 ? 10u * y : y); });
     if (D == 3)
-        for (uint32_t k = 100; k <= kmax; k++) {
-            const uint32_t x = rev_digits(k, 3);
-            rev_hit(x, M.sub(u0, M.mul(lc.brm, x)));
-        }
+        for (uint32_t j = 100; j <= jmax; j++) rev_row(rev_digits(j, 3));
 }
 
 // Primes in [p_med, inf): one thread per prime, whole lines.  At most about
@@ -713,10 +760,15 @@ large_kernel(const uint32_t *__restrict__ primes, uint32_t n, uint32_t p_med,
         if (!large_prime(p, p_med, 0xFFFFFFFFu, X)) continue;
         Mont32 M;
         M.init(p);
-        LineCoeffsM lc;
-        line_coeffs_m(M, a, b, c, D, lc);
-        if (D <= 3 && K <= kDirectK) direct_lines<D <= 3 ? D : 3>(M, lc, kmax, jmax, K, m);
-        else large_lines<D>(M, lc, 1u, (uint32_t)K, 1u, X, kmax, jmax, K, m);
+        if (D <= 3 && K <= kDirectK) {
+            DirectCoeffs o;
+            direct_coeffs(M, a, b, c, D, o);
+            direct_lines<D <= 3 ? D : 3>(M, o, kmax, jmax, K, m);
+        } else {
+            LineCoeffsM lc;
+            line_coeffs_m(M, a, b, c, D, lc);
+            large_lines<D>(M, lc, 1u, (uint32_t)K, 1u, X, kmax, jmax, K, m);
+        }
     }
 }
 
