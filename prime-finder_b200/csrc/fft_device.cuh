@@ -72,6 +72,17 @@ struct Cls {
     static constexpr int RM = R4_ > 1 ? R4_ : R3_;  // radix of the middle sweep
     static constexpr int PADL = RM >= 16 ? 4 : 3;
     static constexpr int WARPS = T / 32;
+    // After the first pass the R1 blocks are transforms of their own: each team
+    // of warps keeps to its share of them (C / TEAMS consecutive points) until
+    // the last inverse pass, so only its own warps wait for one another there.
+    // Where that leaves a team's lanes idle, or saves a barrier of 128 threads
+    // at most (1024 and 2048 points: 8 and 11 % slower), all warps are one team.
+    static constexpr int TEAMS = C_ == 1024 || C_ == 2048                    ? 1
+                                 : R1_ % WARPS == 0                          ? WARPS
+                                 : WARPS % 2 == 0 && R1_ % (WARPS / 2) == 0 ? WARPS / 2
+                                 : WARPS % 4 == 0 && R1_ % (WARPS / 4) == 0 ? WARPS / 4
+                                                                            : 1;
+    static constexpr int TT = T / TEAMS;  // threads of a team
     // short numbers, whose steps are a chain of latencies: the roots and the
     // spectra of N'' and N are copied to shared memory for a quantum
     static constexpr bool RES = C_ <= kResident;
@@ -90,11 +101,11 @@ struct Cls {
 };
 
 constexpr int kClasses = 16;
-using Cls0 = Cls<0, 64, 2, 4, 8, 1, 32, true, true, 8>;
-using Cls1 = Cls<1, 96, 3, 4, 8, 1, 32, true, true, 8>;
-using Cls2 = Cls<2, 128, 4, 4, 8, 1, 32, true, true, 8>;
-using Cls3 = Cls<3, 192, 3, 8, 8, 1, 64, true, true, 8>;
-using Cls4 = Cls<4, 256, 4, 8, 8, 1, 64, true, true, 8>;
+using Cls0 = Cls<0, 64, 4, 4, 4, 1, 32, true, true, 8>;
+using Cls1 = Cls<1, 96, 3, 8, 4, 1, 32, true, true, 8>;
+using Cls2 = Cls<2, 128, 4, 8, 4, 1, 32, true, true, 8>;
+using Cls3 = Cls<3, 192, 3, 4, 4, 4, 64, true, true, 6>;
+using Cls4 = Cls<4, 256, 4, 4, 4, 4, 64, true, true, 6>;
 using Cls5 = Cls<5, 384, 6, 8, 8, 1, 64, true, true, 6>;
 using Cls6 = Cls<6, 512, 8, 8, 8, 1, 64, true, true, 6>;
 using Cls7 = Cls<7, 768, 6, 16, 8, 1, 128, true, true, 4>;
@@ -138,12 +149,12 @@ struct Tab {
     const Cplx *t[2][3];
 };
 
-// The first pass' roots, the same for every length: entry q of a radix-16
+// The first pass' roots, the same for every length: entry q of a radix-32
 // group at the root of the tree.
 // (tree of binary levels), and for a radix 3 r group the root r and r^2 of
 // the ternary level, then for each child the roots of a radix-8 group.
 struct First {
-    Cplx r[2][8];
+    Cplx r[2][16];
     Cplx t[2][2 + 3 * 4];
 };
 __constant__ First c_first;
@@ -179,6 +190,18 @@ __device__ __forceinline__ void cta_sync() {
 #ifdef __CUDA_ARCH__
     if (F::T == 32) __syncwarp();
     else __syncthreads();
+#else
+    __syncthreads();
+#endif
+}
+
+// The threads of this thread's team.
+template <class F>
+__device__ __forceinline__ void team_sync() {
+#ifdef __CUDA_ARCH__
+    if (F::TT == 32) __syncwarp();
+    else if (F::TEAMS == 1) __syncthreads();
+    else asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / F::TT), "n"(F::TT) : "memory");
 #else
     __syncthreads();
 #endif
@@ -316,12 +339,14 @@ __device__ __forceinline__ void load_roots(Cplx *tw, const Cplx *tab, int nodes,
 }
 
 // One pass of radix R over the C points in A: NODES nodes of C / NODES
-// points, element stride SUB.
-template <class F, int R, int NODES, bool INV>
+// points, element stride SUB.  ALL: the next pass is not the team's own.
+template <class F, int R, int NODES, bool INV, bool ALL>
 __device__ __forceinline__ void pass(Cplx *A, const Cplx *tab) {
-    constexpr int SUB = F::C / NODES / R, G = F::C / R;
+    constexpr int SUB = F::C / NODES / R, G = F::C / R / F::TEAMS;  // groups of a team
+    const int g0 = ((int)threadIdx.x / F::TT) * G;
 #pragma unroll 1
-    for (int g = threadIdx.x; g < G; g += F::T) {
+    for (int i = (int)threadIdx.x % F::TT; i < G; i += F::TT) {
+        const int g = g0 + i;
         const int node = g / SUB, j0 = g % SUB, base = node * (R * SUB) + j0;
         Cplx tw[R / 2], v[R];
         load_roots<F, R>(tw, tab, NODES, node);
@@ -332,7 +357,8 @@ __device__ __forceinline__ void pass(Cplx *A, const Cplx *tab) {
 #pragma unroll
         for (int e = 0; e < R; e++) A[padx<F>(base + e * SUB)] = v[e];
     }
-    cta_sync<F>();
+    if (ALL) cta_sync<F>();
+    else team_sync<F>();
 }
 
 enum MidOp { MID_STORE_SQ, MID_STORE_MUL, MID_STORE, MID_SQ, MID_MUL, MID_MULADD };
@@ -347,9 +373,11 @@ enum MidOp { MID_STORE_SQ, MID_STORE_MUL, MID_STORE, MID_SQ, MID_MUL, MID_MULADD
 //   MID_SQ: v^2    MID_MUL: v G    MID_MULADD: v G + S
 template <class F>
 __device__ __forceinline__ void mid(Cplx *A, const Cplx *tab, int op, const Cplx *Gs, Cplx *S, bool res = false) {
-    constexpr int R = F::RM, G = F::C / R;
+    constexpr int R = F::RM, G = F::C / R, GT = G / F::TEAMS;
+    const int g0 = ((int)threadIdx.x / F::TT) * GT;
 #pragma unroll 1
-    for (int g = threadIdx.x; g < G; g += F::T) {
+    for (int i = (int)threadIdx.x % F::TT; i < GT; i += F::TT) {
+        const int g = g0 + i;
         Cplx tw[R / 2], v[R];
         load_roots<F, R>(tw, tab, G, g);
         const int base = padx<F>(g * R);
@@ -389,7 +417,8 @@ __device__ __forceinline__ void mid(Cplx *A, const Cplx *tab, int op, const Cplx
 #pragma unroll
         for (int e = 0; e < R; e++) A[R <= (1 << F::PADL) ? base + e : padx<F>(g * R + e)] = v[e];
     }
-    cta_sync<F>();
+    if (op == MID_STORE_SQ || op == MID_STORE_MUL || op == MID_STORE) cta_sync<F>();
+    else team_sync<F>();
 }
 
 // ---- one candidate's working set -------------------------------------------
@@ -592,13 +621,13 @@ __device__ __forceinline__ void last_pass(const View &w, int b, int dbl, int *lo
 // The passes between the first and the middle one.
 template <class F>
 __device__ __forceinline__ void fwd_inner(Cplx *A, const Cplx *const *t) {
-    pass<F, F::R2, F::R1, false>(A, t[0]);
-    if constexpr (F::NPASS == 4) pass<F, F::R3, F::R1 * F::R2, false>(A, t[1]);
+    pass<F, F::R2, F::R1, false, false>(A, t[0]);
+    if constexpr (F::NPASS == 4) pass<F, F::R3, F::R1 * F::R2, false, false>(A, t[1]);
 }
 template <class F>
 __device__ __forceinline__ void inv_inner(Cplx *A, const Cplx *const *t) {
-    if constexpr (F::NPASS == 4) pass<F, F::R3, F::R1 * F::R2, true>(A, t[1]);
-    pass<F, F::R2, F::R1, true>(A, t[0]);
+    if constexpr (F::NPASS == 4) pass<F, F::R3, F::R1 * F::R2, true, false>(A, t[1]);
+    pass<F, F::R2, F::R1, true, true>(A, t[0]);
 }
 
 // x's limbs as the last step found them.
@@ -684,7 +713,14 @@ __device__ __forceinline__ uint32_t fn_then(uint32_t f, uint32_t g) {  // g afte
     return fn_at(g, fn_at(f, 0u)) | (fn_at(g, fn_at(f, 1u)) << 2) | (fn_at(g, fn_at(f, 2u)) << 4);
 }
 
-// The n limbs L (each within (-3B/4, 2B)) to digits in [0, B); returns the carry
+// Where limb i lies in such an array: a thread's run of n / T limbs is followed
+// by one unused word, so that the runs of a warp start in different banks.
+template <class F>
+__device__ __forceinline__ int lpos(int i) {
+    return i + i / (F::N / F::T);
+}
+
+// The n limbs L (at lpos; each within (-3B/4, 2B)) to digits in [0, B); returns the carry
 // out of the top limb (-1: the number is negative).
 template <class F>
 __device__ int normalize(int *L, int b, uint32_t *sc) {
@@ -694,9 +730,9 @@ __device__ int normalize(int *L, int b, uint32_t *sc) {
     int c = 0;
     bool zero = true, ones = true;
     for (int q = 0; q < W; q++) {
-        const int v = L[t * W + q] + c, d = v & mask;
+        const int v = L[t * (W + 1) + q] + c, d = v & mask;
         c = v >> b;
-        L[t * W + q] = d;
+        L[t * (W + 1) + q] = d;
         zero = zero && d == 0;
         ones = ones && d == mask;
     }
@@ -714,9 +750,9 @@ __device__ int normalize(int *L, int b, uint32_t *sc) {
     const uint32_t before = __shfl_up_sync(FULL, f, 1);
     int carry = (int)(lane ? fn_at(before, cin) : cin) - 1;
     for (int q = 0; q < W && carry; q++) {
-        const int v = L[t * W + q] + carry;
+        const int v = L[t * (W + 1) + q] + carry;
         carry = v >> b;
-        L[t * W + q] = v & mask;
+        L[t * (W + 1) + q] = v & mask;
     }
     cta_sync<F>();
     return (int)tot - 1;
@@ -732,15 +768,19 @@ __device__ __forceinline__ void put_limbs(W *L, const int *lo, const int *hi) {
     }
 }
 
-// L[0..n) <- the canonical digits (base B) of the value of the limbs modulo
+// L (at lpos) <- the canonical digits (base B) of the value of the limbs modulo
 // N, for a value in (-N, N); nl: N's digits.  L overlays A.
 template <class F>
 __device__ void to_digits(const View &w, int b, const uint32_t *nl, const int *lo, const int *hi, int *L) {
     cta_sync<F>();
-    put_limbs<F>(L, lo, hi);
+#pragma unroll
+    for (int e = 0; e < F::R1; e++) {
+        L[lpos<F>(tid1<F>() + e * F::T1)] = lo[e];
+        L[lpos<F>(F::C + tid1<F>() + e * F::T1)] = hi[e];
+    }
     cta_sync<F>();
     if (normalize<F>(L, b, w.sc) < 0) {
-        for (int i = threadIdx.x; i < F::N; i += F::T) L[i] += (int)nl[i];
+        for (int i = threadIdx.x; i < F::N; i += F::T) L[lpos<F>(i)] += (int)nl[i];
         cta_sync<F>();
         normalize<F>(L, b, w.sc);
     }

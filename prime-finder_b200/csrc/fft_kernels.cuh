@@ -98,7 +98,7 @@ __device__ void run_fft_job(JobDev *jp, int max_steps, Tab tab, unsigned char *r
             to_digits<F>(w, b, jb.nl, lo, hi, L);
             bool one = true, nm1 = true;  // N odd: N - 1 differs from N in digit 0 only
             for (int i = threadIdx.x; i < F::N; i += F::T) {
-                const uint32_t y = (uint32_t)L[i], n = jb.nl[i];
+                const uint32_t y = (uint32_t)L[lpos<F>(i)], n = jb.nl[i];
                 one = one && (y == (i == 0 ? 1u : 0u));
                 nm1 = nm1 && (y == (i == 0 ? n - 1u : n));
                 if (phase == 1) jb.res[i] = y;
@@ -202,7 +202,7 @@ __device__ void run_fft_lucas(JobDev *jp, int max_steps, Tab tab, unsigned char 
                 int *L = reinterpret_cast<int *>(w.A);
                 to_digits<F>(w, b, jb.nl, lo, hi, L);
                 bool z = true;
-                for (int i = threadIdx.x; i < F::N; i += F::T) z = z && L[i] == 0;
+                for (int i = threadIdx.x; i < F::N; i += F::T) z = z && L[lpos<F>(i)] == 0;
                 hit = vote_and<F>(z);
             }
         }
@@ -341,7 +341,7 @@ fft_ctx_kernel(const JobDev *jobs, const int *list, const uint64_t *A, const uin
         unsigned long long v = 0;
 #pragma unroll
         for (int q = 0; q < 3; q++)
-            if (i + q < F::N) v |= (unsigned long long)(uint32_t)L[i + q] << (kCtxBits * q);
+            if (i + q < F::N) v |= (unsigned long long)(uint32_t)L[lpos<F>(i + q)] << (kCtxBits * q);
         o[k] = (v >> off) & 0xFFFFull;
     }
     if (F::scratch()) {

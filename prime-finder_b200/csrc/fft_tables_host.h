@@ -63,7 +63,7 @@ inline long long child_angle(int mod, int k) { return top_angle(mod) / 3 + kTurn
 inline First first_roots() {
     First f{};
     for (int mod = 0; mod < 2; mod++) {
-        for (int q = 0; q < 8; q++) f.r[mod][q] = group_root(top_angle(mod), 0, 0, q);
+        for (int q = 0; q < 16; q++) f.r[mod][q] = group_root(top_angle(mod), 0, 0, q);
         f.t[mod][0] = unit_root(child_angle(mod, 0));
         f.t[mod][1] = unit_root(2 * child_angle(mod, 0));
         for (int k = 0; k < 3; k++)

@@ -106,15 +106,25 @@ cudaError_t prep(const Engine &e, int cls, JobDev *jobs, const int *d_list, int 
     return cudaGetLastError();
 }
 
+namespace {
+
+template <class F>
+void launch_ctx(const Tab &tab, const JobDev *jobs, const int *list, int n, const uint64_t *a, const uint64_t *b,
+                uint64_t *out, int n16, int op, Cplx *scratch, int *slots, int n_slots, const CtxExtra *ex,
+                cudaStream_t st) {
+    if constexpr (in_ctx<F>())
+        fft_ctx_kernel<F><<<n, F::T, F::smem(), st>>>(jobs, list, a, b, out, n16, op, tab, scratch, slots, n_slots, ex);
+}
+
+}  // namespace
+
 cudaError_t ctx(const Engine &e, int cls, const JobDev *jobs, const int *d_list, int n, const uint64_t *a,
                 const uint64_t *b, uint64_t *out, int n16, int op, Cplx *scratch, int *slots, int n_slots,
                 const CtxExtra *ex, cudaStream_t st) {
     switch (cls) {
-#define PFB_CLS(F)                                                                                           \
-    case F::ID:                                                                                              \
-        if constexpr (in_ctx<F>())                                                                           \
-            fft_ctx_kernel<F><<<n, F::T, F::smem(), st>>>(jobs, d_list, a, b, out, n16, op, e.tab[F::ID], scratch, \
-                                                          slots, n_slots, ex);                               \
+#define PFB_CLS(F)                                                                                                \
+    case F::ID:                                                                                                   \
+        launch_ctx<F>(e.tab[F::ID], jobs, d_list, n, a, b, out, n16, op, scratch, slots, n_slots, ex, st);        \
         break;
         PFB_FP_CLASSES(PFB_CLS)
 #undef PFB_CLS
