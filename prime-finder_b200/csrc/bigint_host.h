@@ -319,40 +319,51 @@ inline Words sub(const Words &a, const Words &b) {
     return r;
 }
 
-// r = a * x - b * y for a * x >= b * y (a, b single words); r is reused.
-inline void mulsub_small(Words &r, const Words &x, uint64_t a, const Words &y, uint64_t b) {
-    const size_t n = std::max(x.size(), y.size()) + 1;
-    r.assign(n, 0);
-    unsigned __int128 cx = 0, cy = 0;
-    uint64_t borrow = 0;
+// (u, v) <- (+-(a u - b v), +-(c u - d v)) in one sweep, the signs (minus
+// when nu, nv) chosen by the caller so that both results are >= 0; a, b, c, d
+// < 2^62, so that a word's two products and the carry fit a signed 128-bit sum.
+template <bool NU, bool NV>
+inline void mulsub_pair(Words &u, Words &v, uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
+    typedef unsigned __int128 u128;
+    const size_t n = std::max(u.size(), v.size());
+    u.resize(n, 0);
+    v.resize(n, 0);
+    __int128 su = 0, sv = 0;
+    uint64_t *pu = u.data(), *pv = v.data();
     for (size_t i = 0; i < n; i++) {
-        cx += (unsigned __int128)(i < x.size() ? x[i] : 0) * a;
-        cy += (unsigned __int128)(i < y.size() ? y[i] : 0) * b;
-        const uint64_t px = (uint64_t)cx, py = (uint64_t)cy;
-        cx >>= 64;
-        cy >>= 64;
-        const unsigned __int128 d = (unsigned __int128)px - py - borrow;
-        r[i] = (uint64_t)d;
-        borrow = (uint64_t)(d >> 127);
+        const uint64_t x = pu[i], y = pv[i];
+        const __int128 ax = (__int128)((u128)x * a), by = (__int128)((u128)y * b);
+        const __int128 cx = (__int128)((u128)x * c), dy = (__int128)((u128)y * d);
+        su += NU ? by - ax : ax - by;
+        sv += NV ? dy - cx : cx - dy;
+        pu[i] = (uint64_t)su;
+        pv[i] = (uint64_t)sv;
+        su >>= 64;
+        sv >>= 64;
     }
-    trim(r);
+    trim(u);
+    trim(v);
 }
 
-// r = a * x + b * y (a, b single words); r is reused.
-inline void muladd_small(Words &r, const Words &x, uint64_t a, const Words &y, uint64_t b) {
-    const size_t n = std::max(x.size(), y.size()) + 2;
-    r.assign(n, 0);
-    unsigned __int128 cx = 0, cy = 0, c = 0;
+// (x, y) <- (a x + b y, c x + d y) in one sweep (a, b, c, d < 2^62).
+inline void muladd_pair(Words &x, Words &y, uint64_t a, uint64_t b, uint64_t c, uint64_t d) {
+    typedef unsigned __int128 u128;
+    const size_t n = std::max(x.size(), y.size()) + 1;
+    x.resize(n, 0);
+    y.resize(n, 0);
+    u128 sx = 0, sy = 0;
+    uint64_t *px = x.data(), *py = y.data();
     for (size_t i = 0; i < n; i++) {
-        cx += (unsigned __int128)(i < x.size() ? x[i] : 0) * a;
-        cy += (unsigned __int128)(i < y.size() ? y[i] : 0) * b;
-        c += (unsigned __int128)(uint64_t)cx + (uint64_t)cy;
-        cx >>= 64;
-        cy >>= 64;
-        r[i] = (uint64_t)c;
-        c >>= 64;
+        const uint64_t s = px[i], t = py[i];
+        sx += (u128)s * a + (u128)t * b;
+        sy += (u128)s * c + (u128)t * d;
+        px[i] = (uint64_t)sx;
+        py[i] = (uint64_t)sy;
+        sx >>= 64;
+        sy >>= 64;
     }
-    trim(r);
+    trim(x);
+    trim(y);
 }
 
 inline Words add(const Words &a, const Words &b) {
@@ -384,7 +395,7 @@ inline unsigned __int128 bits128(const Words &x, size_t sh) {
 // (mod M), and tu, tv alternate in sign, so every cofactor update adds
 // magnitudes.  Returns false when gcd(a, M) != 1.
 inline bool inv_mod(const Words &a, const Words &M, Words *inv) {
-    Words u = M, v = a, tu, tv(1, 1), u2, v2, t1, t2;
+    Words u = M, v = a, tu, tv(1, 1);
     trim(v);
     int su = -1, sv = 1;  // signs of tu (zero: either) and tv
     const __int128 LIM = (__int128)1 << 62;
@@ -434,22 +445,18 @@ inline bool inv_mod(const Words &a, const Words &M, Words *inv) {
             continue;
         }
         auto mag = [](__int128 x) { return (uint64_t)(x < 0 ? -x : x); };
-        // u' = A u + B v, v' = C u + D v (A, B and C, D of opposite signs or
-        // zero, u', v' >= 0): the positive term is the one of the
-        // non-positive partner's sign opposite (A = 0 after a single step)
-        if (B <= 0) mulsub_small(u2, u, mag(A), v, mag(B));
-        else mulsub_small(u2, v, mag(B), u, mag(A));
-        if (D <= 0) mulsub_small(v2, u, mag(C), v, mag(D));
-        else mulsub_small(v2, v, mag(D), u, mag(C));
         // cofactors: A tu and B tv have one sign, as have C tu and D tv
         const int s1 = A != 0 ? (A > 0 ? su : -su) : (B > 0 ? sv : -sv);
         const int s2 = C != 0 ? (C > 0 ? su : -su) : (D > 0 ? sv : -sv);
-        muladd_small(t1, tu, mag(A), tv, mag(B));
-        muladd_small(t2, tu, mag(C), tv, mag(D));
-        std::swap(u, u2);
-        std::swap(v, v2);
-        std::swap(tu, t1);
-        std::swap(tv, t2);
+        // u' = A u + B v, v' = C u + D v (A, B and C, D of opposite signs or
+        // zero, u', v' >= 0): a non-positive second factor leaves the first
+        // product on top
+        const uint64_t a1 = mag(A), b1 = mag(B), c1 = mag(C), d1 = mag(D);
+        if (B <= 0 && D <= 0) mulsub_pair<false, false>(u, v, a1, b1, c1, d1);
+        else if (B <= 0) mulsub_pair<false, true>(u, v, a1, b1, c1, d1);
+        else if (D <= 0) mulsub_pair<true, false>(u, v, a1, b1, c1, d1);
+        else mulsub_pair<true, true>(u, v, a1, b1, c1, d1);
+        muladd_pair(tu, tv, a1, b1, c1, d1);
         su = s1;
         sv = s2;
     }
