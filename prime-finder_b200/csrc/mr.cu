@@ -1,7 +1,8 @@
 // Batched Miller-Rabin engine: kernels and host driver.
 //
-// One CTA per candidate runs its whole chain of Montgomery squarings on chip
-// (mr_device.cuh).  The host side does the per-modulus set-up the reference
+// One CTA per candidate runs its whole chain of Montgomery squarings on chip:
+// on double-precision FFTs (fft_device.cuh) up to 344 058 bits, on the integer
+// transforms (mr_device.cuh) above.  The host side does the per-modulus set-up the reference
 // does with GMP (barrett.cu:58-107, montgomery.cu:30-45,
 // miller_rabin_runner.cu:315-325): N' = -N^-1 mod R, R mod N, N - 1 = 2^s d.
 #include <cuda_runtime.h>
