@@ -96,7 +96,9 @@ int pfb_mr_powm(pfb_mr_t *e, const pfb_mr_number_t *nums, int n, uint32_t base,
  *   advance  enqueue about `steps` steps of every unfinished candidate on
  *            `stream` (NULL = engine stream): a persistent kernel, one CTA
  *            per SM, hands out quanta of 64 steps round-robin, so the SMs
- *            stay busy whatever the number and lengths of the candidates
+ *            stay busy whatever the number and lengths of the candidates;
+ *            advances on different streams may overlap (a candidate is taken
+ *            by one CTA at a time)
  *   pending  number of unfinished candidates (synchronises the device)
  *   results  verdicts / residues as in pfb_mr_test; PFB_E_STATE while some
  *            candidate is unfinished (its verdict is reported as -2)

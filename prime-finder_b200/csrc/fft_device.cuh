@@ -59,9 +59,9 @@ struct alignas(16) Cplx {
 // pass (T = T1 = C / R1; the second half of a warp repeats the first when T1 =
 // 16): the last inverse pass, the carries and the next first pass stay in
 // registers.  SQS: x^2's spectrum waits in
-// shared memory, XSS: so do x's limbs (else both in global memory); PADL: one
-// unused point per 2^PADL in shared memory against bank conflicts of the last
-// pass.
+// shared memory, XSS: so do x's limbs (else in the candidate's global memory:
+// jb.sq, jb.x); PADL: one unused point per 2^PADL in shared memory against
+// bank conflicts of the last pass.
 constexpr int kResident = 1024;
 template <int ID_, int C_, int R1_, int R2_, int R3_, int R4_, int T_, bool SQS_, bool XSS_, int MINB_>
 struct Cls {
@@ -96,8 +96,6 @@ struct Cls {
         return (size_t)A_PTS * 16 + (SQS_ ? (size_t)C_ * 16 : 0) + (XSS_ ? (size_t)C_ * 8 : 0) +
                (size_t)2 * WARPS * R1_ * 8 + 256 + (RES ? (size_t)(2 * C_ + ROOTS) * 16 : 0);
     }
-    // points of global scratch per CTA
-    static constexpr size_t scratch() { return (SQS_ ? 0 : C_) + (XSS_ ? 0 : C_ / 2); }
 };
 
 constexpr int kClasses = 16;
@@ -120,6 +118,14 @@ using Cls15 = Cls<15, 12288, 24, 8, 8, 8, 512, false, false, 1>;
 #define PFB_FP_CLASSES(F)                                                                                     \
     F(Cls0) F(Cls1) F(Cls2) F(Cls3) F(Cls4) F(Cls5) F(Cls6) F(Cls7) F(Cls8) F(Cls9) F(Cls10) F(Cls11) F(Cls12) \
         F(Cls13) F(Cls14) F(Cls15)
+
+// Whether x^2's spectrum of a class lies in global memory (C points).
+inline bool spectrum_outside(int cls) {
+#define PFB_CLS(F) !F::SQS,
+    static const bool o[kClasses] = {PFB_FP_CLASSES(PFB_CLS)};
+#undef PFB_CLS
+    return o[cls];
+}
 
 inline int class_points(int cls) {
 #define PFB_CLS(F) F::C,
@@ -425,21 +431,24 @@ __device__ __forceinline__ void mid(Cplx *A, const Cplx *tab, int op, const Cplx
 struct View {
     Cplx *A;       // points, padded
     Cplx *S;       // a spectrum, [element][group]
-    int *xs;       // limbs of x: [2 e + half][thread], each thread's own
+    int *xs;       // limbs of x, [half][e][thread]: n words, each thread its own
     int *bnd;      // carries between warps
     uint32_t *sc;  // scratch words of the carry scan and of votes
     Cplx *res;     // RES: roots, then the spectra of N'' and N
 };
 
+// sq (C points), xs (n limbs): where S and xs lie when they are not in shared
+// memory: the candidate's own, so that launches which overlap, on other
+// candidates as the locks see to, share nothing.
 template <class F>
-__device__ __forceinline__ void carve(unsigned char *raw, Cplx *gscratch, View &w) {
+__device__ __forceinline__ void carve(unsigned char *raw, Cplx *sq, int *xs, View &w) {
     w.A = reinterpret_cast<Cplx *>(raw);
     raw += (size_t)F::A_PTS * 16;
     if (F::SQS) {
         w.S = reinterpret_cast<Cplx *>(raw);
         raw += (size_t)F::C * 16;
     } else {
-        w.S = gscratch;
+        w.S = sq;
     }
     w.res = reinterpret_cast<Cplx *>(raw);
     if (F::RES) raw += (size_t)(2 * F::C + F::ROOTS) * 16;
@@ -447,7 +456,7 @@ __device__ __forceinline__ void carve(unsigned char *raw, Cplx *gscratch, View &
         w.xs = reinterpret_cast<int *>(raw);
         raw += (size_t)F::C * 8;
     } else {
-        w.xs = reinterpret_cast<int *>(gscratch + (F::SQS ? 0 : F::C));
+        w.xs = xs;
     }
     w.bnd = reinterpret_cast<int *>(raw);
     raw += (size_t)2 * F::WARPS * F::R1 * 8;
@@ -635,8 +644,8 @@ template <class F>
 __device__ __forceinline__ void load_x(const View &w, int *lo, int *hi) {
 #pragma unroll
     for (int e = 0; e < F::R1; e++) {
-        lo[e] = w.xs[(2 * e) * F::T1 + tid1<F>()];
-        hi[e] = w.xs[(2 * e + 1) * F::T1 + tid1<F>()];
+        lo[e] = w.xs[e * F::T1 + tid1<F>()];
+        hi[e] = w.xs[F::C + e * F::T1 + tid1<F>()];
     }
 }
 
@@ -650,8 +659,8 @@ __device__ __forceinline__ void step(const View &w, const Tab &tab, const Cplx *
     constexpr int R = F::R1, MT = F::NPASS - 2;
 #pragma unroll
     for (int e = 0; e < R; e++) {
-        w.xs[(2 * e) * F::T1 + tid1<F>()] = lo[e];
-        w.xs[(2 * e + 1) * F::T1 + tid1<F>()] = hi[e];
+        w.xs[e * F::T1 + tid1<F>()] = lo[e];
+        w.xs[F::C + e * F::T1 + tid1<F>()] = hi[e];
     }
     // phases: 0 spectrum of x (of its square, of x y) modulo M2 into S, 1 D, 2 m, 3 U
 #pragma unroll 1

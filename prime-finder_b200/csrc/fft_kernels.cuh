@@ -26,7 +26,7 @@ __global__ void __launch_bounds__(F::T, F::MINB) fft_prep_kernel(JobDev *jobs, c
     PFB_DYNAMIC_SMEM(unsigned char, raw);
     const JobDev jb = jobs[list[blockIdx.x]];
     View w;
-    carve<F>(raw, nullptr, w);
+    carve<F>(raw, nullptr, nullptr, w);
     const Cplx *none = nullptr, *none2 = nullptr;
     resident<F>(w, tab, none, none2);
     int lo[F::R1], hi[F::R1];
@@ -67,10 +67,10 @@ __device__ __forceinline__ JobDev load_job(const JobDev *jp) {
 
 // Runs up to max_steps steps of one candidate (strong test or modular power).
 template <class F>
-__device__ void run_fft_job(JobDev *jp, int max_steps, Tab tab, unsigned char *raw, Cplx *gscratch) {
+__device__ void run_fft_job(JobDev *jp, int max_steps, Tab tab, unsigned char *raw, Cplx *scratch) {
     const JobDev jb = load_job(jp);
     View w;
-    carve<F>(raw, gscratch, w);
+    carve<F>(raw, jb.sq ? reinterpret_cast<Cplx *>(jb.sq) : scratch, reinterpret_cast<int *>(jb.x), w);
     const Cplx *nn = reinterpret_cast<const Cplx *>(jb.nn), *nh = reinterpret_cast<const Cplx *>(jb.nh);
     resident<F>(w, tab, nn, nh);
     const int b = jb.fbits;
@@ -134,14 +134,14 @@ __device__ void run_fft_job(JobDev *jp, int max_steps, Tab tab, unsigned char *r
 // and Q^k are kept as limb arrays, each thread reading and writing its own.
 // Up to max_steps ladder bits or final steps.  Every Montgomery step of the
 // ladder goes through one copy of the code: `todo` lists what is left of the
-// current bit.  ys: 2 C points, the spectra of V_(k+1).
+// current bit.
 template <class F>
-__device__ void run_fft_lucas(JobDev *jp, int max_steps, Tab tab, unsigned char *raw, Cplx *gscratch,
-                              Cplx *ys) {
+__device__ void run_fft_lucas(JobDev *jp, int max_steps, Tab tab, unsigned char *raw) {
     const JobDev jb = load_job(jp);
     const LucasDev lc = *jb.lucas;
     View w;
-    carve<F>(raw, gscratch, w);
+    carve<F>(raw, reinterpret_cast<Cplx *>(jb.sq), reinterpret_cast<int *>(jb.x), w);
+    Cplx *ys = reinterpret_cast<Cplx *>(lc.gy);
     const Cplx *nn = reinterpret_cast<const Cplx *>(jb.nn), *nh = reinterpret_cast<const Cplx *>(jb.nh);
     resident<F>(w, tab, nn, nh);
     const int b = jb.fbits, aq = lc.q < 0 ? -lc.q : lc.q;
@@ -230,8 +230,9 @@ __device__ void run_fft_lucas(JobDev *jp, int max_steps, Tab tab, unsigned char 
 // quanta (`quantum` steps of one job) until `total` are handed out; quantum q
 // goes to the first unfinished, unlocked job at or after position q mod n.
 // One warp looks at 32 jobs at a time.  Nothing waits: a CTA that finds every
-// job locked or finished leaves.  scratch: F::scratch() points per
-// CTA, 2 C more for Lucas tests (LUCAS: all jobs are).
+// job locked or finished leaves.  LUCAS: all jobs are Lucas tests.  scratch: C
+// points per CTA, of the classes with spectrum_outside(), for jobs without
+// such a spectrum of their own.
 template <class F, bool LUCAS = false>
 __global__ void __launch_bounds__(F::T, F::MINB)
 fft_persist_kernel(JobDev *jobs, const int *list, int n, int *locks, unsigned int *counter, unsigned int total,
@@ -274,9 +275,8 @@ fft_persist_kernel(JobDev *jobs, const int *list, int n, int *locks, unsigned in
         const int j = s_job;
         __syncthreads();
         if (j < 0) break;
-        Cplx *sc = scratch + (size_t)blockIdx.x * (F::scratch() + (LUCAS ? 2 * F::C : 0));
-        if constexpr (LUCAS) run_fft_lucas<F>(jobs + j, quantum, tab, raw, sc, sc + F::scratch());
-        else run_fft_job<F>(jobs + j, quantum, tab, raw, sc);
+        if constexpr (LUCAS) run_fft_lucas<F>(jobs + j, quantum, tab, raw);
+        else run_fft_job<F>(jobs + j, quantum, tab, raw, scratch + (size_t)blockIdx.x * F::C);
         if (threadIdx.x == 0) {
             __threadfence();
             atomicExch(&locks[j], 0);
@@ -300,7 +300,7 @@ fft_ctx_kernel(const JobDev *jobs, const int *list, const uint64_t *A, const uin
     __shared__ int s_slot;
     const int m = list[blockIdx.x];
     const JobDev jb = jobs[m];
-    if (F::scratch()) {
+    if (!F::SQS) {
         if (threadIdx.x == 0) {
             int at = (int)(blockIdx.x % (unsigned)n_slots);
             for (int tries = 0; tries < (1 << 24) && atomicCAS(&slots[at], 0, 1) != 0; tries++)
@@ -311,7 +311,7 @@ fft_ctx_kernel(const JobDev *jobs, const int *list, const uint64_t *A, const uin
         __syncthreads();
     }
     View w;
-    carve<F>(raw, F::scratch() ? scratch + (size_t)s_slot * F::scratch() : nullptr, w);
+    carve<F>(raw, F::SQS ? nullptr : scratch + (size_t)s_slot * F::C, nullptr, w);
     const Cplx *nn = reinterpret_cast<const Cplx *>(jb.nn), *nh = reinterpret_cast<const Cplx *>(jb.nh);
     resident<F>(w, tab, nn, nh);
     auto digit = [&](const uint64_t *src) {
@@ -344,7 +344,7 @@ fft_ctx_kernel(const JobDev *jobs, const int *list, const uint64_t *A, const uin
             if (i + q < F::N) v |= (unsigned long long)(uint32_t)L[lpos<F>(i + q)] << (kCtxBits * q);
         o[k] = (v >> off) & 0xFFFFull;
     }
-    if (F::scratch()) {
+    if (!F::SQS) {
         __syncthreads();
         if (threadIdx.x == 0) {
             __threadfence();

@@ -101,7 +101,7 @@ namespace {
 
 // Per-candidate device layout inside the arena (32-bit words).
 struct Layout {
-    size_t x, res, nn, nh, npl, nl, exp, yb, lv0, lv1, lqk, lt, lone, gy, raw, ys, total;
+    size_t x, res, nn, nh, npl, nl, exp, yb, lv0, lv1, lqk, lt, lone, gy, raw, ys, sq, total;
 };
 
 Layout layout_for(int logl, size_t exp_words, bool lucas = false, bool raw = false) {
@@ -135,7 +135,8 @@ Layout layout_for(int logl, size_t exp_words, bool lucas = false, bool raw = fal
 }
 
 // Layout of a candidate of the floating-point engine: n = 2 C digits, spectra
-// of C points (4 words each).  ctx_logl: a modulus of a context instead, with
+// of C points (4 words each); x^2's spectrum takes the place of N'', which only
+// the set-up reads.  ctx_logl: a modulus of a context instead, with
 // the buffers of the integer engine's raw products at that transform length.
 Layout layout_fp(int cls, size_t exp_words, bool lucas, int ctx_logl = 0) {
     const size_t C = (size_t)fp::class_points(cls), n = 2 * C;
@@ -148,7 +149,7 @@ Layout layout_fp(int cls, size_t exp_words, bool lucas, int ctx_logl = 0) {
     };
     l.nn = take(4 * C);
     l.nh = take(4 * C);
-    l.npl = take(n);
+    l.npl = l.sq = take(fp::spectrum_outside(cls) && !ctx_logl ? 4 * C : n);
     l.nl = take(n);
     if (ctx_logl) {
         const size_t L = (size_t)1 << ctx_logl;
@@ -167,6 +168,7 @@ Layout layout_fp(int cls, size_t exp_words, bool lucas, int ctx_logl = 0) {
         l.lqk = take(n);
         l.lt = take(n);
         l.lone = take(n);
+        l.gy = take(8 * C);
     }
     l.total = o;
     return l;
@@ -199,14 +201,14 @@ struct ClassRuns {
     }
 };
 
-// Device scratch (points) of one launch of every class' persistent kernel,
-// and where a class' part begins.
-size_t fp_scratch_points(const pfb_mr *e, bool lucas, const int *count, size_t *begin) {
+// The server's device scratch (points) of one launch of every class'
+// persistent kernel, and where a class' part begins.
+size_t fp_scratch_points(const pfb_mr *e, const int *count, size_t *begin) {
     size_t o = 0;
     for (int c = 0; c < fp::kClasses; c++) {
         begin[c] = o;
-        if (count[c])
-            o += fp::scratch_points(c, lucas) * fp::persist_launch(e->fe, lucas, c, count[c], e->num_sms).grid.x;
+        if (count[c] && fp::spectrum_outside(c))
+            o += (size_t)fp::class_points(c) * fp::persist_launch(e->fe, false, c, count[c], e->num_sms).grid.x;
     }
     return o;
 }
@@ -268,8 +270,6 @@ struct pfb_mr_batch {
     unsigned int *d_counter = nullptr;  // quanta handed out in the current launch: integer engine, then per class
     ClassRuns runs;
     int *d_order = nullptr;             // runs.order
-    fp::Cplx *d_scratch = nullptr;      // x^2's spectra, per CTA (classes that need it)
-    size_t scratch_begin[fp::kClasses] = {};
     LucasDev *d_lucas = nullptr;        // [n] (strong Lucas batches only)
     std::vector<HostPrep> hp;
     std::vector<JobDev> jobs;
@@ -337,7 +337,7 @@ int chunk_graph(pfb_mr_batch *b, long long chunk, int quantum, cudaGraphExec_t *
         const int *order = b->d_order + b->runs.first[c];
         unsigned int *cnt = counter + 1 + c;
         fp::Tab tab = b->e->fe.tab[c];
-        fp::Cplx *scratch = b->d_scratch + b->scratch_begin[c];
+        fp::Cplx *scratch = nullptr;  // the jobs have their own
         void *fa[] = {&jobs, &order, &nc, &locks, &cnt, &tc, &qc, &tab, &scratch};
         cudaKernelNodeParams kp{};
         kp.func = l.func;
@@ -383,8 +383,7 @@ int batch_build_on(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base,
     const size_t lucas_bytes = mode == 2 ? (((size_t)n * sizeof(LucasDev) + 255) & ~(size_t)255) : 0;
     b->runs.build(n, [&](int i) { return b->hp[i].ok && b->hp[i].decided < 0; }, [&](int i) { return b->hp[i].fpc; });
     const size_t order_bytes = (b->runs.order.size() * sizeof(int) + 255) & ~(size_t)255;
-    const size_t scratch_bytes = fp_scratch_points(e, mode == 2, b->runs.count, b->scratch_begin) * sizeof(fp::Cplx);
-    const size_t need = job_bytes + lock_bytes + lucas_bytes + order_bytes + scratch_bytes + total * sizeof(uint32_t);
+    const size_t need = job_bytes + lock_bytes + lucas_bytes + order_bytes + total * sizeof(uint32_t);
     if (cudaMalloc(&b->d_arena, need) != cudaSuccess) {
         cudaGetLastError();
         pfb::set_error("pfb_mr: cannot allocate %zu bytes of device memory", need);
@@ -399,8 +398,7 @@ int batch_build_on(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base,
         b->lucas.assign(n, LucasDev{});
     }
     b->d_order = (int *)(b->d_arena + job_bytes + lock_bytes + lucas_bytes);
-    b->d_scratch = (fp::Cplx *)(b->d_arena + job_bytes + lock_bytes + lucas_bytes + order_bytes);
-    uint32_t *d_words = (uint32_t *)(b->d_arena + job_bytes + lock_bytes + lucas_bytes + order_bytes + scratch_bytes);
+    uint32_t *d_words = (uint32_t *)(b->d_arena + job_bytes + lock_bytes + lucas_bytes + order_bytes);
     if (cudaMemsetAsync(b->d_locks, 0, lock_bytes, e->stream) != cudaSuccess) {
         batch_free(b);
         return pfb::cuda_fail(cudaGetLastError(), "lock reset", __FILE__, __LINE__);
@@ -430,6 +428,7 @@ int batch_build_on(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base,
         j.logl = h.logl;
         j.fpc = h.fpc;
         j.fbits = h.fbits;
+        if (h.fpc && fp::spectrum_outside(h.fpc - 1)) j.sq = w + l.sq;
         j.cursor = h.cursor;
         j.extra = mode >= 1 ? h.s - 1 : 0;
         j.phase = 0;
@@ -444,7 +443,7 @@ int batch_build_on(pfb_mr *e, const pfb_mr_number_t *nums, int n, uint32_t base,
             lc.lqk = w + l.lqk;
             lc.lt = w + l.lt;
             lc.lone = w + l.lone;
-            if (!h.fpc) lc.gy = w + l.gy;
+            lc.gy = w + l.gy;
             lc.q = h.q;
             lc.lb = h.lb;
             j.lucas = b->d_lucas + i;
@@ -1158,7 +1157,7 @@ int srv_launch(pfb_mr_server *s) {
         s->runs_stale = false;
     }
     size_t begin[fp::kClasses];
-    const size_t need = fp_scratch_points(e, false, s->runs.count, begin) * sizeof(fp::Cplx);
+    const size_t need = fp_scratch_points(e, s->runs.count, begin) * sizeof(fp::Cplx);
     if (need > s->scratch_bytes) {
         PFB_CUDA(cudaStreamSynchronize(s->stream));
         cudaFree(s->d_scratch);
@@ -1523,8 +1522,8 @@ extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs
     const size_t order_bytes = ((size_t)n_batch * sizeof(int) + 255) & ~(size_t)255;
     size_t region = 0;  // the largest class' scratch
     for (int k = 0; k < fp::kClasses; k++)
-        if (c->runs.count[k] && fp::scratch_points(k, false)) {
-            region = std::max(region, fp::scratch_points(k, false));
+        if (c->runs.count[k] && fp::spectrum_outside(k)) {
+            region = std::max(region, (size_t)fp::class_points(k));
             c->n_slots = e->num_sms * std::max(1, e->fe.ctx_per_sm[k]);
         }
     const size_t slot_ints = ((size_t)c->n_slots * sizeof(int) + 255) & ~(size_t)255;

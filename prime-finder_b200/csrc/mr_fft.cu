@@ -71,16 +71,6 @@ void engine_free(Engine &e) {
     e.mem = nullptr;
 }
 
-size_t scratch_points(int cls, bool lucas) {
-    switch (cls) {
-#define PFB_CLS(F) \
-    case F::ID: return F::scratch() + (lucas ? 2 * (size_t)F::C : 0);
-        PFB_FP_CLASSES(PFB_CLS)
-#undef PFB_CLS
-    }
-    return 0;
-}
-
 Launch persist_launch(const Engine &e, bool lucas, int cls, int n, int sms) {
     Launch l{};
     const int grid = std::max(1, std::min(n, sms * std::max(1, e.per_sm[lucas][cls])));

@@ -20,10 +20,6 @@ struct Engine {
 int engine_create(Engine &e);
 void engine_free(Engine &e);
 
-// Points of device scratch a class needs per CTA (lucas: of the Lucas tests'
-// persistent kernel, else of the others).
-size_t scratch_points(int cls, bool lucas);
-
 // Arguments and launch shape of one launch of the persistent kernel.
 struct Launch {
     void *func;

@@ -29,10 +29,12 @@ struct JobDev {
     // the others digits), nn and nh C complex points.
     int fpc;
     int fbits;
+    uint32_t *sq;  // x^2's spectrum of the classes that keep it in global memory (C points)
 };
 
 // Strong Lucas state of one candidate: H limbs each, Montgomery form: V_k,
-// V_(k+1), Q^k, a product, R mod N; gy the [2][L] spectrum of V_(k+1).
+// V_(k+1), Q^k, a product, R mod N; gy the [2][L] spectrum of V_(k+1)
+// (floating-point engine: its two spectra, 2 C points).
 struct LucasDev {
     uint32_t *lv0, *lv1, *lqk, *lt, *lone, *gy;
     int q;        // Selfridge Q = (1 - D) / 4

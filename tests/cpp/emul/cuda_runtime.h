@@ -129,12 +129,17 @@ inline bool yield() {
     return false;
 }
 
+// Called by the last thread to arrive at each barrier of a CTA: a test may run
+// another CTA there, as a second launch on another SM would (run_cta nests).
+inline std::function<void()> at_barrier;
+
 inline void group_wait(int g) {
     Group &G = (*groups)[g];
     const unsigned long long my = G.gen;
     if (++G.arrived == G.size) {
         G.arrived = 0;
         G.gen++;
+        if (g == 0 && at_barrier) at_barrier();
         return;
     }
     while (G.gen == my)
@@ -166,8 +171,36 @@ inline void trampoline(unsigned lo, unsigned hi) {
     fiber_main((int)lo);
 }
 
+// The emulator's state of the running CTA, put back when a nested one ends.
+struct Saved {
+    std::vector<Fiber> *fibers_ = fibers;
+    std::vector<Group> *groups_ = groups;
+    std::vector<unsigned long long> *vals_ = lane_vals;
+    const std::function<void()> *body_ = body;
+    ucontext_t ctx_ = main_ctx;
+    void *sp_ = main_sp;
+    int current_ = current;
+    unsigned char *smem_ = dyn_smem;
+    emu_dim3 t_ = threadIdx, b_ = blockIdx, bd_ = blockDim, g_ = gridDim;
+    ~Saved() {
+        fibers = fibers_;
+        groups = groups_;
+        lane_vals = vals_;
+        body = body_;
+        main_ctx = ctx_;
+        main_sp = sp_;
+        current = current_;
+        dyn_smem = smem_;
+        threadIdx = t_;
+        blockIdx = b_;
+        blockDim = bd_;
+        gridDim = g_;
+    }
+};
+
 // Runs f once per thread of one CTA of `threads` threads.
 inline void run_cta(int threads, const std::function<void()> &f) {
+    const Saved outer;
     std::vector<Fiber> fs(threads);
     std::vector<Group> gs(1 + (threads + 31) / 32);
     gs[0].size = threads;
@@ -180,14 +213,17 @@ inline void run_cta(int threads, const std::function<void()> &f) {
     blockDim.x = (unsigned)threads;
     const size_t stack_bytes = 256 * 1024;
     static std::vector<void *> stacks;  // reused by every CTA of the process
-    while ((int)stacks.size() < threads) {
+    static int in_use = 0;              // by the CTAs that this one is nested in
+    const int base = in_use;
+    while ((int)stacks.size() < base + threads) {
         void *st = malloc(stack_bytes);
         if (!st) throw std::runtime_error("fiber stack");
         stacks.push_back(st);
     }
+    in_use += threads;
     for (int t = 0; t < threads; t++) {
         Fiber &fb = fs[t];
-        fb.stack = stacks[t];
+        fb.stack = stacks[base + t];
 #ifdef EMU_FAST_SWITCH
         // initial frame: six register slots, then fiber_entry as the return
         // address, then a null slot so that fiber_entry starts as if called
@@ -211,15 +247,13 @@ inline void run_cta(int threads, const std::function<void()> &f) {
 #else
     swapcontext(&main_ctx, &fs[0].ctx);
 #endif
-    fibers = nullptr;
-    groups = nullptr;
-    lane_vals = nullptr;
-    body = nullptr;
+    in_use = base;
 }
 
 // Runs f for every thread of a gx x gy grid of CTAs of `threads` threads,
 // one CTA after another, with smem bytes of dynamic shared memory.
 inline void run_grid(unsigned gx, unsigned gy, int threads, const std::function<void()> &f, size_t smem = 0) {
+    const Saved outer;
     std::vector<unsigned char> buf(smem);
     dyn_smem = smem ? buf.data() : nullptr;
     gridDim.x = gx;
@@ -230,7 +264,6 @@ inline void run_grid(unsigned gx, unsigned gy, int threads, const std::function<
             blockIdx.y = y;
             run_cta(threads, f);
         }
-    dyn_smem = nullptr;
 }
 
 }  // namespace emu

@@ -6,6 +6,10 @@
 //   job mode base N [E]        whole test (mode 1: strong test, 2: strong Lucas
 //                              test) or base^E mod N (mode 0)
 //                              -> class bits verdict residue
+//   overlap base N E N2 E2     two modular powers of one length class, the second
+//                              advanced a step at a time by a launch of its own
+//                              that runs in the middle of the first one's steps
+//                              -> class residue residue2
 //   ctx cls op N a b           an operation of a modular context (mr_job.cuh:
 //                              CtxOp) on plain numbers -> result
 //   step cls bits dbl kind N   one squaring of limbs of a pattern: kind 0
@@ -84,28 +88,58 @@ static fp::Tab tables(std::vector<fp::Cplx> &mem) {
 }
 
 template <class F>
-static void run_job_cls(JobDev &j) {
-    std::vector<fp::Cplx> mem, scratch(F::scratch() + (j.mode == 2 ? 2 * F::C : 0) + 1);
-    const fp::Tab tab = tables<F>(mem);
+static void prep_job(JobDev &j, const fp::Tab &tab) {
     const int list[1] = {0};
     emu::run_grid(1, 1, F::T, [&] { fp::fft_prep_kernel<F>(&j, list, tab); }, F::smem());
+}
+
+// One launch: `total` quanta of `quantum` steps.
+template <class F>
+static void launch_job(JobDev &j, const fp::Tab &tab, unsigned total, int quantum) {
+    const int list[1] = {0};
     int locks[1] = {0};
     unsigned counter = 0;
-    for (int launch = 0; j.phase != 3 && launch < 1 << 20; launch++) {
-        counter = 0;
-        emu::run_grid(1, 1, F::T, [&] {
-            if (j.mode == 2)
-                fp::fft_persist_kernel<F, true>(&j, list, 1, locks, &counter, 8u, 64, tab, scratch.data());
-            else
-                fp::fft_persist_kernel<F>(&j, list, 1, locks, &counter, 8u, 64, tab, scratch.data());
-        }, F::smem());
-    }
+    emu::run_grid(1, 1, F::T, [&] {
+        if (j.mode == 2)
+            fp::fft_persist_kernel<F, true>(&j, list, 1, locks, &counter, total, quantum, tab, nullptr);
+        else
+            fp::fft_persist_kernel<F>(&j, list, 1, locks, &counter, total, quantum, tab, nullptr);
+    }, F::smem());
+}
+
+template <class F>
+static void run_job_cls(JobDev &j) {
+    std::vector<fp::Cplx> mem;
+    const fp::Tab tab = tables<F>(mem);
+    prep_job<F>(j, tab);
+    for (int launch = 0; j.phase != 3 && launch < 1 << 20; launch++) launch_job<F>(j, tab, 8u, 64);
+}
+
+// j2 takes a step whenever j has passed another 13 barriers of the block (the
+// first ones are the scheduler's own, whose shared variable the two share here).
+template <class F>
+static void run_overlap_cls(JobDev &j, JobDev &j2) {
+    std::vector<fp::Cplx> mem;
+    const fp::Tab tab = tables<F>(mem);
+    prep_job<F>(j, tab);
+    prep_job<F>(j2, tab);
+    long barrier = 0;
+    bool nested = false;
+    emu::at_barrier = [&] {
+        if (nested || ++barrier < 8 || barrier % 13 || j2.phase == 3) return;
+        nested = true;
+        launch_job<F>(j2, tab, 1u, 1);
+        nested = false;
+    };
+    launch_job<F>(j, tab, 1u, 64);
+    emu::at_barrier = nullptr;
 }
 
 template <class F>
 static void run_step(int b, int dbl, int kind, const Words &N) {
     const size_t n = F::N;
-    std::vector<fp::Cplx> mem, scratch(F::scratch() + 1), nn(F::C), nh(F::C);
+    std::vector<fp::Cplx> mem, sq(F::C), nn(F::C), nh(F::C);
+    std::vector<int> xs(n);
     const fp::Tab gtab = tables<F>(mem);
     Words inv;
     if (!neg_inv_radix(N, n * b, inv)) {
@@ -125,7 +159,7 @@ static void run_step(int b, int dbl, int kind, const Words &N) {
     emu::run_grid(1, 1, F::T, [&] {
         PFB_DYNAMIC_SMEM(unsigned char, raw);
         fp::View w;
-        fp::carve<F>(raw, scratch.data(), w);
+        fp::carve<F>(raw, sq.data(), xs.data(), w);
         fp::Tab tab = gtab;
         const fp::Cplx *sn = nullptr, *sh = nullptr;
         fp::resident<F>(w, tab, sn, sh);
@@ -155,7 +189,7 @@ template <class F>
 static void run_ctx(int op, const Words &N, const Words &a, const Words &b) {
     const size_t n = F::N;
     const int n16 = (int)((pfb::big::bit_length(N) + 15) / 16);
-    std::vector<fp::Cplx> mem, scratch(2 * F::scratch() + 1), nn(F::C), nh(F::C), ys(2 * F::C);
+    std::vector<fp::Cplx> mem, scratch(2 * F::C), nn(F::C), nh(F::C), ys(2 * F::C);
     const fp::Tab tab = tables<F>(mem);
     Words inv;
     if (!neg_inv_radix(N, n * fp::kCtxBits, inv)) {
@@ -191,6 +225,67 @@ static void run_ctx(int op, const Words &N, const Words &a, const Words &b) {
     std::cout << to_hex(pfb::big::from_u16(o.data(), o.size())) << " " << slots[0] << slots[1] << std::endl;
 }
 
+// A candidate's host set-up and memory, as the host code lays it out.
+struct Job {
+    HostPrep hp;
+    std::vector<uint32_t> x, res, npl, nl, e, lv[5];
+    std::vector<fp::Cplx> nn, nh, sq, gy;
+    JobDev j{};
+    LucasDev lc{};
+    Job(const Job &) = delete;
+    Job(int mode, uint32_t base, const Words &N, const Words &E) {
+        std::vector<uint16_t> limbs(std::max<size_t>(1, (pfb::big::bit_length(N) + 15) / 16));
+        pfb::big::to_u16(N, limbs.data(), limbs.size());
+        std::vector<uint16_t> el(std::max<size_t>(1, (pfb::big::bit_length(E) + 15) / 16));
+        pfb::big::to_u16(E, el.data(), el.size());
+        const pfb_mr_number_t num{limbs.data(), (int)limbs.size()}, ex{el.data(), (int)el.size()};
+        host_prep(num, base, mode, mode ? nullptr : &ex, hp, true);
+        if (!runs()) return;
+        const size_t n = hp.x0.size();
+        x = hp.x0;
+        npl = hp.npl;
+        nl = hp.nl;
+        e = hp.exp;
+        res.resize(n);
+        nn.resize(n / 2);
+        nh.resize(n / 2);
+        j.x = x.data();
+        j.res = res.data();
+        j.nn = reinterpret_cast<uint32_t *>(nn.data());
+        j.nh = reinterpret_cast<uint32_t *>(nh.data());
+        j.npl = npl.data();
+        j.nl = nl.data();
+        j.exp = e.data();
+        j.logl = hp.logl;
+        j.fpc = hp.fpc;
+        j.fbits = hp.fbits;
+        if (fp::spectrum_outside(hp.fpc - 1)) {  // N'' lies at its start, as in the engine's layout
+            sq.resize(n / 2);
+            std::copy(npl.begin(), npl.end(), reinterpret_cast<uint32_t *>(sq.data()));
+            j.npl = j.sq = reinterpret_cast<uint32_t *>(sq.data());
+        }
+        j.cursor = hp.cursor;
+        j.extra = mode >= 1 ? hp.s - 1 : 0;
+        j.base = base;
+        j.mode = mode;
+        if (mode == 2) {
+            for (auto &v : lv) v.resize(n);
+            gy.resize(n);
+            lc.lv0 = lv[0].data();
+            lc.lv1 = lv[1].data();
+            lc.lqk = lv[2].data();
+            lc.lt = lv[3].data();
+            lc.lone = lv[4].data();
+            lc.gy = reinterpret_cast<uint32_t *>(gy.data());
+            lc.q = hp.q;
+            lc.lb = hp.lb;
+            j.lucas = &lc;
+        }
+    }
+    bool runs() const { return hp.ok && hp.decided < 0 && hp.fpc; }
+    std::string residue() const { return to_hex(pfb::big::from_limbs(res.data(), hp.fbits, res.size())); }
+};
+
 int main() {
     fp::c_first = fp::first_roots();
     std::string line;
@@ -222,59 +317,37 @@ int main() {
             }
             continue;
         }
+        if (op == "overlap") {
+            uint32_t base = 2;
+            std::string sn2, se2;
+            in >> base >> sn >> se >> sn2 >> se2;
+            Job a(0, base, from_hex(sn), from_hex(se)), b(0, base, from_hex(sn2), from_hex(se2));
+            switch (a.hp.fpc - 1) {
+#define PFB_CLS(F) \
+    case fp::F::ID: run_overlap_cls<fp::F>(a.j, b.j); break;
+                PFB_FP_CLASSES(PFB_CLS)
+#undef PFB_CLS
+            }
+            std::cout << a.hp.fpc - 1 << " " << a.residue() << " " << b.residue() << std::endl;
+            continue;
+        }
         int mode = 1;
         uint32_t base = 2;
         in >> mode >> base >> sn >> se;
-        const Words N = from_hex(sn), E = from_hex(se);
-        std::vector<uint16_t> limbs(std::max<size_t>(1, (pfb::big::bit_length(N) + 15) / 16));
-        pfb::big::to_u16(N, limbs.data(), limbs.size());
-        std::vector<uint16_t> el(std::max<size_t>(1, (pfb::big::bit_length(E) + 15) / 16));
-        pfb::big::to_u16(E, el.data(), el.size());
-        const pfb_mr_number_t num{limbs.data(), (int)limbs.size()}, ex{el.data(), (int)el.size()};
-        HostPrep hp;
-        host_prep(num, base, mode, mode ? nullptr : &ex, hp, true);
-        if (!hp.ok || hp.decided >= 0 || !hp.fpc) {
+        Job job(mode, base, from_hex(sn), from_hex(se));
+        const HostPrep &hp = job.hp;
+        if (!job.runs()) {
             std::cout << "- 0 " << (hp.ok && hp.decided >= 0 ? hp.decided : -1) << " 0" << std::endl;
             continue;
         }
-        const size_t n = hp.x0.size();
-        std::vector<uint32_t> x = hp.x0, res(n), npl = hp.npl, nl = hp.nl, e = hp.exp;
-        std::vector<fp::Cplx> nn(n / 2), nh(n / 2);
-        JobDev j{};
-        j.x = x.data();
-        j.res = res.data();
-        j.nn = reinterpret_cast<uint32_t *>(nn.data());
-        j.nh = reinterpret_cast<uint32_t *>(nh.data());
-        j.npl = npl.data();
-        j.nl = nl.data();
-        j.exp = e.data();
-        j.logl = hp.logl;
-        j.fpc = hp.fpc;
-        j.fbits = hp.fbits;
-        j.cursor = hp.cursor;
-        j.extra = mode >= 1 ? hp.s - 1 : 0;
-        j.base = base;
-        j.mode = mode;
-        std::vector<uint32_t> lv0(n), lv1(n), lqk(n), lt(n), lone(n);
-        LucasDev lc{};
-        if (mode == 2) {
-            lc.lv0 = lv0.data();
-            lc.lv1 = lv1.data();
-            lc.lqk = lqk.data();
-            lc.lt = lt.data();
-            lc.lone = lone.data();
-            lc.q = hp.q;
-            lc.lb = hp.lb;
-            j.lucas = &lc;
-        }
         switch (hp.fpc - 1) {
 #define PFB_CLS(F) \
-    case fp::F::ID: run_job_cls<fp::F>(j); break;
+    case fp::F::ID: run_job_cls<fp::F>(job.j); break;
             PFB_FP_CLASSES(PFB_CLS)
 #undef PFB_CLS
         }
-        std::cout << hp.fpc - 1 << " " << hp.fbits << " " << (j.phase == 3 ? j.verdict : -2) << " "
-                  << to_hex(pfb::big::from_limbs(res.data(), hp.fbits, n)) << std::endl;
+        std::cout << hp.fpc - 1 << " " << hp.fbits << " " << (job.j.phase == 3 ? job.j.verdict : -2) << " "
+                  << job.residue() << std::endl;
     }
     return 0;
 }

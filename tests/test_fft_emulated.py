@@ -90,6 +90,19 @@ def test_modular_powers_of_every_class(emul):
     assert {int(o[0]) for o in out} == set(range(len(CLASSES)))
 
 
+@pytest.mark.parametrize("bits", [2 * C * b - 9 for C, b in CLASSES[12:]])
+def test_overlapping_launches_of_one_class(emul, bits):
+    """Two launches on candidates of one class (advances of a resident batch on
+    two streams), the second running between the passes of the first one's
+    steps: neither touches what the other keeps in global memory."""
+    rng = random.Random(bits)
+    case = []
+    for _ in range(2):
+        case += [rng.getrandbits(bits) | 1 | (1 << (bits - 1)), rng.getrandbits(7) | 64]
+    o = emul(["overlap 2 %x %x %x %x" % tuple(case)])[0]
+    assert [int(x, 16) for x in o[1:]] == [pow(2, case[1], case[0]), pow(2, case[3], case[2])]
+
+
 def test_strong_lucas_tests(emul):
     rng = random.Random(12)
     ns = [5459, 5777, 10877, 16109, 18971, 3, 5, 7, 11, 13, 25, 49, 1000003, 1000001, (1 << 61) - 1, (1 << 127) - 1]

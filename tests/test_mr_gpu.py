@@ -197,6 +197,27 @@ def test_resident_batch_stepwise_equals_one_shot(mr):
     b.close()
 
 
+def test_advances_of_one_batch_on_two_streams(mr):
+    """Advances of one batch may overlap on the GPU (other streams, other step
+    counts): 150 numbers of the class that keeps x^2's spectrum in global
+    memory, more than it has resident CTAs, give the one-shot result."""
+    import torch
+    rng = random.Random(22)
+    Ns = [rng.getrandbits(123_000) | (1 << 122_999) | 1 for _ in range(150)]
+    want_v, want_r = mr.test(Ns, 2)
+    b = pfb200.MRBatch(mr, Ns, 2)
+    st = [torch.cuda.Stream() for _ in range(2)]
+    for i in range(2 * 123_000 // 3500 + 2):
+        b.advance(2000, st[0].cuda_stream)
+        b.advance(1500, st[1].cuda_stream)
+        if i % 20 == 19 and b.pending() == 0:
+            break
+    while b.pending():
+        b.advance(2000)
+    assert b.results(residues=True) == (want_v, want_r)
+    b.close()
+
+
 def _check_records(mr, recs):
     Ns = [oracle.build_candidate(r["a"], r["b"], r["c"], r["k"], r["j"], bool(r["rev"])) for r in recs]
     ver, res = mr.test(Ns, 2)
