@@ -67,10 +67,10 @@ __device__ __forceinline__ JobDev load_job(const JobDev *jp) {
 
 // Runs up to max_steps steps of one candidate (strong test or modular power).
 template <class F>
-__device__ void run_fft_job(JobDev *jp, int max_steps, Tab tab, unsigned char *raw, Cplx *scratch) {
+__device__ void run_fft_job(JobDev *jp, int max_steps, Tab tab, unsigned char *raw) {
     const JobDev jb = load_job(jp);
     View w;
-    carve<F>(raw, jb.sq ? reinterpret_cast<Cplx *>(jb.sq) : scratch, reinterpret_cast<int *>(jb.x), w);
+    carve<F>(raw, reinterpret_cast<Cplx *>(jb.sq), reinterpret_cast<int *>(jb.x), w);
     const Cplx *nn = reinterpret_cast<const Cplx *>(jb.nn), *nh = reinterpret_cast<const Cplx *>(jb.nh);
     resident<F>(w, tab, nn, nh);
     const int b = jb.fbits;
@@ -230,13 +230,11 @@ __device__ void run_fft_lucas(JobDev *jp, int max_steps, Tab tab, unsigned char 
 // quanta (`quantum` steps of one job) until `total` are handed out; quantum q
 // goes to the first unfinished, unlocked job at or after position q mod n.
 // One warp looks at 32 jobs at a time.  Nothing waits: a CTA that finds every
-// job locked or finished leaves.  LUCAS: all jobs are Lucas tests.  scratch: C
-// points per CTA, of the classes with spectrum_outside(), for jobs without
-// such a spectrum of their own.
+// job locked or finished leaves.  LUCAS: all jobs are Lucas tests.
 template <class F, bool LUCAS = false>
 __global__ void __launch_bounds__(F::T, F::MINB)
 fft_persist_kernel(JobDev *jobs, const int *list, int n, int *locks, unsigned int *counter, unsigned int total,
-                   int quantum, Tab tab, Cplx *scratch) {
+                   int quantum, Tab tab) {
     PFB_DYNAMIC_SMEM(unsigned char, raw);
     __shared__ int s_job;
     const unsigned FULL = 0xffffffffu;
@@ -276,7 +274,7 @@ fft_persist_kernel(JobDev *jobs, const int *list, int n, int *locks, unsigned in
         __syncthreads();
         if (j < 0) break;
         if constexpr (LUCAS) run_fft_lucas<F>(jobs + j, quantum, tab, raw);
-        else run_fft_job<F>(jobs + j, quantum, tab, raw, scratch + (size_t)blockIdx.x * F::C);
+        else run_fft_job<F>(jobs + j, quantum, tab, raw);
         if (threadIdx.x == 0) {
             __threadfence();
             atomicExch(&locks[j], 0);

@@ -201,18 +201,6 @@ struct ClassRuns {
     }
 };
 
-// The server's device scratch (points) of one launch of every class'
-// persistent kernel, and where a class' part begins.
-size_t fp_scratch_points(const pfb_mr *e, const int *count, size_t *begin) {
-    size_t o = 0;
-    for (int c = 0; c < fp::kClasses; c++) {
-        begin[c] = o;
-        if (count[c] && fp::spectrum_outside(c))
-            o += (size_t)fp::class_points(c) * fp::persist_launch(e->fe, false, c, count[c], e->num_sms).grid.x;
-    }
-    return o;
-}
-
 // Quanta of one launch of a class: jobs that each have a CTA of their own run
 // their whole chunk in one quantum.
 void fp_quanta(const pfb_mr *e, bool lucas, int cls, int n, long long chunk, int tuned, int *quantum, unsigned *total) {
@@ -337,8 +325,7 @@ int chunk_graph(pfb_mr_batch *b, long long chunk, int quantum, cudaGraphExec_t *
         const int *order = b->d_order + b->runs.first[c];
         unsigned int *cnt = counter + 1 + c;
         fp::Tab tab = b->e->fe.tab[c];
-        fp::Cplx *scratch = nullptr;  // the jobs have their own
-        void *fa[] = {&jobs, &order, &nc, &locks, &cnt, &tc, &qc, &tab, &scratch};
+        void *fa[] = {&jobs, &order, &nc, &locks, &cnt, &tc, &qc, &tab};
         cudaKernelNodeParams kp{};
         kp.func = l.func;
         kp.gridDim = l.grid;
@@ -849,8 +836,6 @@ struct pfb_mr_server {
     ClassRuns runs;               // resident candidates by engine and class
     int *d_order = nullptr;       // runs.order
     bool runs_stale = true;
-    uint8_t *d_scratch = nullptr; // x^2's spectra, per CTA
-    size_t scratch_bytes = 0;
     cudaStream_t side[fp::kClasses] = {};  // classes run side by side
     cudaEvent_t fork = nullptr, join[fp::kClasses] = {};
     std::vector<SrvSlot> slots;
@@ -1060,6 +1045,7 @@ int srv_admit(pfb_mr_server *s, std::vector<int> &admitted) {
         j.logl = h.logl;
         j.fpc = h.fpc;
         j.fbits = h.fbits;
+        if (h.fpc && fp::spectrum_outside(h.fpc - 1)) j.sq = w + l.sq;
         j.cursor = h.cursor;
         j.extra = h.s - 1;
         j.phase = 0;
@@ -1156,16 +1142,6 @@ int srv_launch(pfb_mr_server *s) {
                                      cudaMemcpyHostToDevice, s->stream));
         s->runs_stale = false;
     }
-    size_t begin[fp::kClasses];
-    const size_t need = fp_scratch_points(e, s->runs.count, begin) * sizeof(fp::Cplx);
-    if (need > s->scratch_bytes) {
-        PFB_CUDA(cudaStreamSynchronize(s->stream));
-        cudaFree(s->d_scratch);
-        s->d_scratch = nullptr;
-        s->scratch_bytes = 0;
-        PFB_CUDA(cudaMalloc(&s->d_scratch, need));
-        s->scratch_bytes = need;
-    }
     PFB_CUDA(cudaMemsetAsync(s->d_counter, 0, (1 + fp::kClasses) * sizeof(unsigned int), s->stream));
     const int quantum = std::min(64, s->cfg.chunk_steps);
     bool forked = false;
@@ -1209,8 +1185,7 @@ int srv_launch(pfb_mr_server *s) {
         const int *order = s->d_order + s->runs.first[c];
         unsigned int *cnt = s->d_counter + 1 + c;
         fp::Tab tab = e->fe.tab[c];
-        fp::Cplx *scratch = (fp::Cplx *)s->d_scratch + begin[c];
-        void *fa[] = {&s->d_jobs, &order, &nc, &s->d_locks, &cnt, &tc, &qc, &tab, &scratch};
+        void *fa[] = {&s->d_jobs, &order, &nc, &s->d_locks, &cnt, &tc, &qc, &tab};
         PFB_CUDA(cudaLaunchKernel(l.func, l.grid, l.block, fa, l.smem, st));
     }
     if (forked)
@@ -1407,7 +1382,6 @@ extern "C" void pfb_mr_server_destroy(pfb_mr_server_t *s) {
         if (sl.mem) cudaFree(sl.mem);
     for (auto &kv : s->pool)
         for (uint8_t *m : kv.second) cudaFree(m);
-    cudaFree(s->d_scratch);
     cudaEventDestroy(s->fork);
     for (int c = 0; c < fp::kClasses; c++) {
         if (s->side[c]) cudaStreamDestroy(s->side[c]);

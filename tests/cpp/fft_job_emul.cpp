@@ -101,9 +101,9 @@ static void launch_job(JobDev &j, const fp::Tab &tab, unsigned total, int quantu
     unsigned counter = 0;
     emu::run_grid(1, 1, F::T, [&] {
         if (j.mode == 2)
-            fp::fft_persist_kernel<F, true>(&j, list, 1, locks, &counter, total, quantum, tab, nullptr);
+            fp::fft_persist_kernel<F, true>(&j, list, 1, locks, &counter, total, quantum, tab);
         else
-            fp::fft_persist_kernel<F>(&j, list, 1, locks, &counter, total, quantum, tab, nullptr);
+            fp::fft_persist_kernel<F>(&j, list, 1, locks, &counter, total, quantum, tab);
     }, F::smem());
 }
 

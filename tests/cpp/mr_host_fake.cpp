@@ -1,0 +1,130 @@
+// Runs the Miller-Rabin engine's host code (mr.cu) unchanged on the CPU
+// against a stand-in CUDA runtime (tests/cpp/emul/cuda_runtime_api_fake.h)
+// whose kernels only mark their candidates as finished, to see what the host
+// does when device memory runs out.  Input lines:
+//
+//   server allow bits   one request of a random number of that many bits, with
+//                       `allow` device allocations granted after the server's
+//                       creation (-1: all) -> "verdict v" or "stopped rc",
+//                       then the engine that ran it (fft, int, none)
+#include <algorithm>
+#include <chrono>
+#include <condition_variable>
+#include <deque>
+#include <iostream>
+#include <random>
+#include <sstream>
+#include <string>
+#include <thread>
+
+#include <cuda_runtime.h>
+#include <cuda_runtime_api_fake.h>
+
+#include "mr.cu"
+
+namespace pfb {
+void set_error(const char *, ...) {}
+int cuda_fail(cudaError_t, const char *, const char *, int) { return PFB_E_CUDA; }
+}  // namespace pfb
+
+static int n_fft, n_int;  // candidates that each engine has finished
+static int fn_fft, fn_int;
+
+namespace pfb {
+namespace mr {
+
+int int_setup(const CrtConsts &, const WideTabs &) { return PFB_OK; }
+void *int_persist_func() { return &fn_int; }
+cudaError_t int_prep(JobDev *, const int *, int, int, const Twiddles &, cudaStream_t) { return cudaSuccess; }
+cudaError_t int_ctx(const JobDev *, const CtxExtra *, int, int, const uint64_t *, const uint64_t *, uint64_t *, int,
+                    int, int, const Twiddles &, cudaStream_t) { return cudaSuccess; }
+cudaError_t int_ctx_check(const uint64_t *, const uint64_t *, const uint64_t *, uint8_t *, int, int, cudaStream_t) {
+    return cudaSuccess;
+}
+
+namespace fp {
+
+int engine_create(Engine &e) {
+    e = Engine{};
+    return PFB_OK;
+}
+void engine_free(Engine &) {}
+Launch persist_launch(const Engine &, bool, int, int n, int sms) {
+    return Launch{&fn_fft, dim3((unsigned)std::min(n, sms)), dim3(32), 0};
+}
+cudaError_t ctx(const Engine &, int, const JobDev *, const int *, int, const uint64_t *, const uint64_t *, uint64_t *,
+                int, int, Cplx *, int *, int, const CtxExtra *, cudaStream_t) { return cudaSuccess; }
+cudaError_t prep(const Engine &, int, JobDev *, const int *, int, cudaStream_t) { return cudaSuccess; }
+
+}  // namespace fp
+}  // namespace mr
+}  // namespace pfb
+
+static void finish(JobDev &j, int &count) {
+    if (j.phase == 3) return;
+    memset(j.res, 0, 4);  // (the kernels write it: it has to be there)
+    j.phase = 3;
+    j.verdict = 0;
+    count++;
+}
+
+static std::function<void()> launch(void *func, void **a) {
+    JobDev *jobs = *(JobDev **)a[0];
+    if (func == &fn_int) {
+        const int n = *(int *)a[1];
+        return [=] {
+            for (int i = 0; i < n; i++)
+                if (!jobs[i].fpc) finish(jobs[i], n_int);
+        };
+    }
+    const int *list = *(const int **)a[1], n = *(int *)a[2];
+    return [=] {
+        for (int i = 0; i < n; i++) finish(jobs[list[i]], n_fft);
+    };
+}
+
+static std::vector<uint16_t> number(int bits) {
+    std::mt19937 rng(bits);
+    std::vector<uint16_t> l((bits + 15) / 16);
+    for (auto &x : l) x = (uint16_t)rng();
+    const int top = (bits - 1) % 16;
+    l.back() = (uint16_t)((l.back() & ((1u << top) - 1u)) | (1u << top));
+    l[0] |= 1u;
+    return l;
+}
+
+static const char *engine() { return n_fft && n_int ? "both" : n_fft ? "fft" : n_int ? "int" : "none"; }
+
+int main() {
+    fake::launch = launch;
+    pfb_mr_t *e = nullptr;
+    if (pfb_mr_create(&e, 0)) return 2;
+    std::string line;
+    while (std::getline(std::cin, line)) {
+        std::istringstream in(line);
+        std::string op;
+        in >> op;
+        n_fft = n_int = 0;
+        if (op == "server") {
+            long allow;
+            int bits;
+            in >> allow >> bits;
+            const std::vector<uint16_t> l = number(bits);
+            pfb_mr_server_t *s = nullptr;
+            if (pfb_mr_server_create(e, nullptr, &s)) return 2;
+            fake::allow = allow;
+            pfb_mr_server_submit(s, l.data(), (int)l.size(), 7, nullptr, 0);
+            pfb_mr_result_t r{};
+            int n = 0;
+            for (int i = 0; i < 200 && n == 0; i++) n = pfb_mr_server_poll(s, &r, 1, 100);
+            if (n == 1) std::cout << "verdict " << (int)r.verdict;
+            else std::cout << "stopped " << n;
+            fake::allow = -1;
+            pfb_mr_server_destroy(s);
+        }
+        std::cout << " " << engine() << std::endl;
+    }
+    pfb_mr_destroy(e);
+    std::cout << "left " << fake::used << std::endl;
+    return 0;
+}

@@ -1,0 +1,37 @@
+"""The Miller-Rabin engine's host code when device memory runs out.
+
+tests/cpp/mr_host_fake.cpp runs csrc/mr.cu unchanged against a stand-in CUDA
+runtime (host memory under a limit, kernels that only mark their candidates
+finished), so that an allocation can fail at any point without a GPU.
+"""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def host(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("fake") / "mr_host_fake")
+    subprocess.run(["g++", "-O1", "-std=c++20", "-w", "-x", "c++",
+                    "-I", os.path.join(ROOT, "tests", "cpp", "emul"),
+                    "-I", os.path.join(ROOT, "prime-finder_b200", "csrc"),
+                    "-I", os.path.join(ROOT, "include"),
+                    os.path.join(ROOT, "tests", "cpp", "mr_host_fake.cpp"), "-o", exe, "-lpthread"], check=True)
+
+    def run(lines):
+        out = subprocess.run([exe], input="\n".join(lines) + "\n", capture_output=True, text=True, check=True,
+                             timeout=300).stdout.strip().split("\n")
+        assert out[-1] == "left 0"  # every block was freed
+        return out[:-1]
+    return run
+
+
+@pytest.mark.parametrize("bits", [3_000, 123_100, 344_000])
+def test_server_needs_no_memory_beyond_the_slot(host, bits):
+    """A server whose device has room for the slot and nothing more runs the
+    request; without room for the slot it reports the request, and stays up."""
+    assert host(["server -1 %d" % bits, "server 1 %d" % bits, "server 0 %d" % bits]) == \
+        ["verdict 0 fft", "verdict 0 fft", "verdict -1 none"]
