@@ -286,30 +286,19 @@ fft_persist_kernel(JobDev *jobs, const int *list, int n, int *locks, unsigned in
 // products) on the listed moduli, one CTA each: operands and results in 16-bit
 // limbs, one per uint64, at A + m n16 and so on for modulus m; digits of 11
 // bits (n = 2 H: the integer engine's radix R' = 2^(22 H) + 1, so the working
-// form is the same).  slots: one scratch region each, claimed for the CTA's
-// life -- launches on several streams may run at once -- with at least as
-// many slots as CTAs of this kernel can be resident.
+// form is the same).  Operands, results and the modulus' own buffers (ex) are
+// all that a CTA touches: the spectrum of x^2 that does not fit shared memory
+// lies where the raw products keep their coefficients.
 constexpr int kCtxBits = 11;
 template <class F>
 __global__ void __launch_bounds__(F::T, F::MINB)
 fft_ctx_kernel(const JobDev *jobs, const int *list, const uint64_t *A, const uint64_t *B, uint64_t *out, int n16,
-               int op, Tab tab, Cplx *scratch, int *slots, int n_slots, const CtxExtra *ex) {
+               int op, Tab tab, const CtxExtra *ex) {
     PFB_DYNAMIC_SMEM(unsigned char, raw);
-    __shared__ int s_slot;
     const int m = list[blockIdx.x];
     const JobDev jb = jobs[m];
-    if (!F::SQS) {
-        if (threadIdx.x == 0) {
-            int at = (int)(blockIdx.x % (unsigned)n_slots);
-            for (int tries = 0; tries < (1 << 24) && atomicCAS(&slots[at], 0, 1) != 0; tries++)
-                at = at + 1 < n_slots ? at + 1 : 0;
-            __threadfence();
-            s_slot = at;
-        }
-        __syncthreads();
-    }
     View w;
-    carve<F>(raw, F::SQS ? nullptr : scratch + (size_t)s_slot * F::C, nullptr, w);
+    carve<F>(raw, reinterpret_cast<Cplx *>(ex[m].raw), nullptr, w);
     const Cplx *nn = reinterpret_cast<const Cplx *>(jb.nn), *nh = reinterpret_cast<const Cplx *>(jb.nh);
     resident<F>(w, tab, nn, nh);
     auto digit = [&](const uint64_t *src) {
@@ -341,13 +330,6 @@ fft_ctx_kernel(const JobDev *jobs, const int *list, const uint64_t *A, const uin
         for (int q = 0; q < 3; q++)
             if (i + q < F::N) v |= (unsigned long long)(uint32_t)L[lpos<F>(i + q)] << (kCtxBits * q);
         o[k] = (v >> off) & 0xFFFFull;
-    }
-    if (!F::SQS) {
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            __threadfence();
-            atomicExch(&slots[s_slot], 0);
-        }
     }
 }
 

@@ -1406,9 +1406,6 @@ struct pfb_mr_ctx {
     // by class; the others, and all raw products, on the integer engine
     ClassRuns runs;
     int *d_order = nullptr;
-    fp::Cplx *d_scratch = nullptr;
-    int *d_slots = nullptr;  // scratch regions in use
-    int n_slots = 0;
     std::vector<HostPrep> hp;
 };
 
@@ -1442,7 +1439,7 @@ int ctx_launch(pfb_mr_ctx *c, const uint64_t *a, const uint64_t *b, uint64_t *ou
         for (int k = 0; k < fp::kClasses; k++)
             if (c->runs.count[k])
                 PFB_CUDA(fp::ctx(c->e->fe, k, c->d_jobs, c->d_order + c->runs.first[k], c->runs.count[k], a,
-                                 b ? b : a, out, c->n16, op, c->d_scratch, c->d_slots, c->n_slots, c->d_ex, st));
+                                 b ? b : a, out, c->n16, op, c->d_ex, st));
         if (!c->runs.n_int) return PFB_OK;
     }
     PFB_CUDA(int_ctx(c->d_jobs, c->d_ex, c->n, c->maxlog, a, b ? b : a, out, c->n16, out_stride, op, c->e->tw, st));
@@ -1494,15 +1491,7 @@ extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs
     const size_t v_bytes = (((size_t)n_batch * n_limbs * sizeof(uint64_t)) + 255) & ~(size_t)255;
     c->runs.build(n_batch, [](int) { return true; }, [&](int i) { return c->hp[i].fpc; });
     const size_t order_bytes = ((size_t)n_batch * sizeof(int) + 255) & ~(size_t)255;
-    size_t region = 0;  // the largest class' scratch
-    for (int k = 0; k < fp::kClasses; k++)
-        if (c->runs.count[k] && fp::spectrum_outside(k)) {
-            region = std::max(region, (size_t)fp::class_points(k));
-            c->n_slots = e->num_sms * std::max(1, e->fe.ctx_per_sm[k]);
-        }
-    const size_t slot_ints = ((size_t)c->n_slots * sizeof(int) + 255) & ~(size_t)255;
-    const size_t fp_bytes = order_bytes + slot_ints + region * c->n_slots * sizeof(fp::Cplx);
-    const size_t need = job_bytes + ex_bytes + 4 * v_bytes + fp_bytes + words * sizeof(uint32_t);
+    const size_t need = job_bytes + ex_bytes + 4 * v_bytes + order_bytes + words * sizeof(uint32_t);
     if (cudaMalloc(&c->d_arena, need) != cudaSuccess) {
         cudaGetLastError();
         pfb::set_error("pfb_mr_ctx_create: cannot allocate %zu bytes of device memory", need);
@@ -1514,11 +1503,8 @@ extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs
     c->d_nm1 = (uint64_t *)(c->d_arena + job_bytes + ex_bytes + v_bytes);
     c->d_tmp = (uint64_t *)(c->d_arena + job_bytes + ex_bytes + 2 * v_bytes);
     c->d_n = (uint64_t *)(c->d_arena + job_bytes + ex_bytes + 3 * v_bytes);
-    uint8_t *d_fp = c->d_arena + job_bytes + ex_bytes + 4 * v_bytes;
-    c->d_order = (int *)d_fp;
-    c->d_slots = (int *)(d_fp + order_bytes);
-    c->d_scratch = (fp::Cplx *)(d_fp + order_bytes + slot_ints);
-    uint32_t *d_words = (uint32_t *)(d_fp + fp_bytes);
+    c->d_order = (int *)(c->d_arena + job_bytes + ex_bytes + 4 * v_bytes);
+    uint32_t *d_words = (uint32_t *)(c->d_arena + job_bytes + ex_bytes + 4 * v_bytes + order_bytes);
     std::vector<JobDev> jobs(n_batch);
     std::vector<CtxExtra> ex(n_batch);
     std::vector<uint64_t> one((size_t)n_batch * n_limbs), nm1((size_t)n_batch * n_limbs);
@@ -1577,8 +1563,7 @@ extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs
     const std::vector<uint64_t> nall(n16.begin(), n16.end());
     PFB_CUDA(cudaMemcpy(c->d_n, nall.data(), nall.size() * 8, cudaMemcpyHostToDevice));
     cudaError_t ce = cudaSuccess;
-    if (c->n_slots) ce = cudaMemsetAsync(c->d_slots, 0, (size_t)c->n_slots * sizeof(int), e->stream);
-    if (ce == cudaSuccess && !c->runs.order.empty())
+    if (!c->runs.order.empty())
         ce = cudaMemcpyAsync(c->d_order, c->runs.order.data(), c->runs.order.size() * sizeof(int),
                              cudaMemcpyHostToDevice, e->stream);
     for (int k = 0; k < fp::kClasses && ce == cudaSuccess; k++)

@@ -36,12 +36,8 @@ int setup_class(Engine &e, std::vector<Cplx> &all) {
                                                            F::smem()));
     PFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e.per_sm[1][F::ID], fft_persist_kernel<F, true>, F::T,
                                                            F::smem()));
-    e.ctx_per_sm[F::ID] = 0;
-    if constexpr (in_ctx<F>()) {
+    if constexpr (in_ctx<F>())
         PFB_CUDA(cudaFuncSetAttribute(fft_ctx_kernel<F>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)F::smem()));
-        PFB_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&e.ctx_per_sm[F::ID], fft_ctx_kernel<F>, F::T,
-                                                               F::smem()));
-    }
     return PFB_OK;
 }
 
@@ -100,22 +96,19 @@ namespace {
 
 template <class F>
 void launch_ctx(const Tab &tab, const JobDev *jobs, const int *list, int n, const uint64_t *a, const uint64_t *b,
-                uint64_t *out, int n16, int op, Cplx *scratch, int *slots, int n_slots, const CtxExtra *ex,
-                cudaStream_t st) {
+                uint64_t *out, int n16, int op, const CtxExtra *ex, cudaStream_t st) {
     if constexpr (in_ctx<F>())
-        fft_ctx_kernel<F><<<n, F::T, F::smem(), st>>>(jobs, list, a, b, out, n16, op, tab, scratch, slots, n_slots, ex);
+        fft_ctx_kernel<F><<<n, F::T, F::smem(), st>>>(jobs, list, a, b, out, n16, op, tab, ex);
 }
 
 }  // namespace
 
 cudaError_t ctx(const Engine &e, int cls, const JobDev *jobs, const int *d_list, int n, const uint64_t *a,
-                const uint64_t *b, uint64_t *out, int n16, int op, Cplx *scratch, int *slots, int n_slots,
-                const CtxExtra *ex, cudaStream_t st) {
+                const uint64_t *b, uint64_t *out, int n16, int op, const CtxExtra *ex,
+                cudaStream_t st) {
     switch (cls) {
 #define PFB_CLS(F)                                                                                                \
-    case F::ID:                                                                                                   \
-        launch_ctx<F>(e.tab[F::ID], jobs, d_list, n, a, b, out, n16, op, scratch, slots, n_slots, ex, st);        \
-        break;
+    case F::ID: launch_ctx<F>(e.tab[F::ID], jobs, d_list, n, a, b, out, n16, op, ex, st); break;
         PFB_FP_CLASSES(PFB_CLS)
 #undef PFB_CLS
     }

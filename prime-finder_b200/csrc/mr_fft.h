@@ -13,8 +13,7 @@ namespace fp {
 struct Engine {
     Cplx *mem = nullptr;     // roots of all classes
     Tab tab[kClasses];
-    int per_sm[2][kClasses];   // resident CTAs per SM: strong tests, Lucas tests
-    int ctx_per_sm[kClasses];  // and of a context's operations
+    int per_sm[2][kClasses];  // resident CTAs per SM: strong tests, Lucas tests
 };
 
 int engine_create(Engine &e);
@@ -29,8 +28,8 @@ struct Launch {
 Launch persist_launch(const Engine &e, bool lucas, int cls, int n, int sms);
 
 cudaError_t ctx(const Engine &e, int cls, const JobDev *jobs, const int *d_list, int n, const uint64_t *a,
-                const uint64_t *b, uint64_t *out, int n16, int op, Cplx *scratch, int *slots, int n_slots,
-                const CtxExtra *ex, cudaStream_t st);
+                const uint64_t *b, uint64_t *out, int n16, int op, const CtxExtra *ex,
+                cudaStream_t st);
 
 cudaError_t prep(const Engine &e, int cls, JobDev *jobs, const int *d_list, int n, cudaStream_t st);
 

@@ -53,7 +53,7 @@ Launch persist_launch(const Engine &, bool, int, int n, int sms) {
     return Launch{&fn_fft, dim3((unsigned)std::min(n, sms)), dim3(32), 0};
 }
 cudaError_t ctx(const Engine &, int, const JobDev *, const int *, int, const uint64_t *, const uint64_t *, uint64_t *,
-                int, int, Cplx *, int *, int, const CtxExtra *, cudaStream_t) { return cudaSuccess; }
+                int, int, const CtxExtra *, cudaStream_t) { return cudaSuccess; }
 cudaError_t prep(const Engine &, int, JobDev *, const int *, int, cudaStream_t) { return cudaSuccess; }
 
 }  // namespace fp

@@ -10,9 +10,12 @@ check_passed, for 512- to 332 000-bit moduli (every transform length the
 engine uses for them, the 100 000-digit one included).  Every check must
 pass on every modulus.
 """
+import ctypes as C
 import os
+import random
 import subprocess
 
+import numpy as np
 import pytest
 
 import pfb200
@@ -50,3 +53,44 @@ def test_batch_mod_ctx_against_gmp(check):
     assert {int(row[1]) for row in rows} == {512, 2048, 20000, 166000, 332000}
     for name, bits, vals, ok, bad in rows:
         assert int(bad) == 0 and int(ok) > 0, (name, bits, vals)
+
+
+def test_more_moduli_than_resident_blocks():
+    """160 moduli of 50 000 digits (one block of the length class fits an SM):
+    a square and a product of each, read back, against Python."""
+    torch = pytest.importorskip("torch")
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    rng = random.Random(12)
+    n, bits = 160, 166_000
+    n16 = (bits + 15) // 16
+    Ns = [rng.getrandbits(bits) | (1 << (bits - 1)) | 1 for _ in range(n)]
+    ab = [[rng.randrange(N) for N in Ns] for _ in range(2)]
+
+    def rows(xs):
+        return np.frombuffer(b"".join(x.to_bytes(2 * n16, "little") for x in xs), dtype=np.uint16).astype(np.uint64)
+
+    def ptr(x):
+        return x.ctypes.data_as(C.POINTER(C.c_uint64))
+
+    L, vp = C.CDLL(pfb200.LIB_PATH), C.c_void_p
+    L.pfb_mr_ctx_modsq.argtypes = [vp, vp, vp, vp]
+    L.pfb_mr_ctx_modmul.argtypes = [vp, vp, vp, vp, vp]
+    L.pfb_mr_ctx_from_residue.argtypes = [vp, vp, C.POINTER(C.c_uint64)]
+    L.pfb_mr_ctx_destroy.argtypes = [vp]
+    eng, ctx = pfb200.MillerRabin(0), vp()
+    assert L.pfb_mr_ctx_create(eng._h, ptr(rows(Ns)), n16, n, C.byref(ctx)) == 0
+    a, b = (torch.from_numpy(rows(xs).astype(np.int64)).cuda() for xs in ab)
+    t = torch.empty_like(a)
+    out = np.zeros(n * n16, dtype=np.uint64)
+    torch.cuda.synchronize()
+    assert L.pfb_mr_ctx_modsq(ctx, a.data_ptr(), t.data_ptr(), None) == 0
+    assert L.pfb_mr_ctx_modmul(ctx, t.data_ptr(), b.data_ptr(), t.data_ptr(), None) == 0
+    assert L.pfb_mr_ctx_from_residue(ctx, t.data_ptr(), ptr(out)) == 0
+    L.pfb_mr_ctx_destroy(ctx)
+    eng.close()
+    got = out.astype(np.uint16).reshape(n, n16)
+    R = (1 << (22 * 8192)) + 1
+    for i in range(n):
+        x = int.from_bytes(got[i].tobytes(), "little")
+        assert x < Ns[i] and (x * R % Ns[i] * R % Ns[i] * R - ab[0][i] ** 2 * ab[1][i]) % Ns[i] == 0, i
