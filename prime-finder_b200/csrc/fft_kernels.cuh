@@ -286,9 +286,8 @@ fft_persist_kernel(JobDev *jobs, const int *list, int n, int *locks, unsigned in
 // products) on the listed moduli, one CTA each: operands and results in 16-bit
 // limbs, one per uint64, at A + m n16 and so on for modulus m; digits of 11
 // bits (n = 2 H: the integer engine's radix R' = 2^(22 H) + 1, so the working
-// form is the same).  Operands, results and the modulus' own buffers (ex) are
-// all that a CTA touches: the spectrum of x^2 that does not fit shared memory
-// lies where the raw products keep their coefficients.
+// form is the same).  Operands, results and the modulus' own buffers are all
+// that a CTA touches.
 constexpr int kCtxBits = 11;
 template <class F>
 __global__ void __launch_bounds__(F::T, F::MINB)
@@ -298,7 +297,7 @@ fft_ctx_kernel(const JobDev *jobs, const int *list, const uint64_t *A, const uin
     const int m = list[blockIdx.x];
     const JobDev jb = jobs[m];
     View w;
-    carve<F>(raw, reinterpret_cast<Cplx *>(ex[m].raw), nullptr, w);
+    carve<F>(raw, reinterpret_cast<Cplx *>(jb.sq), nullptr, w);
     const Cplx *nn = reinterpret_cast<const Cplx *>(jb.nn), *nh = reinterpret_cast<const Cplx *>(jb.nh);
     resident<F>(w, tab, nn, nh);
     auto digit = [&](const uint64_t *src) {

@@ -101,7 +101,7 @@ namespace {
 
 // Per-candidate device layout inside the arena (32-bit words).
 struct Layout {
-    size_t x, res, nn, nh, npl, nl, exp, yb, lv0, lv1, lqk, lt, lone, gy, raw, ys, sq, total;
+    size_t x, res, nn, nh, npl, nl, exp, yb, lv0, lv1, lqk, lt, lone, gy, raw, sq, total;
 };
 
 Layout layout_for(int logl, size_t exp_words, bool lucas = false, bool raw = false) {
@@ -136,8 +136,11 @@ Layout layout_for(int logl, size_t exp_words, bool lucas = false, bool raw = fal
 
 // Layout of a candidate of the floating-point engine: n = 2 C digits, spectra
 // of C points (4 words each); x^2's spectrum takes the place of N'', which only
-// the set-up reads.  ctx_logl: a modulus of a context instead, with
-// the buffers of the integer engine's raw products at that transform length.
+// the set-up reads.  ctx_logl: a modulus of a context instead, with the buffers
+// of the integer engine's raw products at that transform length: the second
+// factor's limbs take the place of N'' too, and a modular product has its
+// second factor's spectra (2 C points) where gy and raw lie, one behind the
+// other.
 Layout layout_fp(int cls, size_t exp_words, bool lucas, int ctx_logl = 0) {
     const size_t C = (size_t)fp::class_points(cls), n = 2 * C;
     Layout l{};
@@ -149,14 +152,12 @@ Layout layout_fp(int cls, size_t exp_words, bool lucas, int ctx_logl = 0) {
     };
     l.nn = take(4 * C);
     l.nh = take(4 * C);
-    l.npl = l.sq = take(fp::spectrum_outside(cls) && !ctx_logl ? 4 * C : n);
+    l.npl = l.sq = l.lt = take(fp::spectrum_outside(cls) ? 4 * C : n);
     l.nl = take(n);
     if (ctx_logl) {
         const size_t L = (size_t)1 << ctx_logl;
-        l.lt = take(L / 2);
         l.gy = take(2 * L);
         l.raw = take(2 * L);
-        l.ys = take(8 * C);
     } else {
         l.x = take(n);
         l.res = take(n);
@@ -1448,12 +1449,8 @@ int ctx_launch(pfb_mr_ctx *c, const uint64_t *a, const uint64_t *b, uint64_t *ou
 
 }  // namespace
 
-extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs, int n_batch, pfb_mr_ctx_t **out) {
-    if (!out || !e || !N_all || n_limbs <= 0 || n_batch <= 0) {
-        pfb::set_error("pfb_mr_ctx_create: bad argument");
-        return PFB_E_ARG;
-    }
-    *out = nullptr;
+static int ctx_create_on(pfb_mr_t *e, const uint64_t *N_all, int n_limbs, int n_batch, bool fft,
+                         pfb_mr_ctx_t **out) {
     PFB_CUDA(cudaSetDevice(e->device));
     pfb_mr_ctx *c = new pfb_mr_ctx();
     c->e = e;
@@ -1479,7 +1476,7 @@ extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs
             return ctx_fail(c, PFB_E_ARG);
         }
         HostPrep &h = c->hp[i];
-        for (int k = 0; k < fp::kClasses && h.logl <= LOG_LCTA; k++)
+        for (int k = 0; k < fp::kClasses && fft && h.logl <= LOG_LCTA; k++)
             if (fp::class_points(k) == 1 << (h.logl - 1)) h.fpc = k + 1;
         lay[i] = h.fpc ? layout_fp(h.fpc - 1, 0, false, h.logl)
                        : layout_for(h.logl, 1, true, true);  // gy [2][L], spare H-word buffers, raw coefficients
@@ -1531,7 +1528,10 @@ extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs
         ex[i].gy = w + l.gy;
         ex[i].yl = w + l.lt;
         ex[i].raw = (unsigned long long *)(w + l.raw);
-        ex[i].ys = h.fpc ? w + l.ys : nullptr;
+        if (h.fpc) {
+            ex[i].ys = w + l.gy;
+            if (fp::spectrum_outside(h.fpc - 1)) j.sq = w + l.sq;
+        }
         const size_t H = h.nl.size();
         std::vector<uint32_t> npl = h.npl, nl = h.nl;
         if (h.fpc) {  // two digits of 11 bits per limb: the radix R' is the same
@@ -1574,6 +1574,18 @@ extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs
     if (ce != cudaSuccess) return ctx_fail(c, pfb::cuda_fail(ce, "pfb_mr_ctx_create", __FILE__, __LINE__));
     *out = c;
     return PFB_OK;
+}
+
+// As a batch: on the integer engine where the device cannot hold the
+// floating-point engine's buffers (at most 22 words a point, against 21).
+extern "C" int pfb_mr_ctx_create(pfb_mr_t *e, const uint64_t *N_all, int n_limbs, int n_batch, pfb_mr_ctx_t **out) {
+    if (!out || !e || !N_all || n_limbs <= 0 || n_batch <= 0) {
+        pfb::set_error("pfb_mr_ctx_create: bad argument");
+        return PFB_E_ARG;
+    }
+    *out = nullptr;
+    const int rc = ctx_create_on(e, N_all, n_limbs, n_batch, true, out);
+    return rc == PFB_E_NOMEM ? ctx_create_on(e, N_all, n_limbs, n_batch, false, out) : rc;
 }
 
 extern "C" void pfb_mr_ctx_destroy(pfb_mr_ctx_t *c) {

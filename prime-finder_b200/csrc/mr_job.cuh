@@ -55,8 +55,8 @@ enum CtxOp : int {
 struct CtxExtra {
     uint32_t *gy;              // [2][L] spectrum of the second factor
     uint32_t *yl;              // H limbs of the second factor
-    unsigned long long *raw;   // L coefficients of a raw product, or x^2's spectrum (C = L / 2 points)
-    uint32_t *ys;              // floating-point engine: spectra of the second factor, 2 C points
+    unsigned long long *raw;   // L coefficients of a raw product
+    uint32_t *ys;              // floating-point engine: spectra of the second factor, 2 C points (over gy and raw)
 };
 
 }  // namespace mr

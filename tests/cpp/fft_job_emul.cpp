@@ -208,7 +208,7 @@ static void run_ctx(int op, const Words &N, const Words &a, const Words &b) {
     j.fbits = fp::kCtxBits;
     CtxExtra ex{};
     ex.ys = reinterpret_cast<uint32_t *>(ys.data());
-    ex.raw = reinterpret_cast<unsigned long long *>(sq.data());
+    j.sq = reinterpret_cast<uint32_t *>(sq.data());
     auto wide = [&](const Words &w) {
         std::vector<uint16_t> t(n16);
         pfb::big::to_u16(w, t.data(), n16);

@@ -7,6 +7,9 @@
 //                       `allow` device allocations granted after the server's
 //                       creation (-1: all) -> "verdict v" or "stopped rc",
 //                       then the engine that ran it (fft, int, none)
+//   ctx bytes bits n    a context of n moduli on a device of that many bytes beyond
+//                       what the engine holds (-1: no limit) -> "rc c", its device
+//                       memory in bytes and the engine that it was set up for
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
@@ -27,7 +30,8 @@ void set_error(const char *, ...) {}
 int cuda_fail(cudaError_t, const char *, const char *, int) { return PFB_E_CUDA; }
 }  // namespace pfb
 
-static int n_fft, n_int;  // candidates that each engine has finished
+static int n_fft, n_int;        // candidates that each engine has finished
+static int prep_fft, prep_int;  // and that each has set up
 static int fn_fft, fn_int;
 
 namespace pfb {
@@ -35,7 +39,10 @@ namespace mr {
 
 int int_setup(const CrtConsts &, const WideTabs &) { return PFB_OK; }
 void *int_persist_func() { return &fn_int; }
-cudaError_t int_prep(JobDev *, const int *, int, int, const Twiddles &, cudaStream_t) { return cudaSuccess; }
+cudaError_t int_prep(JobDev *, const int *, int n, int, const Twiddles &, cudaStream_t) {
+    prep_int += n;
+    return cudaSuccess;
+}
 cudaError_t int_ctx(const JobDev *, const CtxExtra *, int, int, const uint64_t *, const uint64_t *, uint64_t *, int,
                     int, int, const Twiddles &, cudaStream_t) { return cudaSuccess; }
 cudaError_t int_ctx_check(const uint64_t *, const uint64_t *, const uint64_t *, uint8_t *, int, int, cudaStream_t) {
@@ -54,7 +61,10 @@ Launch persist_launch(const Engine &, bool, int, int n, int sms) {
 }
 cudaError_t ctx(const Engine &, int, const JobDev *, const int *, int, const uint64_t *, const uint64_t *, uint64_t *,
                 int, int, const CtxExtra *, cudaStream_t) { return cudaSuccess; }
-cudaError_t prep(const Engine &, int, JobDev *, const int *, int, cudaStream_t) { return cudaSuccess; }
+cudaError_t prep(const Engine &, int, JobDev *, const int *, int n, cudaStream_t) {
+    prep_fft += n;
+    return cudaSuccess;
+}
 
 }  // namespace fp
 }  // namespace mr
@@ -93,7 +103,9 @@ static std::vector<uint16_t> number(int bits) {
     return l;
 }
 
-static const char *engine() { return n_fft && n_int ? "both" : n_fft ? "fft" : n_int ? "int" : "none"; }
+static const char *engine(int fft, int integer) {
+    return fft && integer ? "both" : fft ? "fft" : integer ? "int" : "none";
+}
 
 int main() {
     fake::launch = launch;
@@ -104,7 +116,7 @@ int main() {
         std::istringstream in(line);
         std::string op;
         in >> op;
-        n_fft = n_int = 0;
+        n_fft = n_int = prep_fft = prep_int = 0;
         if (op == "server") {
             long allow;
             int bits;
@@ -121,8 +133,22 @@ int main() {
             else std::cout << "stopped " << n;
             fake::allow = -1;
             pfb_mr_server_destroy(s);
+            std::cout << " " << engine(n_fft, n_int) << std::endl;
+        } else if (op == "ctx") {
+            long long bytes;
+            int bits, n;
+            in >> bytes >> bits >> n;
+            const std::vector<uint16_t> l = number(bits);
+            std::vector<uint64_t> all;
+            for (int i = 0; i < n; i++) all.insert(all.end(), l.begin(), l.end());
+            const size_t held = fake::used;
+            fake::limit = bytes < 0 ? ~(size_t)0 : held + (size_t)bytes;
+            pfb_mr_ctx_t *c = nullptr;
+            const int rc = pfb_mr_ctx_create(e, all.data(), (int)l.size(), n, &c);
+            std::cout << "rc " << rc << " " << fake::used - held << " " << engine(prep_fft, prep_int) << std::endl;
+            pfb_mr_ctx_destroy(c);
+            fake::limit = ~(size_t)0;
         }
-        std::cout << " " << engine() << std::endl;
     }
     pfb_mr_destroy(e);
     std::cout << "left " << fake::used << std::endl;

@@ -35,3 +35,19 @@ def test_server_needs_no_memory_beyond_the_slot(host, bits):
     request; without room for the slot it reports the request, and stays up."""
     assert host(["server -1 %d" % bits, "server 1 %d" % bits, "server 0 %d" % bits]) == \
         ["verdict 0 fft", "verdict 0 fft", "verdict -1 none"]
+
+
+def test_context_fits_where_the_integer_engine_does(host):
+    """Moduli of 166 000 bits go to the integer engine where only its buffers,
+    21 words a point, fit the device; at 20 000 bits the floating-point
+    engine's buffers are no larger than those."""
+    def integer_bytes(points, bits, n):  # with four 64-bit words per 16-bit limb, and tables
+        return n * (21 * 4 * points + 4 * 8 * ((bits + 15) // 16)) + 8192
+
+    rc, size, eng = host(["ctx -1 166000 4"])[0].split()[1:]
+    assert (rc, eng) == ("0", "fft") and int(size) > integer_bytes(8192, 166000, 4)
+    rc, small, eng = host(["ctx %d 166000 4" % (int(size) - 1)])[0].split()[1:]
+    assert (rc, eng) == ("0", "int") and int(small) <= integer_bytes(8192, 166000, 4)
+    assert host(["ctx %d 166000 4" % (int(small) - 1)])[0].split()[1:] == ["-3", "0", "none"]
+    rc, size, eng = host(["ctx -1 20000 4"])[0].split()[1:]
+    assert (rc, eng) == ("0", "fft") and int(size) <= integer_bytes(1024, 20000, 4)
