@@ -174,9 +174,15 @@ __device__ __forceinline__ Cplx ldcg(const Cplx *p) {
     const double2 v = __ldcg(reinterpret_cast<const double2 *>(p));
     return Cplx{v.x, v.y};
 }
+// Barrier id of the block's named barriers, for N threads.
+template <int N>
+__device__ __forceinline__ void bar_sync(int id) { asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(N) : "memory"); }
 __device__ __forceinline__ long long bits_of(double d) { return __double_as_longlong(d); }
 __device__ __forceinline__ double from_bits(long long v) { return __longlong_as_double(v); }
 #else
+void host_bar_sync(int id, int n);  // (the CPU emulation's)
+template <int N>
+inline void bar_sync(int id) { host_bar_sync(id, N); }
 inline Cplx ldg(const Cplx *p) { return *p; }
 inline Cplx ldcg(const Cplx *p) { return *p; }
 inline long long bits_of(double d) {
@@ -193,24 +199,16 @@ inline double from_bits(long long v) {
 
 template <class F>
 __device__ __forceinline__ void cta_sync() {
-#ifdef __CUDA_ARCH__
     if (F::T == 32) __syncwarp();
     else __syncthreads();
-#else
-    __syncthreads();
-#endif
 }
 
 // The threads of this thread's team.
 template <class F>
 __device__ __forceinline__ void team_sync() {
-#ifdef __CUDA_ARCH__
     if (F::TT == 32) __syncwarp();
     else if (F::TEAMS == 1) __syncthreads();
-    else asm volatile("bar.sync %0, %1;" ::"r"(1 + (int)threadIdx.x / F::TT), "n"(F::TT) : "memory");
-#else
-    __syncthreads();
-#endif
+    else bar_sync<F::TT>(1 + (int)threadIdx.x / F::TT);
 }
 
 template <class F>

@@ -97,7 +97,8 @@ template <class T>
 inline T *dynamic_smem() { return reinterpret_cast<T *>(dyn_smem); }
 
 inline std::vector<Fiber> *fibers = nullptr;
-inline std::vector<Group> *groups = nullptr;  // 0: the CTA; 1 + w: warp w
+inline std::vector<Group> *groups = nullptr;  // 0: the CTA; 1 + w: warp w; then kNamed more
+constexpr int kNamed = 16;
 inline std::vector<unsigned long long> *lane_vals = nullptr;
 inline const std::function<void()> *body = nullptr;
 inline ucontext_t main_ctx;
@@ -202,9 +203,10 @@ struct Saved {
 inline void run_cta(int threads, const std::function<void()> &f) {
     const Saved outer;
     std::vector<Fiber> fs(threads);
-    std::vector<Group> gs(1 + (threads + 31) / 32);
+    const int warps = (threads + 31) / 32;
+    std::vector<Group> gs(1 + warps + kNamed);
     gs[0].size = threads;
-    for (int w = 0; w + 1 < (int)gs.size(); w++) gs[1 + w].size = std::min(32, threads - 32 * w);
+    for (int w = 0; w < warps; w++) gs[1 + w].size = std::min(32, threads - 32 * w);
     std::vector<unsigned long long> vals(threads);
     fibers = &fs;
     groups = &gs;
@@ -269,6 +271,16 @@ inline void run_grid(unsigned gx, unsigned gy, int threads, const std::function<
 }  // namespace emu
 
 inline void __syncthreads() { emu::group_wait(0); }
+inline void __syncwarp() { emu::group_wait(1 + (int)(threadIdx.x >> 5)); }
+
+// bar.sync id, n: named barrier `id` for n threads of the CTA.
+namespace emu {
+inline void named_wait(int id, int n) {
+    const int g = (int)groups->size() - kNamed + id;
+    (*groups)[g].size = n;
+    group_wait(g);
+}
+}  // namespace emu
 
 inline unsigned atomicOr(unsigned *p, unsigned v) {
     const unsigned o = *p;

@@ -31,6 +31,8 @@
 #include "mr_prep_host.h"
 
 using namespace pfb::mr;
+
+void pfb::mr::fp::host_bar_sync(int id, int n) { emu::named_wait(id, n); }
 using pfb::big::Words;
 
 static Words from_hex(const std::string &h) {
