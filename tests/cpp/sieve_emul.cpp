@@ -3,9 +3,10 @@
 // launches are those pfb_sieve_run and pfb_sieve_survivors make for one
 // triple (sieve.cu: ensure_split, enqueue_sieve, pfb_sieve_survivors).
 //
-// Input: "K a b c [compact [unique]]", then "n p_1 ... p_n" (the prime list).
+// Input: "K a b c [compact [unique [sms]]]", then "n p_1 ... p_n" (the prime list).
 // unique = 1 splits the list as pfb_sieve_run_noalloc does (split_unique_kernel:
-// repeated entries listed once, into lists of fixed capacity).
+// repeated entries listed once, into lists of fixed capacity).  sms: the SMs of
+// the GPU, by which the row tiles are sized (148 unless given).
 // Output: the mask as hexadecimal little-endian words (one line), then the
 // number of survivors and the 64-bit FNV-1a hash of the survivor list
 // (k<<16|j as little-endian uint32), in decimal (one line; "0 0" when
@@ -26,10 +27,11 @@ int main() {
     std::string first;
     std::getline(std::cin, first);
     std::istringstream f(first);
-    int compact = 1, unique = 0;
+    int compact = 1, unique = 0, sms = 148;
     f >> K >> abc[0] >> abc[1] >> abc[2];
     if (!(f >> compact)) compact = 1;
     if (!(f >> unique)) unique = 0;
+    if (!(f >> sms)) sms = 148;
     std::cin >> n;
     std::vector<uint32_t> primes(n ? n : 1);
     for (uint32_t i = 0; i < n; i++) std::cin >> primes[i];
@@ -55,10 +57,9 @@ int main() {
         emu::run_grid((n_small_all + 127u) / 128u, 1, 128, [&] {
             small_setup_kernel(tiny.data(), small.data(), counts.data(), abc, 1, K, 2u * cap, rec.data());
         });
-        const uint32_t tiles = ((uint32_t)K + kTileRows - 1u) / kTileRows;
-        const uint32_t rows = (uint32_t)K < (uint32_t)kTileRows ? (uint32_t)K : (uint32_t)kTileRows;
-        emu::run_grid(tiles, 1, kBlockTile, [&] {
-            small_tile_kernel(rec.data(), counts.data(), 2u * cap, abc, K, mask.data(), wpt);
+        const uint32_t rows = tile_rows(K, 1, sms);
+        emu::run_grid(((uint32_t)K + rows - 1u) / rows, 1, kBlockTile, [&] {
+            small_tile_kernel(rec.data(), counts.data(), 2u * cap, abc, K, mask.data(), wpt, rows);
         }, tile_smem_bytes(rows, K));
     }
     // medium primes (a warp per prime, a small grid so that the warps take

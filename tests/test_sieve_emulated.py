@@ -42,8 +42,9 @@ def emul(tmp_path_factory):
     return exe
 
 
-def _run(exe, P, a, b, c, K, env=None, compact=True, unique=False):
-    inp = "%d %d %d %d %d %d\n%d %s\n" % (K, a, b, c, int(compact), int(unique), len(P), " ".join(map(str, P)))
+def _run(exe, P, a, b, c, K, env=None, compact=True, unique=False, sms=148):
+    inp = "%d %d %d %d %d %d %d\n%d %s\n" % (K, a, b, c, int(compact), int(unique), sms, len(P),
+                                              " ".join(map(str, P)))
     r = subprocess.run([exe], input=inp, capture_output=True, text=True, env=env, timeout=600)
     assert r.returncode == 0, r.stderr[-2000:]
     first, second = r.stdout.split("\n")[:2]
@@ -131,6 +132,24 @@ def test_line_coefficients_montgomery_and_barrett(tmp_path):
     assert int(r.stdout.split()[1]) >= 200 * 30 * 4
 
 
+@pytest.mark.parametrize("K,sms,rows", [(97, 3, 4), (101, 1, 12), (150, 148, 1), (333, 1, 41), (333, 2, 20),
+                                        (1001, 1, 64), (1001, 2, 62), (1001, 3, 41)])
+def test_emulated_sieve_tile_heights(emul, K, sms, rows):
+    """Row tiles of every height, by the number of SMs: odd K, so that two tiles
+    share a mask word and a tile begins at any bit of one."""
+    assert max(1, min(64, K // (8 * sms))) == rows
+    _check(*_run(emul, P5[:3000], 50000, 30000, 100, K, sms=sms)[:3], P5[:3000], 50000, 30000, 100, K)
+
+
+@pytest.mark.parametrize("K", [1, 9, 10, 99, 100, 179, 180, 181, 256])
+def test_emulated_sieve_around_the_row_by_row_limit(emul, K):
+    """Grids on both sides of kDirectK = 180, and of the digit counts: the large
+    primes' rows one by one against the lattice; exponents of either order."""
+    P = [p for p in P5 if p > 4000][::7] + [2147483629, 2147483647, 4294967279, 4294967291]
+    for a, b, c in [(50000, 30000, 100), (60, 57, 2), (40, 20, 39), (7, 5, 0)]:
+        _check(*_run(emul, P, a, b, c, K)[:3], P, a, b, c, K)
+
+
 def test_emulated_sieve_in_bounds(tmp_path):
     exe = str(tmp_path / "sieve_emul_asan")
     cc = _build(exe, asan=True)
@@ -138,8 +157,9 @@ def test_emulated_sieve_in_bounds(tmp_path):
         pytest.skip("no AddressSanitizer runtime")
     assert cc.returncode == 0, cc.stderr
     env = dict(os.environ, ASAN_OPTIONS="detect_stack_use_after_return=0:detect_leaks=0")
-    for a, b, c, K in [(50000, 30000, 100, 100), (181, 9, 3, 150), (120, 70, 30, 1000)]:
-        got, count, surv, err = _run(exe, P5, a, b, c, K, env=env)
+    for a, b, c, K, sms in [(50000, 30000, 100, 100, 148), (181, 9, 3, 150, 148), (120, 70, 30, 1000, 148),
+                            (120, 70, 30, 1000, 1), (120, 70, 30, 333, 2)]:
+        got, count, surv, err = _run(exe, P5, a, b, c, K, env=env, sms=sms)
         assert "ERROR: AddressSanitizer" not in err
         _check(got, count, surv, P5, a, b, c, K)
 
