@@ -94,3 +94,12 @@ def test_lucas_mersenne_prime_long_transform(mr):
     """M_216091 (216 091 bits): the length-2^15 transforms with the spectra of
     the two NTT primes computed one after the other (D = 5, Q = -1)."""
     assert mr.lucas([(1 << 216091) - 1]) == [1]
+
+
+def test_lucas_primes_of_other_fft_classes(mr):
+    """Known primes at 64 to 4096 points of the floating-point engine, where no
+    Mersenne prime above has them, and composites beside them, in one batch."""
+    ps = [5 * 2**n + 1 for n in (1947, 5947, 13165, 26607)] + [3 * 2**54792 + 1]
+    ps += [(1 << p) - 1 for p in (3217, 4423, 11213, 19937, 86243, 110503)]
+    composites = [p * q for p, q in zip(ps[:3], ps[1:4])]
+    assert mr.lucas(ps + composites) == [1] * len(ps) + [0] * len(composites)

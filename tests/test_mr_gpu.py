@@ -147,6 +147,40 @@ def test_bucket_boundaries(mr):
         assert r == pow(2, 0xDEADBEEF, N), N.bit_length()
 
 
+# complex points and widest limb of the floating-point engine's length classes
+FFT_CLASSES = [(64, 19), (96, 18), (128, 18), (192, 18), (256, 17), (384, 17), (512, 17), (768, 16), (1024, 16),
+               (1536, 16), (2048, 16), (3072, 15), (4096, 15), (6144, 15), (8192, 15), (12288, 14)]
+
+
+def test_fft_class_limits_in_one_batch(mr):
+    """The largest base-2 modulus of every length class (2 C b - 6 bits) and one
+    bit more, in one batch, with more numbers of the first class, and of one
+    with a block per SM, than there are resident blocks (their quanta are
+    shared out)."""
+    rng = random.Random(14)
+    bits = [2 * C * b - 6 + more for C, b in FFT_CLASSES for more in (0, 1)]
+    bits += [2000] * 4000 + [90_000] * 160
+    rng.shuffle(bits)
+    Ns = [rng.getrandbits(b) | (1 << (b - 1)) | 1 for b in bits]
+    Es = [rng.getrandbits(100 if b == 2000 else 70) | (1 << 69) for b in bits]
+    got = mr.powm(Ns, Es, 2)
+    for N, E, r in zip(Ns, Es, got):
+        assert r == (pow(2, E, N) if N.bit_length() < 3000 else _gmp_powm(2, E, N)), N.bit_length()
+
+
+def test_strong_tests_at_fft_class_limits(mr):
+    rng = random.Random(15)
+    Ns = []
+    for C, b in FFT_CLASSES[:8]:
+        for bits in (2 * C * b - 6, 2 * C * b - 5):
+            Ns.append(rng.getrandbits(bits) | (1 << (bits - 1)) | 1)
+    Ns += [5 * 2**1947 + 1, 5 * 2**3313 + 1, 5 * 2**5947 + 1, 5 * 2**13165 + 1]  # primes, s in the thousands
+    ver, res = mr.test(Ns, 2)
+    assert ver[-4:] == [1] * 4
+    for N, v, r in zip(Ns, ver, res):
+        assert (v, r) == (oracle.strong_test(N, 2), oracle.strong_residue(N, 2)[1]), N.bit_length()
+
+
 def _golden(name):
     path = os.path.join(GOLD, name)
     if not os.path.exists(path):
