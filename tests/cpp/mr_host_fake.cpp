@@ -7,6 +7,9 @@
 //                       `allow` device allocations granted after the server's
 //                       creation (-1: all) -> "verdict v" or "stopped rc",
 //                       then the engine that ran it (fft, int, none)
+//   batch bytes bits n  strong tests of n numbers on a device of that many bytes
+//                       beyond what the engine holds (-1: no limit) -> "rc c",
+//                       device memory of the batch and the engine that ran it
 //   ctx bytes bits n    a context of n moduli on a device of that many bytes beyond
 //                       what the engine holds (-1: no limit) -> "rc c", its device
 //                       memory in bytes and the engine that it was set up for
@@ -134,6 +137,19 @@ int main() {
             fake::allow = -1;
             pfb_mr_server_destroy(s);
             std::cout << " " << engine(n_fft, n_int) << std::endl;
+        } else if (op == "batch") {
+            long long bytes;
+            int bits, n;
+            in >> bytes >> bits >> n;
+            const std::vector<uint16_t> l = number(bits);
+            const std::vector<pfb_mr_number_t> nums(n, pfb_mr_number_t{l.data(), (int)l.size()});
+            std::vector<int8_t> verdict(n);
+            const size_t held = fake::used;
+            fake::limit = bytes < 0 ? ~(size_t)0 : held + (size_t)bytes;
+            fake::peak = held;
+            const int rc = pfb_mr_test(e, nums.data(), n, 2u, verdict.data(), nullptr, 0);
+            std::cout << "rc " << rc << " " << fake::peak - held << " " << engine(n_fft, n_int) << std::endl;
+            fake::limit = ~(size_t)0;
         } else if (op == "ctx") {
             long long bytes;
             int bits, n;

@@ -51,3 +51,14 @@ def test_context_fits_where_the_integer_engine_does(host):
     assert host(["ctx %d 166000 4" % (int(small) - 1)])[0].split()[1:] == ["-3", "0", "none"]
     rc, size, eng = host(["ctx -1 20000 4"])[0].split()[1:]
     assert (rc, eng) == ("0", "fft") and int(size) <= integer_bytes(1024, 20000, 4)
+
+
+@pytest.mark.parametrize("bits", [700, 20_000, 123_100, 344_000])
+def test_batch_falls_back_to_the_integer_engine(host, bits):
+    """Where the floating-point engine's buffers do not fit the device, the
+    batch runs on the integer engine; below that it is refused."""
+    rc, size, eng = host(["batch -1 %d 6" % bits])[0].split()[1:]
+    assert (rc, eng) == ("0", "fft")
+    rc, small, eng = host(["batch %d %d 6" % (int(size) - 1, bits)])[0].split()[1:]
+    assert (rc, eng) == ("0", "int") and int(small) < int(size)
+    assert host(["batch %d %d 6" % (int(small) - 1, bits)])[0].split()[1:] == ["-3", "0", "none"]

@@ -155,3 +155,33 @@ def test_slot_allocation_failure_recovery(engine):
     for tag, N in list(zip((10, 11), longs)) + list(zip((20, 21, 22), shorts)):
         assert got[tag]["verdict"] == oracle.strong_test(N, 2)
         assert got[tag]["residue"] == oracle.strong_residue(N, 2)[1]
+
+
+def test_integer_engine_where_its_slot_alone_fits(engine):
+    """A budget of one slot of the integer engine puts a number on that engine
+    at every transform length: the length's largest modulus gives the residue
+    that the floating-point engine gives, and a 50 000-digit number GMP's."""
+    rng = random.Random(23)
+    rec = json.load(open(os.path.join(os.path.dirname(__file__), "golden", "mr_50k_first16.json")))["records"][0]
+    Ns = {}
+    for lg in range(8, 14):
+        bits = 22 * (1 << (lg - 1)) - 36
+        Ns[lg] = rng.getrandbits(bits) | (1 << (bits - 1)) | 1
+    Ns[14] = oracle.build_candidate(rec["a"], rec["b"], rec["c"], rec["k"], rec["j"], bool(rec["rev"]))
+    want_v, want_r = engine.test([Ns[lg] for lg in range(8, 14)], 2)
+    servers, slot = {}, {}
+    for lg, N in Ns.items():
+        H = 1 << (lg - 1)
+        words = [H, H, 2 * H, 2 * H, H, H, (22 * H + 31) // 32 + 1]
+        slot[lg] = sum(4 * ((w + 63) & ~63) for w in words)
+        servers[lg] = pfb200.MRServer(engine, max_resident=1, hbm_budget_bytes=slot[lg], chunk_steps=2048)
+        servers[lg].submit(N, tag=lg, residue=True)
+    got = {}
+    for lg, srv in servers.items():
+        got.update(_drain(srv, 1, 300))
+        assert srv.stats()["bytes_owned"] == slot[lg]
+        srv.close()
+    for lg in range(8, 14):
+        assert (got[lg]["verdict"], got[lg]["residue"]) == (want_v[lg - 8], want_r[lg - 8]), lg
+    n16 = (Ns[14].bit_length() + 15) // 16
+    assert hashlib.sha256(got[14]["residue"].to_bytes(2 * n16, "little")).hexdigest() == rec["sha256"]
