@@ -233,13 +233,17 @@ int pfb_mr_radix16_forms(pfb_mr_t *e, int ctas, int reps, double *ms_butterfly, 
 
 /*
  * Autotuner of the persistent squaring kernel, per transform-length bucket
- * (log2 L from logl_lo to logl_hi, within 8..15; a 50 000-digit modulus is
- * 14, 100 000 digits 15).  For each bucket it times 2048 squarings of
- * synthetic moduli of the bucket's largest size, in batches of one and of two
+ * (log2 L from logl_lo to logl_hi, within 8..15: the integer engine's length
+ * for the longest number of a batch, whichever engine runs it; a 50 000-digit
+ * modulus is 14, 100 000 digits 15).  For each bucket it times 2048 squarings of
+ * synthetic moduli of the bucket's largest size (at 15, of the largest that
+ * the floating-point engine takes), in batches of one and of two
  * candidates per SM, for every pair (quantum: steps of one candidate per
  * scheduling quantum, 16 to 64; chunk: steps per launch, 1024 or 2048), and
  * keeps in the engine, for every later batch of that bucket, the pair with
  * the best sum over the two shapes of its rate relative to the shape's best.
+ * Where every candidate has a block of its own, a launch does not depend on
+ * the quantum: the shape is timed once per chunk, and the rows repeat it.
  * results (optional, cap rows) receives one row per pair; *n_results the rows
  * written.  The defaults before tuning are quantum 64, chunk 2048.
  */

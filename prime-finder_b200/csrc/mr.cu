@@ -513,6 +513,17 @@ int batch_advance(pfb_mr_batch *b, long long steps, cudaStream_t st) {
     return PFB_OK;
 }
 
+// Whether a launch depends on the quantum: not where every candidate has a CTA
+// of its own (fp_quanta).
+bool uses_quantum(const pfb_mr_batch *b) {
+    bool used = b->runs.n_int > 0;
+    for (int c = 0; c < fp::kClasses; c++) {
+        const int n = b->runs.count[c];
+        used = used || (n && n > (int)fp::persist_launch(b->e->fe, b->mode == 2, c, n, b->e->num_sms).grid.x);
+    }
+    return used;
+}
+
 int batch_pending(pfb_mr_batch *b, int *pending, long long *steps_total) {
     PFB_CUDA(cudaStreamSynchronize(b->e->stream));
     PFB_CUDA(cudaDeviceSynchronize());
@@ -683,8 +694,8 @@ extern "C" int pfb_mr_autotune(pfb_mr_t *e, int logl_lo, int logl_hi, pfb_mr_tun
     PFB_CUDA(cudaSetDevice(e->device));
     // quanta above 64 steps leave SMs idle at the end of each launch once a
     // batch holds several candidates per SM, so the search stays below
-    static const int kQuanta[] = {16, 32, 64};
-    static const int kChunks[] = {1024, 2048};
+    static const int kQuanta[] = {64, 32, 16};  // (of equal rates the first, the default, is kept)
+    static const int kChunks[] = {2048, 1024};
     constexpr int NQ = 3, NC = 2, NP = NQ * NC;
     const long long kSteps = 2048;  // timed steps per tried pair and batch shape
     const int sms = std::max(1, e->num_sms);
@@ -695,8 +706,10 @@ extern "C" int pfb_mr_autotune(pfb_mr_t *e, int logl_lo, int logl_hi, pfb_mr_tun
     PFB_CUDA(cudaEventCreate(&ev[1]));
     int rc = PFB_OK;
     for (int lg = logl_lo; lg <= logl_hi && !rc; lg++) {
-        // the longest base-2 modulus of this length: R = 2^(22 L/2) >= 2^(bits + 6)
-        const size_t bits = std::min<size_t>((size_t)LIMB_BITS * ((size_t)1 << (lg - 1)) - 8, PFB_MR_MAX_BITS);
+        // the longest base-2 modulus of this length, R = 2^(22 L/2) >= 2^(bits + 6),
+        // that the floating-point engine takes (all but the last 5 % of 2^15)
+        const size_t fp_bits = (size_t)fp::limb_bits(fp::kClasses - 1) * 2 * fp::class_points(fp::kClasses - 1) - 6;
+        const size_t bits = std::min((size_t)LIMB_BITS * ((size_t)1 << (lg - 1)) - 8, fp_bits);
         const int n16 = (int)((bits + 15) / 16);
         const int q_old = e->quantum[lg], c_old = e->chunk[lg];
         double rate[2][NP] = {};
@@ -723,7 +736,12 @@ extern "C" int pfb_mr_autotune(pfb_mr_t *e, int logl_lo, int logl_hi, pfb_mr_tun
             rc = batch_build(e, nums.data(), n, 2u, 1, nullptr, &b);
             if (rc) break;
             rc = batch_advance(b, 64, e->stream);  // warm-up
+            const bool quantum_used = uses_quantum(b);
             for (int k = 0; k < NP && !rc; k++) {
+                if (k >= NC && !quantum_used) {  // the launches of the first quantum again
+                    rate[shape][k] = rate[shape][k % NC];
+                    continue;
+                }
                 e->quantum[lg] = kQuanta[k / NC];
                 e->chunk[lg] = kChunks[k % NC];
                 long long before = 0, after = 0;

@@ -13,6 +13,8 @@
 //   ctx bytes bits n    a context of n moduli on a device of that many bytes beyond
 //                       what the engine holds (-1: no limit) -> "rc c", its device
 //                       memory in bytes and the engine that it was set up for
+//   tune lg             autotune of one transform length -> "rc c", launches of the
+//                       persistent kernel and the pair kept
 #include <algorithm>
 #include <chrono>
 #include <condition_variable>
@@ -35,6 +37,7 @@ int cuda_fail(cudaError_t, const char *, const char *, int) { return PFB_E_CUDA;
 
 static int n_fft, n_int;        // candidates that each engine has finished
 static int prep_fft, prep_int;  // and that each has set up
+static int launches;
 static int fn_fft, fn_int;
 
 namespace pfb {
@@ -86,12 +89,14 @@ static std::function<void()> launch(void *func, void **a) {
     if (func == &fn_int) {
         const int n = *(int *)a[1];
         return [=] {
+            launches++;
             for (int i = 0; i < n; i++)
                 if (!jobs[i].fpc) finish(jobs[i], n_int);
         };
     }
     const int *list = *(const int **)a[1], n = *(int *)a[2];
     return [=] {
+        launches++;
         for (int i = 0; i < n; i++) finish(jobs[list[i]], n_fft);
     };
 }
@@ -119,7 +124,7 @@ int main() {
         std::istringstream in(line);
         std::string op;
         in >> op;
-        n_fft = n_int = prep_fft = prep_int = 0;
+        n_fft = n_int = prep_fft = prep_int = launches = 0;
         if (op == "server") {
             long allow;
             int bits;
@@ -150,6 +155,12 @@ int main() {
             const int rc = pfb_mr_test(e, nums.data(), n, 2u, verdict.data(), nullptr, 0);
             std::cout << "rc " << rc << " " << fake::peak - held << " " << engine(n_fft, n_int) << std::endl;
             fake::limit = ~(size_t)0;
+        } else if (op == "tune") {
+            int lg, q = 0, ch = 0;
+            in >> lg;
+            const int rc = pfb_mr_autotune(e, lg, lg, nullptr, 0, nullptr);
+            pfb_mr_get_tuning(e, lg, &q, &ch);
+            std::cout << "rc " << rc << " " << launches << " " << q << " " << ch << std::endl;
         } else if (op == "ctx") {
             long long bytes;
             int bits, n;

@@ -62,3 +62,10 @@ def test_batch_falls_back_to_the_integer_engine(host, bits):
     rc, small, eng = host(["batch %d %d 6" % (int(size) - 1, bits)])[0].split()[1:]
     assert (rc, eng) == ("0", "int") and int(small) < int(size)
     assert host(["batch %d %d 6" % (int(small) - 1, bits)])[0].split()[1:] == ["-3", "0", "none"]
+
+
+def test_autotune_times_what_a_quantum_changes(host):
+    """With a block for each candidate the quantum has no part in the launch, so
+    the shape of one candidate per SM is timed once per chunk: 1 + 3 launches,
+    and 1 + 9 with two per SM; equal rates keep the defaults."""
+    assert host(["tune 12", "tune 15"]) == ["rc 0 14 64 2048"] * 2
