@@ -15,10 +15,12 @@ Beside it the line reports:
   plain        the one-candidate-per-call form on the same GPU
   sieve        K = 9999 grid pairs/s over the (a,b,c) triples of the
                wide-grid triple enumeration, and the drop-in 100 x 100 call
-  roofline     INT32 multiplies of the reference's squaring structure
-               (6 length-L transforms + 3 pointwise products, 2 primes, 3
-               multiplies per modmul, L = 32768 at 50 000 digits) per second,
-               over this device's measured INT32 multiply peak
+  roofline     double-precision instructions of the engine's squaring (seven
+               complex transforms of 6144 points at 50 000 digits) per second,
+               over this device's measured rate of fused multiply-adds; beside
+               it the INT32 multiplies that the reference's squaring structure
+               takes for the same work (6 length-L transforms + 3 pointwise
+               products, 2 primes, 3 multiplies per modmul, L = 32768)
   cpu_baseline GMP 6.3 mpz_powm on the host cores, sampled
 
 Multi-GPU: one process per GPU (torchrun), each an independent replica
@@ -44,13 +46,21 @@ SQ_PER_MODMUL = 3  # INT32 multiplies per modular multiplication (reference coun
 METRIC = "MR base-2 tests/s, uniform batch of 256 x 50 000-digit candidates, served/batched"
 WORKLOAD = ("uniform MR batch: 256 x 50 000-digit N/rev(N), (k,j) from the (50000,30000,100) sieve "
             "survivors, splitmix64 seed 1")
-# dram__bytes_read.sum + dram__bytes_write.sum of the timed persist_kernel launch of
-# the uniform batch (1024 squarings x 256 candidates, L2 flushed before it), from one
-# ncu capture of this build (profiles/persist_kernel_uniform_batch_dram.txt), in a run
-# whose autotuner chose 16-step quanta at L = 2^14: a run with longer quanta re-reads
-# the residues less often
-PERSIST_LAUNCH_DRAM_BYTES = 73122560 + 30478080
-PERSIST_LAUNCH_DRAM_QUANTUM = 16
+# complex points and widest limb (bits) of the squaring engine's length classes
+FFT_CLASSES = [(64, 19), (96, 18), (128, 18), (192, 18), (256, 17), (384, 17), (512, 17), (768, 16), (1024, 16),
+               (1536, 16), (2048, 16), (3072, 15), (4096, 15), (6144, 15), (8192, 15), (12288, 14)]
+
+
+def fp64_ops_per_squaring(bits: int) -> int:
+    """Double-precision instructions (adds, multiplies, fused multiply-adds) of
+    one base-2 squaring modulo a number of `bits` bits: per complex point and
+    binary level 3 in each of the four forward transforms and 4 in each of the
+    three inverse ones, 6 and 20/3 for a ternary level, and 37 for the
+    conversions, the pointwise products and the rounding."""
+    points = next(c for c, b in FFT_CLASSES if 2 * c * b >= bits + 6)
+    ternary = points % 3 == 0
+    levels = (points // 3 if ternary else points).bit_length() - 1
+    return points * (24 * levels + 44 * ternary + 37)
 
 
 def ref_modmuls_per_squaring(digits: int) -> int:
@@ -321,8 +331,8 @@ def radix_case(ctas=592, reps=20):
     print(json.dumps(r))
 
 
-# small cases of the squaring kernel for ncu captures: N and rev(N) of four
-# (k, j) at one (a, b, c), 8 candidates (one CTA each), one launch of 64 squarings
+# small cases of the squaring kernel (6144 and 12288 points) for ncu captures: N and
+# rev(N) of four (k, j) at one (a, b, c), 8 candidates (one CTA each), one launch of 64 squarings
 MR_CASES = {
     "50k": ((50000, 30000, 100), None),  # the first four survivors of (50000, 30000, 100)
     "100k": ((100000, 60000, 100), [(1, 99), (2, 84), (4, 60), (5, 84)]),
@@ -539,17 +549,16 @@ def main():
     cands = [pfb200.build_candidate(*abc1, k, j, rev) for (k, j) in pairs for rev in (False, True)]
     sq_per_test = statistics.mean([(N - 1).bit_length() for N in cands])  # bits(d) + 1 check, s = 1
     eng = pfb200.MillerRabin(dev)
-    # per-length tuning of the persistent kernel (quantum, steps per launch)
+    # per-length tuning of the persistent kernels (quantum, steps per launch)
     tune = eng.autotune(14, 15)
     autotune = {"chosen": {str(k): {"quantum": v[0], "chunk": v[1]} for k, v in tune["chosen"].items()},
                 "tried": [[r["logl"], r["quantum"], r["chunk"], round(r["squarings_per_s_1"]),
                            round(r["squarings_per_s_2"])] for r in tune["tried"]],
                 "columns": "logl, quantum, chunk, squarings/s at 1 and at 2 candidates per SM",
-                "fixed": {"lengths": "powers of two 2^8..2^15 (the NTT primes have no factor 3 in p - 1)",
-                          "radix": "16 (remainder pass 2, 4 or 8)",
-                          "product_form": "one length-L square up to 2^14, cyclic and negacyclic "
-                                          "halves at 2^15 (shared-memory capacity)",
-                          "candidates_per_cta": "1 (512 threads x 128 registers fill the register file)",
+                "fixed": {"lengths": "16 classes of 2^k and 3 2^k complex points, 64 to 12288; the integer "
+                                     "engine above 344 058 bits",
+                          "radix": "4 to 24 by class, three or four passes",
+                          "candidates_per_cta": "1 (32 to 512 threads by class)",
                           "cluster": "1"}}
     batch = pfb200.MRBatch(eng, cands, 2)
     flush = torch.empty(256 * 1024 * 1024, dtype=torch.uint8, device="cuda")
@@ -621,22 +630,20 @@ def main():
                               "b ~ U[c+1,a-1], k,j ~ U[1,9999], N or rev(N); 256 squarings each per step"}
 
     # roofline of the squaring kernel
-    peak_lo, peak_hi = pfb200.measure_int32_peak(dev)
+    peak = pfb200.measure_fp64_peak(dev)
+    int_peak = pfb200.measure_int32_peak(dev)[0]
     digits = len(str(cands[0]))
+    ops = statistics.mean(fp64_ops_per_squaring(N.bit_length()) for N in cands)
     ref_mults = ref_modmuls_per_squaring(digits) * SQ_PER_MODMUL
-    achieved = squarings / t_mr * ref_mults  # INT32 multiplies / s (one GPU)
-    roofline = {"bound": "int32", "achieved": achieved / 1e12, "peak": peak_lo / 1e12, "unit": "Tmul/s",
-                "frac": achieved / peak_lo,
-                # DRAM bytes (read + write) of one timed launch of this workload, from one ncu
-                # capture of this build (see PERSIST_LAUNCH_DRAM_BYTES); the quantum of that
-                # capture and this run's are both reported
-                "traffic": PERSIST_LAUNCH_DRAM_BYTES if chunk == 1024 and n == 256 else None,
-                "traffic_source": "ncu capture of this build's timed launch (profiles/"
-                                  "persist_kernel_uniform_batch_dram.txt), %d-step quanta" % PERSIST_LAUNCH_DRAM_QUANTUM,
+    achieved = squarings / t_mr * ops  # FP64 instructions (per thread) / s (one GPU)
+    roofline = {"bound": "fp64", "achieved": achieved / 1e12, "peak": peak / 1e12, "unit": "T FP64 instructions/s",
+                "frac": achieved / peak,
+                "peak_source": "measured live: pfb_measure_fp64_peak (fused multiply-adds)",
+                "work": "%d FP64 instructions per squaring" % round(ops),
                 "quantum": eng.tuning(14)[0],
-                "peak_source": "measured live: pfb_measure_int32_peak (mul.lo)",
-                "mul_hi_peak": peak_hi / 1e12,
-                "work": "%d INT32 multiplies per squaring (reference structure at %d digits)" % (ref_mults, digits)}
+                "reference_structure": {"int32_mults_per_squaring": ref_mults,
+                                        "equivalent_tmul_per_s": squarings / t_mr * ref_mults / 1e12,
+                                        "measured_int32_peak_tmul_per_s": int_peak / 1e12}}
 
     # --- serving: continuous batching under Poisson arrivals ---------------
     serving = None
@@ -732,7 +739,7 @@ def main():
         "metric": METRIC,
         "value": tests_s, "unit": "tests/s", "n_gpus": world, "steps": args.steps, "warmup": args.warmup,
         "ms_per_step": ms_per_step, "higher_is_better": True, "scaling": "weak", "vs_baseline": None,
-        "dtype": "u32", "data": "synthetic",
+        "dtype": "f64", "data": "synthetic",
         "config": {"workload": WORKLOAD, "candidates": n, "squarings_per_step": chunk, "squarings_per_test": sq_per_test,
                    "l2": "flushed between timed steps (256 MiB write)", "parallelism": "replicas"},
         "plain": {"value": plain_tests_s, "unit": "tests/s", "seconds": plain_s,

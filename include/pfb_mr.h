@@ -213,9 +213,11 @@ void pfb_mr_server_destroy(pfb_mr_server_t *s);
  * the engine's throughput counters. */
 long long pfb_mr_test_cost(const uint16_t *limbs, int n_limbs);
 
-/* Sustained 32-bit integer multiply rate of the device (ops/s), for the
- * low-half and high-half forms: the roofline denominator of the squaring
- * kernel.  No counterpart in the reference (a measurement utility). */
+/* Sustained rates of the device (ops/s): double-precision fused multiply-adds,
+ * and 32-bit integer multiplies in the low-half and high-half forms: the
+ * roofline denominators of the two squaring engines.  No counterpart in the
+ * reference (measurement utilities). */
+int pfb_measure_fp64_peak(int device, double *fma_per_s);
 int pfb_measure_int32_peak(int device, double *mul_lo_per_s, double *mul_hi_per_s);
 
 /*

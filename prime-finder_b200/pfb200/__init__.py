@@ -368,6 +368,8 @@ def _batch_lib():
         L.pfb_mr_batch_destroy.restype = None
         L.pfb_measure_int32_peak.argtypes = [C.c_int, C.POINTER(C.c_double), C.POINTER(C.c_double)]
         L.pfb_measure_int32_peak.restype = C.c_int
+        L.pfb_measure_fp64_peak.argtypes = [C.c_int, C.POINTER(C.c_double)]
+        L.pfb_measure_fp64_peak.restype = C.c_int
         L._batch_ready = True
     return L
 
@@ -433,6 +435,13 @@ def radix16_forms(engine: "MillerRabin", ctas: int = 592, reps: int = 20) -> dic
     tb, tt, bad, err = C.c_double(), C.c_double(), C.c_longlong(), C.c_int()
     _check(f(engine._h, ctas, reps, C.byref(tb), C.byref(tt), C.byref(bad), C.byref(err)), "pfb_mr_radix16_forms")
     return {"ms_butterfly": tb.value, "ms_tensor": tt.value, "mismatches": bad.value, "tensor_timeout": err.value}
+
+
+def measure_fp64_peak(device: int = 0):
+    """Double-precision fused multiply-adds per second sustained on `device`."""
+    r = C.c_double(0)
+    _check(_batch_lib().pfb_measure_fp64_peak(device, C.byref(r)), "pfb_measure_fp64_peak")
+    return r.value
 
 
 def measure_int32_peak(device: int = 0):

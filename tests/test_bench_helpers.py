@@ -19,6 +19,14 @@ def test_reference_work_count():
     assert bench.ref_modmuls_per_squaring(50000) == 2 * (6 * (L // 2) * 15 + 3 * L)
 
 
+def test_engine_work_count():
+    """FP64 instructions of one squaring against the counter of a run
+    (smsp__inst_executed_pipe_fp64 warp instructions, 64 squarings of four
+    numbers): within 2 % at 2^k and 3 2^k points."""
+    for bits, warp_instructions in ((32760, 8844), (49144, 14220), (184312, 66072), (245752, 89136)):
+        assert abs(bench.fp64_ops_per_squaring(bits) / 32 / warp_instructions - 1) < 0.02, bits
+
+
 def test_mr_cases_are_eight_candidates():
     for name, (abc, pairs) in bench.MR_CASES.items():
         a, b, c = abc
