@@ -5,8 +5,9 @@
  * (miller_rabin_gpu/: BatchModCtx batch_mod_ctx.cuh:101-228,
  * gpu_miller_rabin_s1 / gpu_miller_rabin miller_rabin_runner.cuh:26-49) and
  * of the CPU phase-2 call miller_rabin_test (miller_rabin.h:24-25), with the
- * arithmetic on the GPU: exact NTT squaring over two 30-bit primes,
- * Montgomery reduction and carry propagation fused in one CTA per candidate.
+ * arithmetic on the GPU: exact Montgomery squarings, one CTA per candidate,
+ * on double-precision FFTs up to 344 058 bits (base 2) and on integer
+ * transforms over two 30-bit primes above.
  *
  * Numbers cross this boundary as little-endian 16-bit limbs, the limb format
  * of the reference (ntt_merge.cuh:14-19, candidate.cuh:11-18); candidates of
@@ -37,7 +38,7 @@ typedef struct {
     int n_limbs;
 } pfb_mr_number_t;
 
-/* Engine on `device`: twiddle tables and constants are set up once. */
+/* Engine on `device`: roots, twiddle tables and constants are set up once. */
 int pfb_mr_create(pfb_mr_t **out, int device);
 void pfb_mr_destroy(pfb_mr_t *e);
 /* Device the engine was created on, or -1 for NULL. */
@@ -92,11 +93,15 @@ int pfb_mr_powm(pfb_mr_t *e, const pfb_mr_number_t *nums, int n, uint32_t base,
  * miller_rabin_runner.cu:281-359, with the candidates' state kept in device
  * memory between calls).  A step is one modular squaring of every unfinished
  * candidate (or one verdict check).
- *   create   host set-up, upload and transforms of N and N' (synchronous)
+ *   create   host set-up, upload and transforms of N and N' (synchronous);
+ *            0.47 MB of device memory per 50 000-digit number, 0.93 MB at
+ *            100 000 digits; where that does not fit, the whole batch on the
+ *            integer engine (0.28 and 0.63 MB)
  *   advance  enqueue about `steps` steps of every unfinished candidate on
- *            `stream` (NULL = engine stream): a persistent kernel, one CTA
- *            per SM, hands out quanta of 64 steps round-robin, so the SMs
- *            stay busy whatever the number and lengths of the candidates;
+ *            `stream` (NULL = engine stream): one persistent kernel per
+ *            length class, side by side, with as many CTAs as fit the SMs;
+ *            a CTA takes a candidate for the whole launch where each has
+ *            one, else for quanta of 64 steps (pfb_mr_autotune) round-robin;
  *            advances on different streams may overlap (a candidate is taken
  *            by one CTA at a time)
  *   pending  number of unfinished candidates (synchronises the device)
@@ -120,7 +125,7 @@ void pfb_mr_batch_destroy(pfb_mr_batch_t *b);
  * the engine one Montgomery step per call.  Operands use the reference's
  * layout: n_limbs 16-bit limbs per modulus, one per uint64, little-endian,
  * n_batch moduli back to back.  The working form ("residue") of x is
- * x R mod N, fully reduced, with R = 2^(22 H) of the modulus' transform
+ * x R mod N, fully reduced, with R = 2^(22 H) + 1 of the modulus' transform
  * length H (the reference's Montgomery form with its own R).
  *   create        host set-up of every modulus (odd, > 1, at most
  *                 PFB_MR_MAX_BITS bits; PFB_E_ARG otherwise) and transforms
@@ -160,9 +165,11 @@ int pfb_mr_ctx_mul_raw(pfb_mr_ctx_t *c, const uint64_t *d_a, const uint64_t *d_b
  * Requests arrive one by one from any thread; host workers do the set-up;
  * a driver thread admits prepared requests into free device slots as slots
  * and the HBM budget allow, advances every resident candidate by
- * chunk_steps per launch of the persistent kernel (candidates of different
- * lengths share every launch), and retires finished ones.  Per-candidate
- * residue and exponent cursor live in device memory for the whole test.
+ * chunk_steps per launch of the persistent kernels (one per length class,
+ * side by side), and retires finished ones.  All that a candidate needs lives
+ * in its slot of device memory (0.47 MB at 50 000 digits, 0.93 MB at 100 000)
+ * for the whole test; a request whose slot exceeds the whole budget is set up
+ * for the integer engine, whose slots are about half as large.
  * If a slot allocation fails below the budget (device memory held
  * elsewhere), the server frees its pooled slot memory and retries; failing
  * that, the request waits until resident candidates retire, or gets verdict
@@ -234,7 +241,7 @@ int pfb_mr_radix16_forms(pfb_mr_t *e, int ctas, int reps, double *ms_butterfly, 
                          long long *mismatches, int *tensor_error);
 
 /*
- * Autotuner of the persistent squaring kernel, per transform-length bucket
+ * Autotuner of the persistent squaring kernels, per transform-length bucket
  * (log2 L from logl_lo to logl_hi, within 8..15: the integer engine's length
  * for the longest number of a batch, whichever engine runs it; a 50 000-digit
  * modulus is 14, 100 000 digits 15).  For each bucket it times 2048 squarings of

@@ -5,8 +5,8 @@
 // Bound: the double-precision pipe (64 fused multiply-adds per clock and SM)
 // for long numbers, the chain of passes and block barriers for short ones.
 // Measured per squaring of one candidate on one SM, integer engine -> this
-// one: 600 digits 14 -> 3.4 us, 10 000 digits 33 -> 8.3 us, 50 000 digits
-// 98.6 -> 53.4 us.
+// one: 600 digits 14 -> 3.2 us, 9800 digits 33 -> 8.0 us, 50 000 digits
+// 98.6 -> 43 us, 100 000 digits 186 -> 79 us.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>

@@ -6,9 +6,9 @@ include/batch_mod_ctx.cuh, libpfb200.so and GMP (the declaration-only
 oracle/include/gmp.h over the image's libgmp.so.10), and runs it: residue
 round trips, raw squares and products against mpz_mul, modsq and modmul,
 16 chained squarings, x^0xDEADBEEF against mpz_powm_ui, (N-1)^2 = 1 and
-check_passed, for 512- to 332 000-bit moduli (every transform length the
-engine uses for them, the 100 000-digit one included).  Every check must
-pass on every modulus.
+check_passed, for 512- to 332 000-bit moduli (five lengths, the longest, of
+100 000 digits, on the integer engine).  Every check must pass on every
+modulus.
 """
 import ctypes as C
 import os

@@ -20,9 +20,10 @@ def test_reference_work_count():
 
 
 def test_engine_work_count():
-    """FP64 instructions of one squaring against the counter of a run
-    (smsp__inst_executed_pipe_fp64 warp instructions, 64 squarings of four
-    numbers): within 2 % at 2^k and 3 2^k points."""
+    """FP64 instructions of one squaring against the counter of runs whose
+    lanes were all busy (smsp__inst_executed_pipe_fp64 warp instructions, 64
+    squarings of four numbers; 1536 and 6144 points before their passes were
+    split among teams of warps): within 2 %."""
     for bits, warp_instructions in ((32760, 8844), (49144, 14220), (184312, 66072), (245752, 89136)):
         assert abs(bench.fp64_ops_per_squaring(bits) / 32 / warp_instructions - 1) < 0.02, bits
 

@@ -91,8 +91,8 @@ def test_lucas_mersenne_primes(mr, p):
 
 
 def test_lucas_mersenne_prime_long_transform(mr):
-    """M_216091 (216 091 bits): the length-2^15 transforms with the spectra of
-    the two NTT primes computed one after the other (D = 5, Q = -1)."""
+    """M_216091 (216 091 bits): 8192 points, x^2's spectrum in the candidate's
+    global memory (D = 5, Q = -1)."""
     assert mr.lucas([(1 << 216091) - 1]) == [1]
 
 

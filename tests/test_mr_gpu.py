@@ -133,7 +133,8 @@ def test_invalid_inputs_flagged(mr):
 
 
 def test_bucket_boundaries(mr):
-    # largest modulus of each transform length, and one bit more
+    # largest modulus of each of the integer engine's transform lengths, and one
+    # bit more (the last one is too long for the floating-point engine)
     rng = random.Random(13)
     Ns = []
     for lg in range(8, 16):
@@ -273,9 +274,9 @@ def test_uniform_batch_every_candidate_residue(mr):
 
 def test_uneven_batch_subset_residues(mr):
     """The first 128 of the 512 uneven-batch candidates (50 000 - 100 000
-    digits; 12 of them at the shorter transform length, so both lengths share
-    the batch's launches) against GMP: residues word for word (SHA-256 and
-    low 64 bits), verdicts bit for bit."""
+    digits: 6144, 8192 and 12 288 points, whose launches run side by side)
+    against GMP: residues word for word (SHA-256 and low 64 bits), verdicts bit
+    for bit."""
     from pfb200.workloads import uneven_tuples
     name = "mr_uneven_first128.json"
     if not os.path.exists(os.path.join(GOLD, name)):
@@ -283,7 +284,7 @@ def test_uneven_batch_subset_residues(mr):
     recs = _golden(name)["records"]
     assert [(r["a"], r["b"], r["c"], r["k"], r["j"], bool(r["rev"])) for r in recs] == \
         uneven_tuples(512)[:len(recs)]
-    assert len({r["bits"] > 22 * (1 << 13) - 36 for r in recs}) == 2  # both transform lengths
+    assert len({r["bits"] > 22 * (1 << 13) - 36 for r in recs}) == 2  # both integer lengths
     _check_records(mr, recs)
 
 

@@ -95,13 +95,13 @@ def test_invalid_requests_reported(engine):
 
 
 def test_full_size_requests_in_the_mix(engine):
-    """Ten 50 000 - 100 000-digit requests of the uneven workload (both
-    transform lengths: four at <= 54 250 digits) through a server with eight
+    """Ten 50 000 - 100 000-digit requests of the uneven workload (of several
+    length classes: four at <= 54 250 digits) through a server with eight
     slots: two requests wait for a slot and are admitted while the others run.
     Every residue must hash to GMP's (tests/golden/mr_uneven_first32.json)."""
     path = os.path.join(os.path.dirname(__file__), "golden", "mr_uneven_first32.json")
     recs = json.load(open(path))["records"]
-    pick = [0, 1, 2, 4, 6, 3, 5, 7, 22, 23]   # 3, 5, 22, 23: the shorter transform length
+    pick = [0, 1, 2, 4, 6, 3, 5, 7, 22, 23]   # 3, 5, 22, 23: the shorter ones
     assert sum(1 for i in pick if recs[i]["a"] <= 54250) == 4
     srv = pfb200.MRServer(engine, max_resident=8, chunk_steps=256)
     Ns = {}
