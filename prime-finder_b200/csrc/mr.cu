@@ -1149,6 +1149,16 @@ void srv_retire(pfb_mr_server *s) {
     }
 }
 
+// Whether a class has a stream and an event of its own, made on first use;
+// where they cannot be made, it runs on the server's stream after the others.
+bool srv_side(pfb_mr_server *s, int c) {
+    if (s->side[c]) return true;
+    if (!s->join[c] && cudaEventCreateWithFlags(&s->join[c], cudaEventDisableTiming) != cudaSuccess) s->join[c] = nullptr;
+    if (s->join[c] && cudaStreamCreateWithFlags(&s->side[c], cudaStreamNonBlocking) != cudaSuccess) s->side[c] = nullptr;
+    if (!s->side[c]) cudaGetLastError();
+    return s->side[c] != nullptr;
+}
+
 // Enqueues one launch of the persistent kernel per engine and length class
 // with residents, side by side, and joins them on the server's stream.
 int srv_launch(pfb_mr_server *s) {
@@ -1190,11 +1200,7 @@ int srv_launch(pfb_mr_server *s) {
         int nc = s->runs.count[c], qc = 0;
         if (!nc) continue;
         cudaStream_t st = s->stream;
-        if (forked) {
-            if (!s->side[c]) {
-                PFB_CUDA(cudaStreamCreateWithFlags(&s->side[c], cudaStreamNonBlocking));
-                PFB_CUDA(cudaEventCreateWithFlags(&s->join[c], cudaEventDisableTiming));
-            }
+        if (forked && srv_side(s, c)) {
             st = s->side[c];
             PFB_CUDA(cudaStreamWaitEvent(st, s->fork, 0));
         }
@@ -1209,7 +1215,7 @@ int srv_launch(pfb_mr_server *s) {
     }
     if (forked)
         for (int c = 0; c < fp::kClasses; c++)
-            if (s->runs.count[c]) {
+            if (s->runs.count[c] && s->side[c]) {
                 PFB_CUDA(cudaEventRecord(s->join[c], s->side[c]));
                 PFB_CUDA(cudaStreamWaitEvent(s->stream, s->join[c], 0));
             }

@@ -46,7 +46,7 @@ inline std::mutex mu;
 inline std::map<void *, size_t> blocks;
 inline size_t used = 0, peak = 0, limit = ~(size_t)0;
 inline long allow = -1;  // allocations left (-1: no limit)
-inline long refused = 0;
+inline bool no_streams = false;  // no further stream can be created
 
 // What a launch of `func` with these arguments does, ready to be called once
 // the argument array is gone; set by the test.
@@ -66,7 +66,6 @@ template <class T>
 inline cudaError_t cudaMalloc(T **p, size_t n) {
     std::lock_guard<std::mutex> lk(fake::mu);
     if (fake::allow == 0 || fake::used + n > fake::limit) {
-        fake::refused++;
         return cudaErrorMemoryAllocation;
     }
     if (fake::allow > 0) fake::allow--;
@@ -110,6 +109,7 @@ inline cudaError_t cudaDeviceGetAttribute(int *v, int, int) {
     return cudaSuccess;
 }
 inline cudaError_t cudaStreamCreateWithFlags(cudaStream_t *s, int) {
+    if (fake::no_streams) return cudaErrorMemoryAllocation;
     *s = new int(0);
     return cudaSuccess;
 }

@@ -7,6 +7,8 @@
 //                       `allow` device allocations granted after the server's
 //                       creation (-1: all) -> "verdict v" or "stopped rc",
 //                       then the engine that ran it (fft, int, none)
+//   mixed streams       a server with two requests of different length classes, that
+//                       can (1) or cannot (0) create further streams -> as server
 //   batch bytes bits n  strong tests of n numbers on a device of that many bytes
 //                       beyond what the engine holds (-1: no limit) -> "rc c",
 //                       device memory of the batch and the engine that ran it
@@ -16,6 +18,7 @@
 //   tune lg             autotune of one transform length -> "rc c", launches of the
 //                       persistent kernel and the pair kept
 #include <algorithm>
+#include <atomic>
 #include <chrono>
 #include <condition_variable>
 #include <deque>
@@ -38,6 +41,7 @@ int cuda_fail(cudaError_t, const char *, const char *, int) { return PFB_E_CUDA;
 static int n_fft, n_int;        // candidates that each engine has finished
 static int prep_fft, prep_int;  // and that each has set up
 static int launches;
+static std::atomic<bool> held;  // the FFT kernels finish nothing while set
 static int fn_fft, fn_int;
 
 namespace pfb {
@@ -97,6 +101,7 @@ static std::function<void()> launch(void *func, void **a) {
     const int *list = *(const int **)a[1], n = *(int *)a[2];
     return [=] {
         launches++;
+        if (held) return;
         for (int i = 0; i < n; i++) finish(jobs[list[i]], n_fft);
     };
 }
@@ -140,6 +145,34 @@ int main() {
             if (n == 1) std::cout << "verdict " << (int)r.verdict;
             else std::cout << "stopped " << n;
             fake::allow = -1;
+            pfb_mr_server_destroy(s);
+            std::cout << " " << engine(n_fft, n_int) << std::endl;
+        } else if (op == "mixed") {
+            int streams;
+            in >> streams;
+            pfb_mr_server_t *s = nullptr;
+            if (pfb_mr_server_create(e, nullptr, &s)) return 2;
+            fake::no_streams = !streams;
+            held = true;
+            for (int bits : {3000, 9000}) {
+                const std::vector<uint16_t> l = number(bits);
+                pfb_mr_server_submit(s, l.data(), (int)l.size(), (uint64_t)bits, nullptr, 0);
+            }
+            pfb_mr_server_stats_t st{};
+            for (int i = 0; i < 200 && !st.error && st.resident < 2; i++) {
+                std::this_thread::sleep_for(std::chrono::milliseconds(20));
+                pfb_mr_server_stats(s, &st);
+            }
+            held = false;
+            pfb_mr_result_t r[2];
+            int n = 0;
+            for (int i = 0; i < 50 && n >= 0 && n < 2; i++) {
+                const int k = pfb_mr_server_poll(s, r + n, 2 - n, 100);
+                n = k < 0 ? k : n + k;
+            }
+            if (n == 2) std::cout << "verdict " << (int)r[0].verdict << " " << (int)r[1].verdict;
+            else std::cout << "stopped " << n;
+            fake::no_streams = false;
             pfb_mr_server_destroy(s);
             std::cout << " " << engine(n_fft, n_int) << std::endl;
         } else if (op == "batch") {

@@ -69,3 +69,9 @@ def test_autotune_times_what_a_quantum_changes(host):
     the shape of one candidate per SM is timed once per chunk: 1 + 3 launches,
     and 1 + 9 with two per SM; equal rates keep the defaults."""
     assert host(["tune 12", "tune 15"]) == ["rc 0 14 64 2048"] * 2
+
+
+def test_server_runs_classes_in_turn_without_more_streams(host):
+    """Two length classes run side by side on streams of their own, or one
+    after the other where no further stream can be created."""
+    assert host(["mixed 1", "mixed 0"]) == ["verdict 0 0 fft"] * 2
